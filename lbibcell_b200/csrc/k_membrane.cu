@@ -232,13 +232,17 @@ struct Stencil {
     int x0, x1, y0, y1;
 };
 
+__device__ __forceinline__ bool stencil_on_lattice(const Stencil& s, int nx, int ny) {
+    const int wx = s.x1 - s.x0, wy = s.y1 - s.y0;
+    return wx >= 3 && wx <= 4 && wy >= 3 && wy <= 4 && s.x0 >= 0 && s.y0 >= 0 && s.x1 < nx && s.y1 < ny;
+}
+
 __device__ __forceinline__ bool stencil_range(double X, double Y, int nx, int ny, Stencil& s) {
     s.x0 = (int)ceil(X - 2.0);
     s.y0 = (int)ceil(Y - 2.0);
     s.x1 = (int)floor(X + 2.0);
     s.y1 = (int)floor(Y + 2.0);
-    const int wx = s.x1 - s.x0, wy = s.y1 - s.y0;
-    return wx >= 3 && wx <= 4 && wy >= 3 && wy <= 4 && s.x0 >= 0 && s.y0 >= 0 && s.x1 < nx && s.y1 < ny;
+    return stencil_on_lattice(s, nx, ny);
 }
 
 // Is lattice node (x, y) bound by the stencil (the last writer of its slot)?
@@ -605,56 +609,116 @@ __device__ __forceinline__ bool needs_perturbation(double X, double Y) {
     return false;
 }
 
+// Four lanes per membrane node, one per column of its stencil (eight nodes per
+// warp).  A lane forms its column's and its row's Dirac factor (the rows'
+// factors are shared by shuffles), loads the column's four rows of both
+// velocity components at once and leaves the 16 products per component in
+// shared memory by slot; then one lane per component adds them in slot order
+// (the order of collectVelocity's sum is part of the result).
+// With one thread per node the 16 loads, weights and additions formed one
+// serial chain: 9.3 us for a single cell's 500 nodes and 14.3 us (FP64 18.1)
+// for 150k nodes.  This form takes 2.8 us, and 11.2 us (FP64 13.7), where the
+// L1 pipe (gathers, products) bounds it.
+constexpr int kInterpBlock = 128;
+constexpr int kInterpNodes = kInterpBlock / 4;  // nodes per block
+// Place of (slot, node e) in a warp's products: eight nodes per slot, swapped
+// about by the slot's column so that the four columns of two nodes, which a
+// quarter warp stores at once, lie in different banks.
+__device__ __forceinline__ int interp_place(int slot, int e) { return slot * 8 + (e ^ ((slot >> 2) << 1)); }
+
 template <typename Real>
-__global__ void interp_move_kernel(MembraneDev m, const Real* u, int nx, int ny, size_t L, CrossDev c, Status* st,
-                                   unsigned iteration) {
+__global__ void __launch_bounds__(kInterpBlock) interp_move_kernel(MembraneDev m, const Real* u, int nx, int ny,
+                                                                   size_t L, CrossDev c, Status* st,
+                                                                   unsigned iteration) {
     pdl_wait();
     if (st->halt) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.topo->M) return;
-    const double X = m.x[i], Y = m.y[i];
-    Stencil sc;
-    if (!stencil_range(m.bx[i], m.by[i], nx, ny, sc)) {
-        raise_error(st, ERR_STENCIL, i, ST_INTERP_MOVE);
-        return;
+    __shared__ double2 prod[kInterpBlock / 32][16 * 8];
+    const int M = m.topo->M;
+    const int lane = threadIdx.x & 31, col = lane & 3, e = lane >> 2;
+    double2* p = prod[threadIdx.x >> 5];
+    const int i = blockIdx.x * kInterpNodes + (int)(threadIdx.x >> 2);
+    if (i - e >= M) return;  // the whole warp
+    const bool live = i < M;
+    double X = 0.0, Y = 0.0, bind = 32.0;
+    if (live) {
+        X = m.x[i];
+        Y = m.y[i];
+        bind = col < 2 ? m.bx[i] : m.by[i];
     }
+    // stencil_range, one of its four bounds per lane
+    const int bound = (col & 1) ? (int)floor(bind + 2.0) : (int)ceil(bind - 2.0);
+    Stencil sc;
+    sc.x0 = __shfl_sync(0xffffffffu, bound, lane & ~3);
+    sc.x1 = __shfl_sync(0xffffffffu, bound, (lane & ~3) + 1);
+    sc.y0 = __shfl_sync(0xffffffffu, bound, (lane & ~3) + 2);
+    sc.y1 = __shfl_sync(0xffffffffu, bound, (lane & ~3) + 3);
+    const bool ok = live && stencil_on_lattice(sc, nx, ny);
+    if (live && !ok && col == 0) raise_error(st, ERR_STENCIL, i, ST_INTERP_MOVE);
     // the Dirac factors of the stencil's columns and rows, each formed once:
     // (fa * fb) / 16 is calculateDiscreteDeltaDirac's expression
     const double halfPi = M_PI / 2.0;
-    double fa[5], fb[5];
+    const double fa = 1.0 + fast_cos(halfPi * ((double)(sc.x0 + col) - X));
+    const double fbOwn = 1.0 + fast_cos(halfPi * ((double)(sc.y0 + col) - Y));
+    double fb[4];
 #pragma unroll
-    for (int q = 0; q < 5; ++q) {
-        fa[q] = 1.0 + fast_cos(halfPi * ((double)(sc.x0 + q) - X));
-        fb[q] = 1.0 + fast_cos(halfPi * ((double)(sc.y0 + q) - Y));
+    for (int q = 0; q < 4; ++q) fb[q] = __shfl_sync(0xffffffffu, fbOwn, (lane & ~3) + q);
+    if (ok) {
+        if (sc.x1 - sc.x0 == 3 && sc.y1 - sc.y0 == 3) {
+            const size_t n0 = (size_t)sc.y0 * nx + (sc.x0 + col);
+            Real ux[4], uy[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                ux[q] = u[n0 + (size_t)q * nx];
+                uy[q] = u[L + n0 + (size_t)q * nx];
+            }
+            const int slot0 = 4 * (sc.x0 + col) + sc.y0;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const double dl = (fa * fb[q]) / 16.0;
+                p[interp_place((slot0 + q) & 15, e)] = make_double2((double)ux[q] * dl, (double)uy[q] * dl);
+            }
+        } else {
+            // wider stencil: the node bound to each slot (the slot's last writer)
+            for (int k = 4 * col; k < 4 * col + 4; ++k) {
+                int xk, yk;
+                stencil_slot(sc, k, xk, yk);
+                const size_t n = (size_t)yk * nx + xk;
+                const double dl = dirac((double)xk - X, (double)yk - Y);
+                p[interp_place(k, e)] = make_double2((double)u[n] * dl, (double)u[L + n] * dl);
+            }
+        }
     }
-    auto pick = [](const double* v, int i) {
-        return i == 0 ? v[0] : i == 1 ? v[1] : i == 2 ? v[2] : i == 3 ? v[3] : v[4];
-    };
-    double vx = 0.0, vy = 0.0;
-    for (int k = 0; k < 16; ++k) {
-        int xk, yk;
-        stencil_slot(sc, k, xk, yk);
-        const size_t n = (size_t)yk * nx + xk;
-        const double dl = (pick(fa, xk - sc.x0) * pick(fb, yk - sc.y0)) / 16.0;
-        vx += (double)u[n] * dl;
-        vy += (double)u[L + n] * dl;
+    __syncwarp();
+    double v = 0.0;  // lane 0 of the node: x component, lane 1: y component
+    if (ok && col < 2) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v += reinterpret_cast<const double*>(p + interp_place(k, e))[col];
+    }
+    const double vOther = __shfl_xor_sync(0xffffffffu, v, 1);
+    if (!ok || col > 1) return;
+    const double vx = col == 0 ? v : vOther, vy = col == 0 ? vOther : v;
+    const double CS = 1 / sqrt(3.0);
+    const bool fast = ((vx * vx) + (vy * vy)) > CS;
+    const double Xn = X + vx, Yn = Y + vy;
+    if (col == 1) {
+        m.vy[i] = vy;
+        if (fast) return;
+        m.oy[i] = Y;
+        m.y[i] = Yn;
+        return;
     }
     m.vx[i] = vx;
-    m.vy[i] = vy;
-    const double CS = 1 / sqrt(3.0);
-    if (((vx * vx) + (vy * vy)) > CS) {
+    if (fast) {
         raise_error(st, ERR_SPEED, i, ST_INTERP_MOVE);
         return;
     }
     m.ox[i] = X;
-    m.oy[i] = Y;
-    const double Xn = X + vx, Yn = Y + vy;
     m.x[i] = Xn;
-    m.y[i] = Yn;
+    // listed for the host; the next kernel raises the halt, so that every
+    // block here sees the same halt word and moves its nodes
     if (needs_perturbation(Xn, Yn)) {
         const int k = atomicAdd(&st->nPerturbNode, 1);
         if (k < c.perturbCap) c.perturbList[k] = i;
-        raise_halt(st, ST_INTERP_MOVE);
     }
 }
 
@@ -662,7 +726,8 @@ template <typename Real>
 void launch_interp_move(const MembraneDev& m, const Real* u, int nx, int ny, size_t L, CrossDev& c, Status* st,
                         unsigned iteration, cudaStream_t s) {
     if (m.Mcap == 0) return;
-    launch_pdl(interp_move_kernel<Real>, (m.Mcap + 127) / 128, 128, 0, s, m, u, nx, ny, L, c, st, iteration);
+    launch_pdl(interp_move_kernel<Real>, (m.Mcap + kInterpNodes - 1) / kInterpNodes, kInterpBlock, 0, s, m, u, nx, ny, L,
+               c, st, iteration);
 }
 template void launch_interp_move<double>(const MembraneDev&, const double*, int, int, size_t, CrossDev&, Status*,
                                          unsigned, cudaStream_t);
@@ -708,9 +773,14 @@ void launch_force_adjoint(const MembraneDev& m, const double* G, int nx, int ny,
 // counted and listed (up to cap); the crossing kernel, the next, raises the
 // halt, so that every block here sees the same halt word and the list is
 // complete.
+// The kernel first raises the halt for the nodes that the move listed.
 __global__ void perturb_conn_kernel(MembraneDev m, Status* st, int* list, int cap) {
     pdl_wait();
     if (st->halt) return;
+    if (st->nPerturbNode > 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
+        return;
+    }
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.topo->C) return;
     const int a = m.ca[c], b = m.cb[c];
@@ -722,8 +792,8 @@ __global__ void perturb_conn_kernel(MembraneDev m, Status* st, int* list, int ca
 
 void launch_perturb_conn_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s, int* list,
                                int cap) {
-    if (m.Ccap == 0) return;
-    launch_pdl(perturb_conn_kernel, (m.Ccap + 127) / 128, 128, 0, s, m, st, list, cap);
+    if (m.Mcap == 0 && m.Ccap == 0) return;
+    launch_pdl(perturb_conn_kernel, m.Ccap > 0 ? (m.Ccap + 127) / 128 : 1, 128, 0, s, m, st, list, cap);
 }
 
 // ---------------------------------------------------------------------------
