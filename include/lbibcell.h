@@ -8,7 +8,8 @@
  * abort across the ABI; lbib_last_error() gives the message and the index of
  * the node or connection involved.  The caller owns every host buffer; the
  * handle owns every device buffer.  A handle uses one CUDA stream and is not
- * thread-safe.
+ * thread-safe; the calls that copy large states to the host use further
+ * streams and threads of their own, which end with the call.
  *
  * The comment of each call names the reference interface it replaces (paths
  * relative to the LBIBCell project root).
@@ -86,6 +87,10 @@ int lbib_get_sizes(lbib_handle* h, long long* sizes);
  * Any pointer may be NULL.  FP32-shifted state is converted to f = h + w. */
 int lbib_download_lattice(lbib_handle* h, double* f, double* g, double* vel, double* force, unsigned* dom,
                           unsigned* ctype);
+
+/* The species' concentrations c[S][L]: per node the five values of g, added in
+ * lbib_download_lattice's slot order (PhysicalNode's CDE getC()). */
+int lbib_concentrations(lbib_handle* h, double* c);
 
 /* Overwrites the distributions (reference slot layout) and, if non-NULL, the
  * spread force field.  Replaces SimulationRunner::initSolvers(file)

@@ -22,6 +22,7 @@ SYMBOLS = (
     "lbib_read_vtm_geometry", "lbib_upload_membrane", "lbib_cure_lattice", "lbib_accumulated_concentrations",
     "lbib_set_cell_types", "lbib_get_cell_types", "lbib_init_velocity", "lbib_diff_mass", "lbib_diff_fluid_seed",
     "lbib_diff_force_params", "lbib_diff_motion", "lbib_diff_positions", "lbib_download_forces", "lbib_set_species_sources",
+    "lbib_concentrations",
 )
 
 _lib = None
@@ -57,6 +58,8 @@ def load() -> ctypes.CDLL:
     L.lbib_get_sizes.argtypes = [vp, vp]
     L.lbib_download_lattice.restype = ip
     L.lbib_download_lattice.argtypes = [vp] + [vp] * 6
+    L.lbib_concentrations.restype = ip
+    L.lbib_concentrations.argtypes = [vp, vp]
     L.lbib_upload_lattice.restype = ip
     L.lbib_upload_lattice.argtypes = [vp, vp, vp, vp]
     L.lbib_init_velocity.restype = ip

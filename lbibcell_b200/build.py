@@ -31,6 +31,7 @@ UNITS = [
     ("k_topology.cu", ["--fmad=false"]),
     ("k_forces.cu", ["--fmad=false"]),
     ("lbib_host.cu", ["--fmad=false"]),
+    ("k_readout.cu", ["--fmad=false"]),
     ("k_lattice32.cu", []),
     ("k_adjoint.cu", []),
     ("vtk_io.cu", []),

@@ -354,6 +354,24 @@ void launch_motion_adjoint(const double* X, const double* Y, const double* fx, c
                            double* ly, const double* uo, const double* G, double* gfx, double* gfy, int M, int nx,
                            int ny, size_t L, cudaStream_t s);
 
+// The state in the host's layouts (k_readout.cu): the parts of a read-out, in
+// the order they are packed (8-byte elements first).
+enum ReadoutPart { RO_F, RO_G, RO_C, RO_VEL, RO_FORCE, RO_STATE, RO_DOM, RO_CTYPE, RO_IDS, RO_CONN, RO_PARTS };
+struct ReadoutArgs {
+    int nx;
+    size_t L;
+    bool fp64;
+    const void* f; const void* g; const void* u; const void* force;
+    const int* tileCount;
+    int tilesX;
+    const uint32_t* dom;
+    const uint32_t* ctypeTab;
+    int nDomains;
+    bool cellTypesCopied;
+    MembraneDev m;
+};
+void launch_readout(const ReadoutArgs& a, int part, size_t e0, size_t n, void* out, cudaStream_t s);
+
 // Opt-in shared-memory sizes of the kernels that need more than 48 KB; called
 // once before any launch (and so before any stream capture).
 void init_kernel_attributes();

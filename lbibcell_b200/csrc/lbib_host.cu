@@ -12,6 +12,7 @@
 // order and resumes the step at the stage after the one that halted.  Steps
 // without such events run with no host round trip.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstddef>
@@ -26,6 +27,7 @@
 #include <sstream>
 #include <stdexcept>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include <cub/cub.cuh>
@@ -207,6 +209,100 @@ struct DiffCtx {
 constexpr size_t kTopoOffset = (sizeof(Status) + 63) / 64 * 64;
 constexpr size_t kAreaOffset = kTopoOffset + (sizeof(Topo) + 63) / 64 * 64;
 
+// A lane of the read-out (read_out): a stream, and two pinned buffers with
+// their device counterparts.
+constexpr size_t kReadChunk = 1u << 20;
+struct ReadLane {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t done[2] = {nullptr, nullptr};
+    char* dev = nullptr;
+    char* host = nullptr;
+
+    cudaError_t make() {
+        cudaError_t e = cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking);
+        for (cudaEvent_t& d : done)
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&d, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaMalloc(&dev, 2 * kReadChunk);
+        if (e == cudaSuccess) e = cudaHostAlloc(&host, 2 * kReadChunk, cudaHostAllocPortable);
+        return e;
+    }
+    ~ReadLane() {
+        if (dev) cudaFree(dev);
+        if (host) cudaFreeHost(host);
+        for (cudaEvent_t d : done)
+            if (d) cudaEventDestroy(d);
+        if (stream) cudaStreamDestroy(stream);
+    }
+};
+
+// The lanes of one device, shared by its handles (pinning a lane's 2 MB takes
+// up to 4 ms, a small simulation's whole read-out 0.1 ms): at most kReadLanes
+// kept, freed with the last handle that used them.  A call takes lanes out and
+// puts them back; calls from several threads on several handles share what
+// there is, and one that finds none makes one for itself.
+constexpr int kReadLanes = 8;
+class LanePool {
+public:
+    void join() {
+        std::lock_guard<std::mutex> lock(m_);
+        ++handles_;
+    }
+    void leave() {
+        std::lock_guard<std::mutex> lock(m_);
+        if (--handles_ == 0) {
+            kept_ -= (int)free_.size();
+            free_.clear();
+        }
+    }
+    // At least one lane and at most `want`; fails only if not one can be made.
+    cudaError_t take(int want, std::vector<std::unique_ptr<ReadLane>>& out) {
+        std::lock_guard<std::mutex> lock(m_);
+        while ((int)out.size() < want) {
+            if (!free_.empty()) {
+                out.push_back(std::move(free_.back()));
+                free_.pop_back();
+                continue;
+            }
+            if (kept_ >= kReadLanes && !out.empty()) break;
+            std::unique_ptr<ReadLane> l(new ReadLane());
+            const cudaError_t e = l->make();
+            if (e != cudaSuccess) {
+                if (out.empty()) return e;
+                cudaGetLastError();
+                break;
+            }
+            ++kept_;
+            out.push_back(std::move(l));
+        }
+        return cudaSuccess;
+    }
+    void give(std::vector<std::unique_ptr<ReadLane>>& lanes) {
+        std::lock_guard<std::mutex> lock(m_);
+        for (auto& l : lanes) {
+            if (kept_ > kReadLanes || handles_ == 0) {
+                --kept_;
+                l.reset();
+            } else {
+                free_.push_back(std::move(l));
+            }
+        }
+        lanes.clear();
+    }
+
+private:
+    std::mutex m_;
+    std::vector<std::unique_ptr<ReadLane>> free_;
+    int kept_ = 0;     // lanes made and not freed
+    int handles_ = 0;  // handles that have read out
+};
+
+static LanePool& lane_pool(int device) {
+    static std::mutex m;
+    static std::map<int, LanePool>* pools = new std::map<int, LanePool>();  // outlives every handle
+    std::lock_guard<std::mutex> lock(m);
+    return (*pools)[device];
+}
+
 struct Handle {
     // parameters
     int nx = 0, ny = 0, S = 0;
@@ -342,6 +438,9 @@ struct Handle {
 
     DiffCtx* diff = nullptr;
 
+    cudaEvent_t readReady = nullptr;  // the state a read-out waits for
+    bool inLanePool = false;          // counted in the device's read-out lanes
+
     ~Handle();
 };
 
@@ -379,6 +478,8 @@ Handle::~Handle() {
     fr(fs.binKey); fr(fs.binKeySorted); fr(fs.binIdx); fr(fs.binIdxSorted); fr(fs.sortTmp); fr(fs.closest);
     fr(fs.binStart); fr(fs.binHead); fr(fs.binNext); fr(fs.linkKey); fr(fs.linkPrevM);
     fr(fs.inCnt); fr(fs.inOff); fr(fs.inList); fr(fs.inFill);
+    if (readReady) cudaEventDestroy(readReady);
+    if (inLanePool) lane_pool(device).leave();
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -813,6 +914,126 @@ static void pull_topology(Handle& h) {
                            cdesc[c] >= 0 && cdesc[c] < (int)h.descTable.size() ? h.descTable[cdesc[c]] : std::string()};
     h.m.M = M;
     h.m.C = C;
+}
+
+// ---------------------------------------------------------------------------
+// Read-out: parts of the state into the caller's arrays.  The parts' bytes form
+// one sequence, cut into chunks; a lane packs a chunk on the device
+// (k_readout.cu), copies it to its pinned buffer and from there to the caller's
+// memory, with the next chunk under way meanwhile.  The copy to the caller's
+// memory (its first touch, mostly) bounds a large read-out, so several host
+// threads run a lane each, one per 2 MB up to eight; a small one is one chunk
+// on the calling thread.
+constexpr size_t kReadPerLane = 2u << 20;
+
+struct ReadPart {
+    int part;
+    void* dst;
+    size_t count;   // elements
+    size_t size;    // bytes of an element
+    size_t offset;  // of the part in the sequence
+};
+
+static void read_out(Handle& h, std::vector<ReadPart> parts) {
+    size_t total = 0;
+    for (ReadPart& p : parts) {
+        p.offset = total;
+        total += p.count * p.size;
+    }
+    if (total == 0) return;
+    ReadoutArgs a{};
+    a.nx = h.nx;
+    a.L = h.L;
+    a.fp64 = h.precision == LBIB_FP64;
+    a.f = h.f[h.cur];
+    a.g = h.g[h.cur];
+    a.u = h.u;
+    a.force = h.force;
+    a.tileCount = h.tiles.count;
+    a.tilesX = h.tiles.tilesX;
+    a.dom = h.dom;
+    a.ctypeTab = h.ctypeTab;
+    a.nDomains = (int)h.ctypeHost.size();
+    a.cellTypesCopied = h.cellTypesCopied;
+    a.m = h.m;
+
+    const size_t chunk = kReadChunk;
+    const int nChunks = (int)((total + chunk - 1) / chunk);
+    const int want = (int)std::min<size_t>({(size_t)kReadLanes, 1 + total / kReadPerLane, (size_t)nChunks,
+                                            std::max(1u, std::thread::hardware_concurrency())});
+    if (!h.readReady) CK(cudaEventCreateWithFlags(&h.readReady, cudaEventDisableTiming));
+    CK(cudaEventRecord(h.readReady, h.stream));
+    LanePool& pool = lane_pool(h.device);
+    if (!h.inLanePool) {
+        pool.join();
+        h.inLanePool = true;
+    }
+    std::vector<std::unique_ptr<ReadLane>> lanes;
+    CK(pool.take(want, lanes));
+
+    std::atomic<int> next{0};
+    std::atomic<int> failed{(int)cudaSuccess};
+    const int device = h.device;
+    auto run = [&](ReadLane& l) {
+        auto ok = [&](cudaError_t e) {
+            int none = (int)cudaSuccess;
+            if (e != cudaSuccess) failed.compare_exchange_strong(none, (int)e);
+            return e == cudaSuccess;
+        };
+        auto issue = [&](int c, int slot) {  // pack chunk c and copy it to the lane's buffer
+            const size_t b0 = (size_t)c * chunk, b1 = std::min(total, b0 + chunk);
+            char* dev = l.dev + (size_t)slot * chunk;
+            for (const ReadPart& p : parts) {
+                const size_t lo = std::max(b0, p.offset), hi = std::min(b1, p.offset + p.count * p.size);
+                if (lo >= hi) continue;
+                launch_readout(a, p.part, (lo - p.offset) / p.size, (hi - lo) / p.size, dev + (lo - b0), l.stream);
+            }
+            return ok(cudaGetLastError()) &&
+                   ok(cudaMemcpyAsync(l.host + (size_t)slot * chunk, dev, b1 - b0, cudaMemcpyDeviceToHost, l.stream)) &&
+                   ok(cudaEventRecord(l.done[slot], l.stream));
+        };
+        if (!ok(cudaSetDevice(device)) || !ok(cudaStreamWaitEvent(l.stream, h.readReady, 0))) return;
+        int c = next++, slot = 0;
+        bool go = c < nChunks && issue(c, slot);
+        while (go) {
+            const int n = next++;
+            const bool more = n < nChunks;
+            if (more && !issue(n, slot ^ 1)) break;
+            if (!ok(cudaEventSynchronize(l.done[slot]))) break;
+            const size_t b0 = (size_t)c * chunk, b1 = std::min(total, b0 + chunk);
+            const char* src = l.host + (size_t)slot * chunk;
+            for (const ReadPart& p : parts) {
+                const size_t lo = std::max(b0, p.offset), hi = std::min(b1, p.offset + p.count * p.size);
+                if (lo < hi) std::memcpy((char*)p.dst + (lo - p.offset), src + (lo - b0), hi - lo);
+            }
+            if (!more) break;
+            c = n;
+            slot ^= 1;
+        }
+        cudaStreamSynchronize(l.stream);  // nothing of a lane is in flight after the call
+    };
+    std::vector<std::thread> helpers;
+    helpers.reserve(lanes.size());
+    for (size_t i = 1; i < lanes.size(); ++i) {
+        try {
+            helpers.emplace_back(run, std::ref(*lanes[i]));
+        } catch (const std::exception&) {
+            break;  // no more threads: the others take the chunks
+        }
+    }
+    run(*lanes[0]);
+    for (std::thread& t : helpers) t.join();
+    pool.give(lanes);
+    CK((cudaError_t)failed.load());
+}
+
+// The membrane counts on the device, without the topology.
+static void pull_counts(Handle& h) {
+    Topo tp{};
+    CK(cudaMemcpyAsync(&tp, h.m.topo, sizeof(Topo), cudaMemcpyDeviceToHost, h.stream));
+    CK(cudaStreamSynchronize(h.stream));
+    h.m.M = tp.M;
+    h.m.C = tp.C;
 }
 
 // Copies the device's area targets to the host mirror (they are set on the
@@ -2597,62 +2818,22 @@ int lbib_get_sizes(lbib_handle* hh, long long* s) {
 int lbib_download_lattice(lbib_handle* hh, double* f, double* g, double* vel, double* force, unsigned* dom,
                           unsigned* ctype) {
     API_BEGIN(hh)
-    const size_t L = h.L;
-    const int S = h.S;
-    const bool fp64 = h.precision == LBIB_FP64;
-    const size_t rs = fp64 ? 8 : 4;
-    std::vector<char> buf;
-    auto fetch = [&](const void* src, size_t count) {
-        buf.resize(count * rs);
-        CK(cudaMemcpyAsync(buf.data(), src, count * rs, cudaMemcpyDeviceToHost, h.stream));
-        CK(cudaStreamSynchronize(h.stream));
-    };
-    auto val = [&](size_t i) -> double {
-        return fp64 ? ((const double*)buf.data())[i] : (double)((const float*)buf.data())[i];
-    };
-    static const int INV9[9] = {0, 3, 4, 1, 2, 7, 8, 5, 6};
-    static const int INV5[5] = {0, 3, 4, 1, 2};
-    static const double W9[9] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0,
-                                 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0, 1.0 / 36.0};
-    if (f) {
-        fetch(h.f[h.cur], 9 * L);
-        for (size_t n = 0; n < L; ++n)
-            for (int d = 0; d < 9; ++d) {
-                const int q = INV9[d];
-                f[n * 9 + d] = fp64 ? val(q * L + n) : val(q * L + n) + W9[q];
-            }
-    }
-    if (g && S > 0) {
-        fetch(h.g[h.cur], (size_t)S * 5 * L);
-        for (int k = 0; k < S; ++k)
-            for (size_t n = 0; n < L; ++n)
-                for (int d = 0; d < 5; ++d) g[((size_t)k * L + n) * 5 + d] = val(((size_t)k * 5 + INV5[d]) * L + n);
-    }
-    if (vel) {
-        fetch(h.u, 2 * L);
-        for (size_t n = 0; n < L; ++n) { vel[2 * n] = val(n); vel[2 * n + 1] = val(L + n); }
-    }
-    if (force) {
-        fetch(h.force, 2 * L);
-        std::vector<int> tc(h.tiles.nTiles);
-        CK(cudaMemcpyAsync(tc.data(), h.tiles.count, sizeof(int) * tc.size(), cudaMemcpyDeviceToHost, h.stream));
-        CK(cudaStreamSynchronize(h.stream));
-        for (size_t n = 0; n < L; ++n) {
-            const int x = (int)(n % h.nx), y = (int)(n / h.nx);
-            const bool act = tc[(y / lbib::kTile) * h.tiles.tilesX + x / lbib::kTile] > 0;
-            force[2 * n] = act ? val(n) : 0.0;
-            force[2 * n + 1] = act ? val(L + n) : 0.0;
-        }
-    }
-    if (dom || ctype) {
-        std::vector<uint32_t> d(L);
-        CK(cudaMemcpyAsync(d.data(), h.dom, sizeof(uint32_t) * L, cudaMemcpyDeviceToHost, h.stream));
-        CK(cudaStreamSynchronize(h.stream));
-        for (size_t n = 0; n < L; ++n) {
-            if (dom) dom[n] = d[n];
-            if (ctype) ctype[n] = h.cellTypesCopied ? (d[n] < h.ctypeHost.size() ? h.ctypeHost[d[n]] : 1u) : 0u;
-        }
-    }
+    const size_t L = h.L, S = (size_t)h.S;
+    std::vector<lbib::ReadPart> parts;
+    if (f) parts.push_back({lbib::RO_F, f, 9 * L, 8, 0});
+    if (g && S > 0) parts.push_back({lbib::RO_G, g, 5 * S * L, 8, 0});
+    if (vel) parts.push_back({lbib::RO_VEL, vel, 2 * L, 8, 0});
+    if (force) parts.push_back({lbib::RO_FORCE, force, 2 * L, 8, 0});
+    if (dom) parts.push_back({lbib::RO_DOM, dom, L, 4, 0});
+    if (ctype) parts.push_back({lbib::RO_CTYPE, ctype, L, 4, 0});
+    lbib::read_out(h, parts);
+    API_END
+}
+
+int lbib_concentrations(lbib_handle* hh, double* c) {
+    API_BEGIN(hh)
+    if (!c && h.S > 0) lbib::fail(LBIB_ERR_INPUT, "lbib_concentrations: null argument");
+    lbib::read_out(h, {{lbib::RO_C, c, (size_t)h.S * h.L, 8, 0}});
     API_END
 }
 
@@ -2714,25 +2895,19 @@ int lbib_init_velocity(lbib_handle* hh, double ux, double uy) {
 
 int lbib_download_membrane(lbib_handle* hh, unsigned* ids, double* state) {
     API_BEGIN(hh)
-    lbib::pull_topology(h);
-    lbib::HostMembrane hm;
-    lbib::download_membrane(h, hm);
-    for (size_t i = 0; i < h.ids.size(); ++i) {
-        if (ids) ids[i] = h.ids[i];
-        if (state) {
-            double* o = state + 6 * i;
-            o[0] = hm.x[i]; o[1] = hm.y[i]; o[2] = hm.vx[i]; o[3] = hm.vy[i]; o[4] = hm.fx[i]; o[5] = hm.fy[i];
-        }
-    }
+    lbib::pull_counts(h);
+    const size_t M = (size_t)h.m.M;
+    std::vector<lbib::ReadPart> parts;
+    if (state) parts.push_back({lbib::RO_STATE, state, 6 * M, 8, 0});
+    if (ids) parts.push_back({lbib::RO_IDS, ids, M, 4, 0});
+    lbib::read_out(h, parts);
     API_END
 }
 
 int lbib_download_connections(lbib_handle* hh, unsigned* conn) {
     API_BEGIN(hh)
-    lbib::pull_topology(h);
-    for (size_t c = 0; c < h.conns.size(); ++c) {
-        conn[3 * c] = h.conns[c].id1; conn[3 * c + 1] = h.conns[c].id2; conn[3 * c + 2] = h.conns[c].dom;
-    }
+    lbib::pull_counts(h);
+    lbib::read_out(h, {{lbib::RO_CONN, conn, 3 * (size_t)h.m.C, 4, 0}});
     API_END
 }
 

@@ -137,8 +137,8 @@ class Simulation:
     def lattice(self) -> LatticeState:
         z = self.sizes()
         L, S = z["nx"] * z["ny"], z["S"]
-        f = np.zeros((L, 9)); g = np.zeros((S, L, 5)); vel = np.zeros((L, 2)); force = np.zeros((L, 2))
-        dom = np.zeros(L, np.uint32); ctype = np.zeros(L, np.uint32)
+        f = np.empty((L, 9)); g = np.empty((S, L, 5)); vel = np.empty((L, 2)); force = np.empty((L, 2))
+        dom = np.empty(L, np.uint32); ctype = np.empty(L, np.uint32)
         self._check(self._L.lbib_download_lattice(self._h, _p(f), _p(g), _p(vel), _p(force), _p(dom), _p(ctype)))
         return LatticeState(f, g, vel, force, dom, ctype)
 
@@ -154,13 +154,13 @@ class Simulation:
     def membrane(self):
         """(ids[M], state[M, 6]) with state = x, y, vx, vy, fx, fy, in id order."""
         M = self.sizes()["M"]
-        ids = np.zeros(M, np.uint32); st = np.zeros((M, 6))
+        ids = np.empty(M, np.uint32); st = np.empty((M, 6))
         self._check(self._L.lbib_download_membrane(self._h, _p(ids), _p(st)))
         return ids, st
 
     def connections(self) -> np.ndarray:
         C = self.sizes()["C"]
-        c = np.zeros((C, 3), np.uint32)
+        c = np.empty((C, 3), np.uint32)
         self._check(self._L.lbib_download_connections(self._h, _p(c)))
         return c
 
@@ -395,7 +395,10 @@ class Simulation:
 
     def concentrations(self) -> np.ndarray:
         """C_k(x) = sum of species k's distributions, shape (S, Nx*Ny)."""
-        return self.lattice().g.sum(axis=2)
+        z = self.sizes()
+        c = np.empty((z["S"], z["nx"] * z["ny"]))
+        self._check(self._L.lbib_concentrations(self._h, _p(c)))
+        return c
 
 
 def read_vtm_geometry(path: str):
