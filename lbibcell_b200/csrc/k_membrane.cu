@@ -6,10 +6,10 @@
 //                    (ForceStructs.hpp:49-588).
 //   spread           SimulationRunner::distributeForce + GeometryNode::distributeForce
 //                    (SimulationRunner.cpp:425-453, GeometryNode.cpp:228-235) as a
-//                    deterministic gather: each 16x16 lattice tile collects the
+//                    deterministic sum: each 16x16 lattice tile collects the
 //                    membrane nodes whose 4x4 stencil overlaps it, sorts them by
-//                    id and every lattice node sums its contributions in id order
-//                    (the reference's serial map order).  No floating-point atomics.
+//                    id and adds their contributions in id order (the
+//                    reference's serial map order).  No floating-point atomics.
 //   interp_move      GeometryNode::collectVelocity (GeometryNode.cpp:216-226, slot
 //                    order (4x+y) mod 16 from GeometryHandler.cpp:641), the speed
 //                    check (LagrangianPoint.cpp:92-103) and GeometryNode::move
@@ -63,8 +63,8 @@ __device__ __forceinline__ int tile_agg_add(int* arr, int tile, bool valid);
 __device__ void tile_slot_node(const MembraneDev& m, TileDev& t, int i, bool ok, int nx, int ny, Status* st);
 
 // `begin`: the first kernel of a step (begin_step).
-// `slots`: also enter the node in the per-tile lists of the FP32-shifted
-// spread (the tile counts were cleared before the launch).
+// `slots`: also enter the node in the per-tile lists of the spread (which left
+// the tile counts at zero).
 __global__ void force_eval_kernel(MembraneDev m, Status* st, unsigned iteration, int begin, TileDev t, int nx,
                                   int ny, int slots) {
     pdl_wait();
@@ -209,7 +209,6 @@ void launch_force_eval(const MembraneDev& m, Status* st, unsigned iteration, cud
     TileDev t{};
     if (tiles) {
         t = *tiles;
-        cudaMemsetAsync(t.count, 0, sizeof(int) * (t.nTiles + 1), s);
     }
     launch_pdl(force_eval_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, st, iteration, begin ? 1 : 0, t, nx, ny,
                tiles ? 1 : 0);
@@ -283,8 +282,8 @@ __device__ __forceinline__ int tile_agg_add(int* arr, int tile, bool valid) {
     return base + __popc(grp & ((1u << lane) - 1u));
 }
 
-// FP32-shifted runs: node i into the fixed-size slot lists of the (up to 2 x 2)
-// tiles its stencil covers.
+// Node i into the fixed-size slot lists of the (up to 2 x 2) tiles its stencil
+// covers.
 __device__ void tile_slot_node(const MembraneDev& m, TileDev& t, int i, bool ok, int nx, int ny, Status* st) {
     Stencil sc{0, 0, 0, 0};
     if (ok && !stencil_range(m.bx[i], m.by[i], nx, ny, sc)) {
@@ -311,159 +310,157 @@ __global__ void tile_slot_kernel(MembraneDev m, TileDev t, int nx, int ny, Statu
     tile_slot_node(m, t, i, i < m.topo->M, nx, ny, st);
 }
 
-__global__ void tile_count_kernel(MembraneDev m, TileDev t, int nx, int ny, Status* st, int pass) {
-    pdl_wait();
-    if (st->halt) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool ok = i < m.topo->M;
-    Stencil sc{0, 0, 0, 0};
-    if (ok && !stencil_range(m.bx[i], m.by[i], nx, ny, sc)) {
-        raise_error(st, ERR_STENCIL, i, ST_SPREAD);
-        ok = false;
-    }
-    const int tx0 = sc.x0 / kTile, tx1 = sc.x1 / kTile, ty0 = sc.y0 / kTile, ty1 = sc.y1 / kTile;
-    // up to 2 x 2 tiles per stencil; all lanes run the four rounds together
-    for (int j = 0; j < 4; ++j) {
-        const int tx = tx0 + (j & 1), ty = ty0 + (j >> 1);
-        const bool v = ok && tx <= tx1 && ty <= ty1;
-        const int tile = v ? ty * t.tilesX + tx : -1;
-        if (pass == 0) {
-            tile_agg_add(t.count, tile, v);
-        } else {
-            const int slot = tile_agg_add(t.fill, tile, v);
-            if (v) {
-                const int pos = t.start[tile] + slot;
-                if (pos < t.cap) t.list[pos] = i;
-            }
-        }
-    }
-}
-
-// Membrane stencils per tile held in shared memory: most tiles hold fewer than
-// kSpreadSmall; the others go to the kSpreadLarge variant.
-constexpr int kSpreadSmall = 256;
-constexpr int kSpreadLarge = 768;
-constexpr size_t spread_smem(int cap) {
-    return (size_t)cap * (12 * sizeof(double) + 2 * sizeof(int) + 8 * sizeof(unsigned short));
-}
-
 // Per-tile entry: the stencil origin relative to the tile (+4) and the stencil
 // widths, packed in one word: ox | oy << 8 | (x1-x0) << 16 | (y1-y0) << 20.
 __device__ __forceinline__ int pack_stencil(const Stencil& s, int tileX0, int tileY0) {
     return (s.x0 - tileX0 + 4) | ((s.y0 - tileY0 + 4) << 8) | ((s.x1 - s.x0) << 16) | ((s.y1 - s.y0) << 20);
 }
 
-// Sorts the tile's membrane indices ascending (= id order) into `out`.
-template <int ITEMS>
-__device__ __forceinline__ void sort_tile_list(const int* list, int cnt, int sortBits, int* out, void* tmp) {
-    typedef cub::BlockRadixSort<int, 256, ITEMS> Sort;
-    int keys[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int k = threadIdx.x * ITEMS + j;
-        keys[j] = k < cnt ? list[k] : 0x7fffffff;
+// The tile's list as the spread takes it: its length, noted for the readers of
+// the force field, and the counter left at zero for the next step's lists (a
+// memset node between two kernels of the step cost 3.5 us).
+__device__ __forceinline__ int take_tile_count(const TileDev& t, int tile) {
+    __shared__ int count;
+    if (threadIdx.x == 0) {
+        count = t.count[tile];
+        t.active[tile] = count;
+        if (count != 0) t.count[tile] = 0;
     }
-    Sort(*(typename Sort::TempStorage*)tmp).Sort(keys, 0, sortBits);
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-        const int k = threadIdx.x * ITEMS + j;
-        if (k < cnt) out[k] = keys[j];
-    }
+    __syncthreads();
+    return count;
 }
 
-// Each 16x16 tile: its membrane nodes sorted by id; per node the Dirac factors
+// FP64 runs, whose sums must be formed in the reference's order: each 16x16
+// tile sorts its membrane nodes by index (= id order; the rank of an entry is
+// the number of smaller ones) and forms per node the Dirac factors
 // A_i = 1 + fastCos(pi/2 (x0 + i - X)) and B_j = 1 + fastCos(pi/2 (y0 + j - Y)),
 // so that the weight of lattice node (x0+i, y0+j) is (A_i * B_j) / 16, the same
-// expression as calculateDiscreteDeltaDirac (GeometryNode.cpp:89-94).  Each warp
-// covers two rows of the tile and first collects, in id order, the entries
-// whose stencil rows meet its rows; every lattice node then adds its
-// contributions in id order.
-// Used by FP64 runs, whose summation order must be the reference's.
-template <typename Real, int kSpreadMax, int kMinCount>
+// expression as calculateDiscreteDeltaDirac (GeometryNode.cpp:89-94; A is kept
+// as A / 16, an exact scaling).  Each warp owns two rows of the tile and takes,
+// in id order, the entries whose stencil rows meet them; the lane of a lattice
+// node adds an entry's products to it in registers, without a branch, so that
+// the entries' loads and products overlap and only the additions form a chain.  Longer lists go through in chunks, in order.
+// With lists built by count, scan and fill, a radix sort per tile and a lane per
+// node testing every entry, the spread took 96 us for 150k nodes on 1024^2 and
+// 21 us for one cell.  Adding each entry's 16 products to shared memory, a
+// lane each, took 48 and 17 us (a chain of shared-memory round trips); this
+// form takes 40 (instruction issue) and 6.5 us.  Four rows per warp of a
+// 128-thread block: 40 and 8.2 us.
+constexpr int kSpreadMax = 768;    // entries of a tile
+constexpr int kSpreadChunk = 128;  // entries whose factors are held at once
+template <typename Real>
 __global__ void __launch_bounds__(256) spread_kernel(MembraneDev m, TileDev t, Real* force, int nx, int ny, size_t L,
-                                                     Status* st, int sortBits) {
+                                                     Status* st) {
     pdl_wait();
     if (st->halt) return;
     const int tile = blockIdx.x;
-    const int cnt = t.count[tile];
-    // each size class handles the tiles whose count it fits best
-    if (cnt == 0 || cnt < kMinCount || (kMinCount == 0 && cnt > kSpreadMax)) return;
-    if (cnt > kSpreadMax || t.start[tile] + cnt > t.cap) {
+    const int cnt = take_tile_count(t, tile);
+    if (cnt == 0) return;
+    if (cnt > kSpreadMax) {
         if (threadIdx.x == 0) raise_error(st, ERR_CAPACITY, tile, ST_SPREAD);
         return;
     }
-    extern __shared__ __align__(16) unsigned char smem[];
-    double* fac = (double*)smem;                          // kSpreadMax x 10: A[5], B[5]
-    double* sfx = fac + 10 * kSpreadMax;
-    double* sfy = sfx + kSpreadMax;
-    int* code = (int*)(sfy + kSpreadMax);
-    int* order = code + kSpreadMax;                      // sorted membrane indices
-    unsigned short* wlist = (unsigned short*)(order + kSpreadMax);  // 8 warps x kSpreadMax
-    __shared__ __align__(16) unsigned char sortTmp[sizeof(typename cub::BlockRadixSort<int, 256, (kSpreadMax + 255) / 256>::TempStorage)];
-    const int* list = t.list + t.start[tile];
-    if (kSpreadMax <= 256 || cnt <= 256) sort_tile_list<1>(list, cnt, sortBits, order, sortTmp);
-    else if (kSpreadMax <= 512 || cnt <= 512) sort_tile_list<2>(list, cnt, sortBits, order, sortTmp);
-    else sort_tile_list<(kSpreadMax + 255) / 256>(list, cnt, sortBits, order, sortTmp);
-    __syncthreads();
+    __shared__ __align__(16) double fac[kSpreadChunk][10];  // A[5] / 16, B[5]
+    __shared__ double2 sF[kSpreadChunk];
+    __shared__ int code[kSpreadChunk];
+    __shared__ int order[kSpreadMax];               // sorted membrane indices
+    __shared__ unsigned wlist[8][kSpreadChunk];     // per warp: pack_stencil and the entry's place << 24
+    {
+        int* raw = (int*)fac;  // free until the factors are formed
+        static_assert(sizeof(fac) >= (kSpreadMax + 3) * sizeof(int), "the unsorted list fits the factors' place");
+        const int* list = t.slots + (size_t)tile * kTileSlots;
+        const int cnt4 = (cnt + 3) & ~3;
+        for (int k = threadIdx.x; k < cnt4; k += blockDim.x) raw[k] = k < cnt ? list[k] : 0x7fffffff;
+        __syncthreads();
+        for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
+            const int v = raw[k];
+            int r = 0;
+            for (int j = 0; j < cnt4; j += 4) {
+                const int4 w = *(const int4*)(raw + j);
+                r += (w.x < v) + (w.y < v) + (w.z < v) + (w.w < v);
+            }
+            order[r] = v;
+        }
+        __syncthreads();
+    }
     const int tx = tile % t.tilesX, ty = tile / t.tilesX;
     const int tileX0 = tx * kTile, tileY0 = ty * kTile;
     const double halfPi = M_PI / 2.0;
-    for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
-        const int i = order[k];
-        const double X = m.x[i], Y = m.y[i];
-        sfx[k] = m.fx[i];
-        sfy[k] = m.fy[i];
-        Stencil sc;
-        stencil_range(m.bx[i], m.by[i], nx, ny, sc);
-        code[k] = pack_stencil(sc, tileX0, tileY0);
-        double* f = fac + 10 * k;
-#pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            f[q] = 1.0 + fast_cos(halfPi * ((double)(sc.x0 + q) - X));
-            f[5 + q] = 1.0 + fast_cos(halfPi * ((double)(sc.y0 + q) - Y));
-        }
-    }
-    __syncthreads();
-    // per-warp list of the entries whose stencil rows meet the warp's rows
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int wy0 = (warp << 1) + 4;  // local rows + 4
-    unsigned short* wl = wlist + warp * kSpreadMax;
-    int wn = 0;
-    for (int k0 = 0; k0 < cnt; k0 += 32) {
-        const int k = k0 + lane;
-        bool rel = false;
-        if (k < cnt) {
-            const int c = code[k];
-            const int oy = (c >> 8) & 0xff, hy = (c >> 20) & 0xf;
-            rel = !(oy + hy < wy0 || oy > wy0 + 1);
-        }
-        const unsigned bal = __ballot_sync(0xffffffffu, rel);
-        if (rel) wl[wn + __popc(bal & ((1u << lane) - 1u))] = (unsigned short)k;
-        wn += __popc(bal);
-    }
-    __syncwarp();
-    const int lx = lane & 15, ly = threadIdx.x >> 4;
-    const int x = tileX0 + lx, y = tileY0 + ly;
+    const int wy0 = 2 * warp;  // the warp's first row in the tile
+    const int lx = lane & 15, ly = wy0 + (lane >> 4);
     double ax = 0.0, ay = 0.0;
-    for (int e = 0; e < wn; ++e) {
-        const int k = wl[e];
-        const int c = code[k];
-        const int ox = c & 0xff, oy = (c >> 8) & 0xff, hx = (c >> 16) & 0xf, hy = (c >> 20) & 0xf;
-        const int dx = lx + 4 - ox, dy = ly + 4 - oy;
-        bool hit;
-        if (hx == 3 && hy == 3) {
-            hit = (unsigned)dx < 4u && (unsigned)dy < 4u;
+    for (int c0 = 0; c0 < cnt; c0 += kSpreadChunk) {
+        const int nc = min(kSpreadChunk, cnt - c0);
+        // two threads per entry: the column factors and the row factors
+        for (int k2 = threadIdx.x; k2 < 2 * nc; k2 += blockDim.x) {
+            const int k = k2 >> 1, half = k2 & 1;
+            const int i = order[c0 + k];
+            Stencil sc;
+            stencil_range(m.bx[i], m.by[i], nx, ny, sc);
+            const double X = half ? m.y[i] : m.x[i];
+            const int o = half ? sc.y0 : sc.x0;
+            const double scale = half ? 1.0 : 1.0 / 16.0;
+            double* f = &fac[k][5 * half];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) f[q] = (1.0 + fast_cos(halfPi * ((double)(o + q) - X))) * scale;
+            reinterpret_cast<double*>(sF + k)[half] = half ? m.fy[i] : m.fx[i];
+            if (half == 0) code[k] = pack_stencil(sc, tileX0, tileY0);
+        }
+        __syncthreads();
+        // the entries whose stencil rows meet the warp's rows, in order
+        int wn = 0;
+        bool wide = false;
+        for (int k0 = 0; k0 < nc; k0 += 32) {
+            const int k = k0 + lane;
+            bool rel = false;
+            int c = 0;
+            if (k < nc) {
+                c = code[k];
+                const int oy = ((c >> 8) & 0xff) - 4, hy = (c >> 20) & 0xf;
+                rel = oy + hy >= wy0 && oy <= wy0 + 1;
+                wide |= rel && (c >> 16) != 0x33;
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, rel);
+            if (rel) wlist[warp][wn + __popc(bal & ((1u << lane) - 1u))] = (unsigned)c | ((unsigned)k << 24);
+            wn += __popc(bal);
+        }
+        wide = __any_sync(0xffffffffu, wide);
+        __syncwarp();
+        if (!wide) {
+#pragma unroll 4
+            for (int e = 0; e < wn; ++e) {
+                const unsigned c = wlist[warp][e];
+                const unsigned k = c >> 24;
+                const int dx = lx + 4 - (int)(c & 0xffu), dy = ly + 4 - (int)((c >> 8) & 0xffu);
+                const bool hit = (unsigned)dx < 4u && (unsigned)dy < 4u;
+                const double dl = fac[k][dx & 3] * fac[k][5 + (dy & 3)];
+                const double2 F = sF[k];
+                const double sx = ax + F.x * dl, sy = ay + F.y * dl;
+                if (hit) {
+                    ax = sx;
+                    ay = sy;
+                }
+            }
         } else {
-            Stencil sc{ox - 4 + tileX0, ox - 4 + tileX0 + hx, oy - 4 + tileY0, oy - 4 + tileY0 + hy};
-            hit = in_stencil(sc, x, y);
+            // stencils of five columns or rows among them: the nodes bound by
+            // the slots' last writers
+            for (int e = 0; e < wn; ++e) {
+                const unsigned c = wlist[warp][e];
+                const int k = c >> 24;
+                const int ox = (int)(c & 0xffu) - 4, oy = (int)((c >> 8) & 0xffu) - 4;
+                const Stencil sc{ox + tileX0, ox + tileX0 + (int)((c >> 16) & 0xfu), oy + tileY0,
+                                 oy + tileY0 + (int)((c >> 20) & 0xfu)};
+                const int x = tileX0 + lx, y = tileY0 + ly;
+                if (!in_stencil(sc, x, y)) continue;
+                const double dl = fac[k][x - sc.x0] * fac[k][5 + y - sc.y0];
+                ax += sF[k].x * dl;
+                ay += sF[k].y * dl;
+            }
         }
-        if (hit) {
-            const double* f = fac + 10 * k;
-            const double dl = (f[dx] * f[5 + dy]) / 16.0;
-            ax += sfx[k] * dl;
-            ay += sfy[k] * dl;
-        }
+        __syncthreads();
     }
+    const int x = tileX0 + lx, y = tileY0 + ly;
     if (x >= nx || y >= ny) return;
     const size_t n = (size_t)y * nx + x;
     force[n] = (Real)ax;
@@ -483,7 +480,7 @@ __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDe
     pdl_wait();
     if (st->halt) return;
     const int tile = blockIdx.x;
-    const int cnt = min(t.count[tile], kTileSlots);
+    const int cnt = min(take_tile_count(t, tile), kTileSlots);
     if (cnt == 0) return;
     // each 64-bit fixed-point sum is kept as a signed high part (bits 22..63)
     // and an unsigned low part (bits 0..21), each summed with 32-bit integer
@@ -570,27 +567,17 @@ __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDe
 template <typename Real>
 void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny, size_t L, Status* st,
                    unsigned iteration, cudaStream_t s, bool slotsFilled) {
-    if (!slotsFilled) cudaMemsetAsync(t.count, 0, sizeof(int) * (t.nTiles + 1), s);
-    if (m.Mcap == 0) return;
-    const int blocks = (m.Mcap + 127) / 128;
-    if constexpr (sizeof(Real) == 4) {
-        // one pass into fixed per-tile slots (done by the force kernel when
-        // slotsFilled), then the fixed-point scatter
-        if (!slotsFilled) launch_pdl(tile_slot_kernel, blocks, 128, 0, s, m, t, nx, ny, st);
-        launch_pdl(spread_fixed_kernel, t.nTiles, 256, 0, s, m, t, (float*)force, nx, ny, L, st);
-    } else {
-        // exact lists (count, scan, fill), then the ordered gather
-        cudaMemsetAsync(t.fill, 0, sizeof(int) * t.nTiles, s);
-        launch_pdl(tile_count_kernel, blocks, 128, 0, s, m, t, nx, ny, st, 0);
-        cub::DeviceScan::ExclusiveSum(t.scanTmp, t.scanTmpBytes, t.count, t.start, t.nTiles + 1, s);
-        launch_pdl(tile_count_kernel, blocks, 128, 0, s, m, t, nx, ny, st, 1);
-        int bits = 1;
-        while ((1 << bits) < m.Mcap + 1 && bits < 31) ++bits;
-        launch_pdl(spread_kernel<Real, kSpreadSmall, 0>, t.nTiles, 256, spread_smem(kSpreadSmall), s, m, t, force, nx,
-                   ny, L, st, bits);
-        launch_pdl(spread_kernel<Real, kSpreadLarge, kSpreadSmall + 1>, t.nTiles, 256, spread_smem(kSpreadLarge), s, m,
-                   t, force, nx, ny, L, st, bits);
+    if (m.Mcap == 0) {
+        cudaMemsetAsync(t.active, 0, sizeof(int) * t.nTiles, s);
+        return;
     }
+    // fixed per-tile slot lists (filled by the force kernel when slotsFilled),
+    // then the sums: FP64 in id order, FP32-shifted in exact fixed point
+    if (!slotsFilled) launch_pdl(tile_slot_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, t, nx, ny, st);
+    if constexpr (sizeof(Real) == 4)
+        launch_pdl(spread_fixed_kernel, t.nTiles, 256, 0, s, m, t, (float*)force, nx, ny, L, st);
+    else
+        launch_pdl(spread_kernel<Real>, t.nTiles, 256, 0, s, m, t, force, nx, ny, L, st);
 }
 template void launch_spread<double>(const MembraneDev&, TileDev&, double*, int, int, size_t, Status*, unsigned,
                                     cudaStream_t, bool);
@@ -1881,8 +1868,6 @@ void launch_motion_adjoint(const double* X, const double* Y, const double* fx, c
 namespace lbib {
 
 void init_kernel_attributes() {
-    cudaFuncSetAttribute(spread_kernel<double, kSpreadSmall, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spread_smem(kSpreadSmall));
-    cudaFuncSetAttribute(spread_kernel<double, kSpreadLarge, kSpreadSmall + 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)spread_smem(kSpreadLarge));
     cudaFuncSetAttribute(reinit_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReinitSmem);
     cudaFuncSetAttribute(reinit_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReinitSmem);
     init_kernel_attributes_topology();

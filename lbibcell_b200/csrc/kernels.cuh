@@ -122,14 +122,9 @@ struct CrossDev {
 // Tiles for force spreading.
 struct TileDev {
     int tilesX, tilesY, nTiles;
-    int* count;     // nTiles
-    int* fill;      // nTiles
-    int* start;     // nTiles + 1
-    int* list;      // capacity entries
-    int cap;
-    void* scanTmp;  // CUB temporary storage
-    size_t scanTmpBytes;
-    int* slots;     // FP32-shifted runs: nTiles x kTileSlots membrane indices (unordered)
+    int* count;     // nTiles: entries of each tile's list while it is filled; zero between spreads
+    int* active;    // nTiles: entries the last spread used (0: the force there is zero)
+    int* slots;     // nTiles x kTileSlots membrane indices (unordered)
 };
 
 // Entries a tile's slot list holds (the fixed-point spread's 32-bit low parts
@@ -181,8 +176,8 @@ void launch_init32(float* f, float* g, float* u, int nS, size_t L, double tauF, 
 
 // Membrane pipeline.  `Real` is the lattice precision (velocity / force planes).
 template <typename Real>
-// `tiles`: also fill the FP32-shifted spread's per-tile slot lists (then call
-// launch_spread with slotsFilled).
+// `tiles`: also fill the spread's per-tile slot lists (then call launch_spread
+// with slotsFilled).
 void launch_force_eval(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s, bool begin = false,
                        TileDev* tiles = nullptr, int nx = 0, int ny = 0);
 template <typename Real>

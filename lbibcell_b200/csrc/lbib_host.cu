@@ -454,7 +454,7 @@ Handle::~Handle() {
     fr(m.prev); fr(m.next); fr(m.ca); fr(m.cb); fr(m.cdom); fr(m.foff); fr(m.ftype); fr(m.fpartner); fr(m.fpar);
     fr(m.ringStart); fr(m.ringNode); fr(m.ringDom);
     fr(outPos); fr(inPos); fr(target); fr(areaAcc);  // area lives in the status allocation
-    fr(tiles.count); fr(tiles.fill); fr(tiles.start); fr(tiles.list); fr(tiles.scanTmp); fr(tiles.slots);
+    fr(tiles.count); fr(tiles.active); fr(tiles.slots);
     fr(cross.bnDist); fr(cross.bnConn); fr(cross.bnDom); fr(cross.wDom); fr(cross.mark);
     fr(cross.changedNode); fr(cross.changedDom); fr(cross.perturbList); fr(cross.reinitDone); fr(cross.waitList);
     fr(cross.nWait);
@@ -949,7 +949,7 @@ static void read_out(Handle& h, std::vector<ReadPart> parts) {
     a.g = h.g[h.cur];
     a.u = h.u;
     a.force = h.force;
-    a.tileCount = h.tiles.count;
+    a.tileCount = h.tiles.active;
     a.tilesX = h.tiles.tilesX;
     a.dom = h.dom;
     a.ctypeTab = h.ctypeTab;
@@ -1140,7 +1140,7 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
         auto fr = [](void* p) { if (p) cudaFree(p); };
         fr(h.m.x); fr(h.m.y); fr(h.m.ox); fr(h.m.oy); fr(h.m.vx); fr(h.m.vy); fr(h.m.fx); fr(h.m.fy); fr(h.m.bx); fr(h.m.by);
         fr(h.m.id); fr(h.m.prev); fr(h.m.next); fr(h.outPos); fr(h.inPos); fr(h.cross.perturbList);
-        fr(h.m.foff); fr(h.m.ringNode); fr(h.tiles.list);
+        fr(h.m.foff); fr(h.m.ringNode);
         fr(h.td.nflag); fr(h.td.nrank); fr(h.td.dalt); fr(h.td.id2); fr(h.td.prev2); fr(h.td.next2);
         fr(h.td.inConn); fr(h.td.outConn); fr(h.td.removed); fr(h.td.ncA); fr(h.td.ncB); fr(h.td.ncDom);
         fr(h.td.ncDesc); fr(h.td.ncAlive); fr(h.td.members); fr(h.td.succ); fr(h.td.dist); fr(h.td.rngList);
@@ -1164,8 +1164,6 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
         h.cross.perturbList = dalloc<int>(n); h.cross.perturbCap = n;
         h.m.foff = dalloc<int>(n + 1);
         h.m.ringNode = dalloc<int>(n);
-        h.tiles.cap = 4 * n;
-        h.tiles.list = dalloc<int>(h.tiles.cap);
     }
     if (grow(C, h.Ccap)) {
         auto fr = [](void* p) { if (p) cudaFree(p); };
@@ -1351,7 +1349,7 @@ static LatticeArgs<Real> lattice_args(Handle& h, unsigned iteration, int parity)
     a.gout = (Real*)h.g[1 - parity];
     a.u = (Real*)h.u;
     a.force = (const Real*)h.force;
-    a.tileCount = h.tiles.count;
+    a.tileCount = h.tiles.active;
     a.tilesX = h.tiles.tilesX;
     a.dom = h.dom;
     bool area = false;
@@ -1407,16 +1405,15 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
     long long nl = 0;
     if (fromStage <= ST_FORCE) {
         // the step's counters are reset by the force kernel, or alone without a
-        // membrane; in FP32-shifted runs the force kernel also fills the
-        // spread's per-tile lists
-        if (hasM) launch_force_eval<Real>(h.m, h.st, it, s, true, sizeof(Real) == 4 ? &h.tiles : nullptr, h.nx, h.ny);
+        // membrane; the force kernel also fills the spread's per-tile lists
+        if (hasM) launch_force_eval<Real>(h.m, h.st, it, s, true, &h.tiles, h.nx, h.ny);
         else launch_pdl(step_begin_kernel, 1, 1, 0, s, h.st);
         nl += 1;
     }
     if (fromStage <= ST_SPREAD) {
-        const bool filled = sizeof(Real) == 4 && hasM && fromStage <= ST_FORCE;
+        const bool filled = hasM && fromStage <= ST_FORCE;
         launch_spread<Real>(h.m, h.tiles, (Real*)h.force, h.nx, h.ny, h.L, h.st, it, s, filled);
-        nl += hasM ? (sizeof(Real) == 8 ? 6 : (filled ? 1 : 2)) : 0;
+        nl += hasM ? (filled ? 1 : 2) : 0;
     }
     if (fromStage <= ST_COLLIDE) {
         if (evCollideA) cudaEventRecord(evCollideA, s);
@@ -2082,15 +2079,11 @@ static void create(Handle& h, const std::string& params, const std::string& geom
     h.tiles.tilesX = (h.nx + kTile - 1) / kTile;
     h.tiles.tilesY = (h.ny + kTile - 1) / kTile;
     h.tiles.nTiles = h.tiles.tilesX * h.tiles.tilesY;
-    // count has one extra zero entry: the exclusive scan over nTiles + 1
-    // items yields start[nTiles] = total
-    h.tiles.count = dalloc<int>(h.tiles.nTiles + 1);
-    h.tiles.fill = dalloc<int>(h.tiles.nTiles);
-    h.tiles.start = dalloc<int>(h.tiles.nTiles + 1);
-    CK(cudaMemsetAsync(h.tiles.count, 0, sizeof(int) * (h.tiles.nTiles + 1), h.stream));
-    cub::DeviceScan::ExclusiveSum(nullptr, h.tiles.scanTmpBytes, h.tiles.count, h.tiles.start, h.tiles.nTiles + 1, h.stream);
-    CK(cudaMalloc(&h.tiles.scanTmp, std::max<size_t>(h.tiles.scanTmpBytes, 16)));
-    if (h.precision == LBIB_FP32_SHIFTED) h.tiles.slots = dalloc<int>((size_t)h.tiles.nTiles * kTileSlots);
+    h.tiles.count = dalloc<int>(h.tiles.nTiles);
+    h.tiles.active = dalloc<int>(h.tiles.nTiles);
+    h.tiles.slots = dalloc<int>((size_t)h.tiles.nTiles * kTileSlots);
+    CK(cudaMemsetAsync(h.tiles.count, 0, sizeof(int) * h.tiles.nTiles, h.stream));
+    CK(cudaMemsetAsync(h.tiles.active, 0, sizeof(int) * h.tiles.nTiles, h.stream));
 
     // crossing planes
     h.cross.bnDist = dalloc<unsigned long long>(4 * h.L);
@@ -2877,7 +2870,7 @@ int lbib_upload_lattice(lbib_handle* hh, const double* f, const double* g, const
         put(h.force, v);
         // mark every tile active so that the lattice kernels read the field
         std::vector<int> ones(h.tiles.nTiles, 1);
-        CK(cudaMemcpyAsync(h.tiles.count, ones.data(), sizeof(int) * ones.size(), cudaMemcpyHostToDevice, h.stream));
+        CK(cudaMemcpyAsync(h.tiles.active, ones.data(), sizeof(int) * ones.size(), cudaMemcpyHostToDevice, h.stream));
         CK(cudaStreamSynchronize(h.stream));
     }
     API_END

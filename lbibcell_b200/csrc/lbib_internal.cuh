@@ -268,7 +268,7 @@ struct LatticeArgs {
     Real* gout;           // S*5*L
     Real* u;              // 2*L
     const Real* force;    // 2*L (valid where tileCount > 0)
-    const int* tileCount; // per 16x16 tile: membrane stencils overlapping it
+    const int* tileCount; // per 16x16 tile: membrane stencils overlapping it (TileDev::active)
     int tilesX;
     const uint32_t* dom;  // L
     const double* massTab;     // per-domain rhoToAdd (nullptr: none)
