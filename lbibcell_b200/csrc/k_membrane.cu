@@ -754,35 +754,6 @@ void launch_force_adjoint(const MembraneDev& m, const double* G, int nx, int ny,
     launch_pdl(force_adjoint_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, G, nx, ny, L, gfx, gfy);
 }
 
-// Connection::perturbConnection's tests (Connection.cpp:339, 363).
-// Connections whose end points share an x or a y to within EPSILON
-// (Connection::perturbConnection's tests, Connection.cpp:339-340, 363-364) are
-// counted and listed (up to cap); the crossing kernel, the next, raises the
-// halt, so that every block here sees the same halt word and the list is
-// complete.
-// The kernel first raises the halt for the nodes that the move listed.
-__global__ void perturb_conn_kernel(MembraneDev m, Status* st, int* list, int cap) {
-    pdl_wait();
-    if (st->halt) return;
-    if (st->nPerturbNode > 0) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
-        return;
-    }
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.topo->C) return;
-    const int a = m.ca[c], b = m.cb[c];
-    if (fabs(m.x[a] - m.x[b]) < kEPSILON || fabs(m.y[a] - m.y[b]) < kEPSILON) {
-        const int k = atomicAdd(&st->nPerturbConn, 1);
-        if (k < cap) list[k] = c;
-    }
-}
-
-void launch_perturb_conn_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s, int* list,
-                               int cap) {
-    if (m.Mcap == 0 && m.Ccap == 0) return;
-    launch_pdl(perturb_conn_kernel, m.Ccap > 0 ? (m.Ccap + 127) / 128 : 1, 128, 0, s, m, st, list, cap);
-}
-
 // ---------------------------------------------------------------------------
 // Crossings: three passes over the connections.
 //   pass 0: closest distance per (node, slot) by atomicMin on the distance bits
@@ -800,11 +771,17 @@ __device__ __forceinline__ int slot_code(int d) {  // E,N,W,S -> 0..3
 // Pass 0: every crossing of a connection with a lattice line is a candidate
 // boundary node for one (node, slot) key.  The closest distance per key is
 // found by atomicMin on the distance's bits; each candidate is recorded for
-// passes 1 and 2 and for the reset of its key at the end of the step.  A warp
-// reserves its records with one atomic.  A connection may be long (the
-// cut across a cell that a division adds, until remeshing splits it): the
-// loops run over the lattice lines between its end points, which the bounds
-// test below keeps on the lattice.
+// passes 1 and 2 and for the reset of its key at the end of the step.
+//
+// Almost every connection meets at most one vertical and one horizontal line:
+// its (up to four) records are formed once, in registers.  A connection may be
+// long (the cut across a cell that a division adds, until remeshing splits
+// it): the general form enumerates the lattice lines between its end points,
+// which the bounds test below keeps on the lattice, once to count and once to
+// emit.  A block reserves its records with one atomic (a warp did: 4,700 of
+// them on one address for 150k connections).  12.5 -> XX us at 150k
+// connections, 3.8 -> XX us for one cell; with the perturbation test, a kernel
+// of its own before (3.3 and 2.1 us), inside.
 
 struct CrossRec {
     uint32_t key;
@@ -821,24 +798,6 @@ __device__ __forceinline__ bool make_record(int nx, int ny, int px, int py, int 
     r.key = (uint32_t)(node * 4 + slot_code(dirSlot));
     r.dom = bdom;
     return true;
-}
-
-// Exclusive prefix of `count` over the active lanes plus one atomicAdd per warp.
-__device__ __forceinline__ int warp_reserve(int* counter, int count) {
-    const unsigned act = __activemask();
-    const int lane = threadIdx.x & 31;
-    int incl = count;
-    for (int off = 1; off < 32; off <<= 1) {
-        const int v = __shfl_up_sync(act, incl, off);
-        if (lane >= off && ((act >> (lane - off)) & 1u)) incl += v;
-    }
-    const int last = 31 - __clz(act);
-    const int total = __shfl_sync(act, incl, last);
-    const int leader = __ffs(act) - 1;
-    int base = 0;
-    if (lane == leader && total > 0) base = atomicAdd(counter, total);
-    base = __shfl_sync(act, base, leader);
-    return base + incl - count;
 }
 
 // Calls fn(k, record) for the candidate records of connection cn in a fixed
@@ -892,41 +851,144 @@ __device__ __forceinline__ int for_each_record(const MembraneDev& m, int cn, int
     return k;
 }
 
-__global__ void crossings_kernel(MembraneDev m, CrossDev c, int nx, int ny, Status* st) {
+// `check`: the first kernel after the move.  It raises the halt for the nodes
+// that the move listed for the host's perturbation, and lists the connections
+// whose end points share an x or a y to within EPSILON
+// (Connection::perturbConnection's tests, Connection.cpp:339-340, 363-364) in
+// `perturb` (up to perturbCap) instead of crossing them; the next kernel raises
+// the halt for those, so that every block here sees the same halt word and the
+// list is complete.  The halted step's records are reset like any other's
+// (domain_fill_kernel), and the crossings run again once the host is done.
+constexpr int kCrossBlock = 128;
+__global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, CrossDev c, int nx, int ny, Status* st,
+                                                                int check, int* perturb, int perturbCap) {
     pdl_wait();
     if (st->halt) return;
-    if (st->nPerturbConn > 0) {
-        // connections to perturb first (perturb_conn_kernel): the host does it
-        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_PERTURB_CONN);
+    if (check && st->nPerturbNode > 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
         return;
     }
-    const int cn = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool live = cn < m.topo->C;
+    const int cn = blockIdx.x * kCrossBlock + threadIdx.x;
     int nrec = 0;
-    if (live) {
-        nrec = for_each_record(m, cn, nx, ny, st, true, [](int, const CrossRec&) {});
-        if (nrec < 0) nrec = 0;
-    }
-    // records of this step (they also list the keys to reset at the end of
-    // the step) and the closest distance per key
-    const int rb = warp_reserve(&st->pad[2], nrec);
-    if (nrec > 0) {
-        for_each_record(m, cn, nx, ny, st, false, [&](int k, const CrossRec& r) {
-            const int idx = rb + k;
-            if (idx < c.recCap) {
-                c.recKey[idx] = r.key; c.recConn[idx] = (uint32_t)cn; c.recDom[idx] = r.dom; c.recDist[idx] = r.bits;
-            } else {
-                raise_error(st, ERR_CAPACITY, cn, ST_CROSSINGS);
+    bool simple = false;
+    CrossRec r[4];
+    bool have[4] = {false, false, false, false};
+    if (cn < m.topo->C) {
+        const int a = m.ca[cn], b = m.cb[cn];
+        const uint32_t D = m.cdom[cn];
+        const double x1 = m.x[a], y1 = m.y[a], x2 = m.x[b], y2 = m.y[b];
+        if (check && (fabs(x1 - x2) < kEPSILON || fabs(y1 - y2) < kEPSILON)) {
+            const int k = atomicAdd(&st->nPerturbConn, 1);
+            if (k < perturbCap) perturb[k] = cn;
+        } else {
+            const double maxX = x1 < x2 ? x2 : x1, maxY = y1 < y2 ? y2 : y1;
+            const double minX = x2 < x1 ? x2 : x1, minY = y2 < y1 ? y2 : y1;
+            const double mm = (y2 - y1) / (x2 - x1);
+            const int iv = (int)ceil(minX), ih = (int)ceil(minY);
+            const int nv = (int)floor(maxX) - iv + 1, nh = (int)floor(maxY) - ih + 1;
+            // one line each way at most, inside the lattice with room to spare
+            simple = isfinite(mm) && minX >= 1.0 && maxX <= nx - 2.0 && minY >= 1.0 && maxY <= ny - 2.0 && nv <= 1 &&
+                     nh <= 1;
+            if (simple) {
+                const double nn = y1 - mm * x1;
+                if (nv == 1) {
+                    // fluidS gets its N slot, fluidN its S slot (Connection.cpp:273-279)
+                    const double yc = mm * iv + nn;
+                    const bool eastward = x1 < x2;
+                    have[0] = make_record(nx, ny, iv, (int)floor(yc), N, (double)iv, yc, eastward ? 0u : D, r[0]);
+                    have[1] = make_record(nx, ny, iv, (int)ceil(yc), S, (double)iv, yc, eastward ? D : 0u, r[1]);
+                }
+                if (nh == 1) {
+                    // fluidW gets its E slot, fluidE its W slot (Connection.cpp:307-313)
+                    const double xc = (ih - nn) / mm;
+                    const bool southward = y1 > y2;
+                    have[2] = make_record(nx, ny, (int)floor(xc), ih, E, xc, (double)ih, southward ? 0u : D, r[2]);
+                    have[3] = make_record(nx, ny, (int)ceil(xc), ih, W, xc, (double)ih, southward ? D : 0u, r[3]);
+                }
+                nrec = have[0] + have[1] + have[2] + have[3];
+                // a crossing off the lattice: the general form reports it
+                simple = nrec == 2 * (max(nv, 0) + max(nh, 0));
             }
-            atomicMin(&c.bnDist[r.key], r.bits);
-        });
+            if (!simple) {
+                nrec = for_each_record(m, cn, nx, ny, st, true, [](int, const CrossRec&) {});
+                if (nrec < 0) nrec = 0;
+            }
+        }
+    }
+    // the block's records, in any order (they also list the keys to reset at
+    // the end of the step), and the closest distance per key
+    __shared__ int warpSum[kCrossBlock / 32], blockBase;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int incl = nrec;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, off);
+        if (lane >= off) incl += v;
+    }
+    if (lane == 31) warpSum[warp] = incl;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int total = 0;
+#pragma unroll
+        for (int w = 0; w < kCrossBlock / 32; ++w) {
+            const int v = warpSum[w];
+            warpSum[w] = total;
+            total += v;
+        }
+        blockBase = total > 0 ? atomicAdd(&st->pad[2], total) : 0;
+    }
+    __syncthreads();
+    if (nrec == 0) return;
+    const int rb = blockBase + warpSum[warp] + incl - nrec;
+    auto emit = [&](int k, const CrossRec& q) {
+        const int idx = rb + k;
+        if (idx < c.recCap) {
+            c.recKey[idx] = q.key; c.recConn[idx] = (uint32_t)cn; c.recDom[idx] = q.dom; c.recDist[idx] = q.bits;
+        } else {
+            raise_error(st, ERR_CAPACITY, cn, ST_CROSSINGS);
+        }
+        atomicMin(&c.bnDist[q.key], q.bits);
+    };
+    if (simple) {
+        int k = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (have[j]) emit(k++, r[j]);
+    } else {
+        for_each_record(m, cn, nx, ny, st, false, emit);
     }
 }
 
+// GeometryHandler::connectGeometryNodesToPhysicalNodes for one node
+// (GeometryHandler.cpp:608-644): a node that left its previous unit cell
+// (GeometryNode::isUpdateNeeded, GeometryNode.cpp:256-261, Rectangle.cpp
+// pointWithinBounds) is bound again from its current position, after the
+// edge test; the others keep their binding.
+__device__ __forceinline__ void edge_check_node(const MembraneDev& m, int i, int nx, int ny, Status* st, int stage) {
+    const double X = m.x[i], Y = m.y[i], ox = m.ox[i], oy = m.oy[i];
+    const bool within = (X >= floor(ox)) && (X < ceil(ox)) && (Y <= ceil(oy)) && (Y > floor(oy));
+    if (within) return;
+    m.bx[i] = X;
+    m.by[i] = Y;
+    if (X - 2.0 < 0) raise_error(st, ERR_EDGE_W, i, stage);
+    else if (Y - 2.0 < 0) raise_error(st, ERR_EDGE_S, i, stage);
+    else if (X + 2.0 > nx) raise_error(st, ERR_EDGE_E, i, stage);
+    else if (Y + 2.0 > ny) raise_error(st, ERR_EDGE_N, i, stage);
+}
+
 // Pass 1: among records at the closest distance, the earliest connection.
-__global__ void cross_tie_kernel(CrossDev c, Status* st) {
+// And, over the same grid, GeometryHandler::connectGeometryNodesToPhysicalNodes'
+// edge test of the moved nodes.  The kernel first raises the halt for the
+// connections that pass 0 listed for the host's perturbation.
+__global__ void cross_tie_kernel(CrossDev c, MembraneDev m, int nx, int ny, Status* st) {
     pdl_wait();
     if (st->halt) return;
+    if (st->nPerturbConn > 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_PERTURB_CONN);
+        return;
+    }
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.topo->M; i += gridDim.x * blockDim.x)
+        edge_check_node(m, i, nx, ny, st, ST_CROSSINGS);
     const int n = min(st->pad[2], c.recCap);
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const uint32_t key = c.recKey[r];
@@ -970,23 +1032,6 @@ __device__ __forceinline__ void record_noflux(const MembraneDev& m, CrossDev& c,
     if (k < c.nfCap) c.nfKeys[k] = key;
 }
 
-// GeometryHandler::connectGeometryNodesToPhysicalNodes for one node
-// (GeometryHandler.cpp:608-644): a node that left its previous unit cell
-// (GeometryNode::isUpdateNeeded, GeometryNode.cpp:256-261, Rectangle.cpp
-// pointWithinBounds) is bound again from its current position, after the
-// edge test; the others keep their binding.
-__device__ __forceinline__ void edge_check_node(const MembraneDev& m, int i, int nx, int ny, Status* st, int stage) {
-    const double X = m.x[i], Y = m.y[i], ox = m.ox[i], oy = m.oy[i];
-    const bool within = (X >= floor(ox)) && (X < ceil(ox)) && (Y <= ceil(oy)) && (Y > floor(oy));
-    if (within) return;
-    m.bx[i] = X;
-    m.by[i] = Y;
-    if (X - 2.0 < 0) raise_error(st, ERR_EDGE_W, i, stage);
-    else if (Y - 2.0 < 0) raise_error(st, ERR_EDGE_S, i, stage);
-    else if (X + 2.0 > nx) raise_error(st, ERR_EDGE_E, i, stage);
-    else if (Y + 2.0 > ny) raise_error(st, ERR_EDGE_N, i, stage);
-}
-
 __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom, int nx, int ny, Status* st) {
     pdl_wait();
     if (st->halt) return;
@@ -1022,10 +1067,6 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
             }
         }
     }
-    // GeometryHandler::connectGeometryNodesToPhysicalNodes' edge test of the
-    // moved nodes, over the same grid
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.topo->M; i += gridDim.x * blockDim.x)
-        edge_check_node(m, i, nx, ny, st, ST_CROSSINGS);
 }
 
 // Clears the previous step's no-flux boundary nodes (after the stream-collide
@@ -1064,24 +1105,28 @@ __global__ void edge_check_kernel(MembraneDev m, int nx, int ny, Status* st, int
 
 template <typename Real>
 void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, size_t L, Status* st,
-                      unsigned iteration, cudaStream_t s) {
-    if (m.Ccap == 0) return;
-    const int blocks = (m.Ccap + 127) / 128;
+                      unsigned iteration, cudaStream_t s, bool check, int* perturb, int perturbCap) {
+    const int blocks = (m.Ccap + kCrossBlock - 1) / kCrossBlock;
+    if (m.Ccap == 0) {  // nodes without connections: the halt of the listed nodes alone
+        if (check && m.Mcap > 0)
+            launch_pdl(crossings_kernel, 1, kCrossBlock, 0, s, m, c, nx, ny, st, 1, perturb, perturbCap);
+        return;
+    }
     if (c.nfTab != nullptr) launch_pdl(noflux_reset_kernel, 1, 1024, 0, s, c);
     if (c.bounceW != nullptr) launch_pdl(bounce_reset_kernel, 1, 1024, 0, s, c);
     // the record count (st->pad[2]) is zero here: cleared with the status
     // word before a run and by the first kernel of each step
-    launch_pdl(crossings_kernel, blocks, 128, 0, s, m, c, nx, ny, st);
+    launch_pdl(crossings_kernel, blocks, kCrossBlock, 0, s, m, c, nx, ny, st, check ? 1 : 0, perturb, perturbCap);
     // grid-stride over the step's records (their count is known on the device
     // only): 8 blocks per SM, so that each thread's chain of dependent loads
     // overlaps many others
-    launch_pdl(cross_tie_kernel, 148 * 8, 256, 0, s, c, st);
+    launch_pdl(cross_tie_kernel, 148 * 8, 256, 0, s, c, m, nx, ny, st);
     launch_pdl(cross_win_kernel, 148 * 8, 256, 0, s, c, m, dom, nx, ny, st);
 }
 template void launch_crossings<double>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
-                                       unsigned, cudaStream_t);
+                                       unsigned, cudaStream_t, bool, int*, int);
 template void launch_crossings<float>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
-                                      unsigned, cudaStream_t);
+                                      unsigned, cudaStream_t, bool, int*, int);
 
 void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s) {
     if (m.Mcap == 0) return;

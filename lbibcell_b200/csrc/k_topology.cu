@@ -713,7 +713,7 @@ __global__ void ring_done_kernel(MembraneDev m, TopoDev t) {
     if (d == 0) m.topo->changed = 0;
 }
 
-// The listed connections to perturb (perturb_conn_kernel, t.rngList), each
+// The listed connections to perturb (crossings_kernel, t.rngList), each
 // with its place in its cell's ring walk (the rings are current: the host
 // rebuilds them first when the topology changed).  The walk visits the
 // connection leaving the ring's last node first (the domain's first

@@ -186,11 +186,12 @@ void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny
 template <typename Real>
 void launch_interp_move(const MembraneDev& m, const Real* u, int nx, int ny, size_t L, CrossDev& c, Status* st,
                         unsigned iteration, cudaStream_t s);
-void launch_perturb_conn_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s, int* list,
-                               int cap);
+// `check`: first raise the halts of the move's listed nodes and of connections
+// that need the host's perturbation (listed in perturb[0..perturbCap)).
 template <typename Real>
 void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, size_t L, Status* st,
-                      unsigned iteration, cudaStream_t s);
+                      unsigned iteration, cudaStream_t s, bool check = false, int* perturb = nullptr,
+                      int perturbCap = 0);
 template <typename Real>
 void launch_reinit(CrossDev& c, uint32_t* dom, Real* g, const Real* u, int nS, const SpeciesConst* sp,
                    const double* srcTab, int nDomains, const uint32_t* ctypeTab, int cellTypesCopied, int nx,

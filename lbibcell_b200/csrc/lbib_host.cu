@@ -1431,12 +1431,10 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
         launch_interp_move<Real>(h.m, (const Real*)h.u, h.nx, h.ny, h.L, h.cross, h.st, it, s);
         nl += hasM;
     }
-    if (fromStage <= ST_PERTURB_CONN) {
-        launch_perturb_conn_check(h.m, h.st, it, s, h.td.rngList, h.Mcap);
-        nl += hasM;
-    }
     if (fromStage <= ST_CROSSINGS) {
-        launch_crossings<Real>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, it, s);
+        // ST_PERTURB_CONN: the test runs with the crossings
+        launch_crossings<Real>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, it, s, fromStage <= ST_PERTURB_CONN,
+                               h.td.rngList, h.Mcap);
         nl += hasM ? 3 : 0;
     }
     if (fromStage <= ST_REINIT) {
