@@ -779,8 +779,8 @@ __device__ __forceinline__ int slot_code(int d) {  // E,N,W,S -> 0..3
 // it): the general form enumerates the lattice lines between its end points,
 // which the bounds test below keeps on the lattice, once to count and once to
 // emit.  A block reserves its records with one atomic (a warp did: 4,700 of
-// them on one address for 150k connections).  12.5 -> XX us at 150k
-// connections, 3.8 -> XX us for one cell; with the perturbation test, a kernel
+// them on one address for 150k connections).  12.5 -> 7.8 us at 150k
+// connections, 3.8 -> 3.6 us for one cell, with the perturbation test, a kernel
 // of its own before (3.3 and 2.1 us), inside.
 
 struct CrossRec {
@@ -1052,7 +1052,10 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
             if (k < c.bounceCap) c.bounceKeys[k] = key;
             else raise_error(st, ERR_CAPACITY, (int)node, ST_CROSSINGS);
         }
-        if (s == 2) c.wDom[node] = bdom + 1;
+        if (s == 2) {
+            c.wDom[node] = bdom + 1;
+            c.rowNow[(uint32_t)node / (uint32_t)nx] = 1;
+        }
         bool last = true;
         for (int s2 = s + 1; s2 < 4; ++s2)
             if (c.bnDist[node * 4 + s2] != kEmpty) last = false;
@@ -1061,6 +1064,7 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
             if (k < c.changedCap) {
                 c.changedNode[k] = (uint32_t)node;
                 c.changedDom[k] = bdom;
+                c.rowNow[(uint32_t)node / (uint32_t)nx] = 1;
                 c.mark[node] = k + 1;  // the node's position in the list, for the re-initialisation
             } else {
                 raise_error(st, ERR_CAPACITY, (int)node, ST_CROSSINGS);
@@ -1140,95 +1144,136 @@ void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigne
 // takes its new domain and re-initialises from its E,N,W,S neighbours of the
 // same domain that have no boundary node on the link, reading neighbours that
 // come earlier in the order with their new state and later ones with their old
-// state.  Here one block sorts the changed nodes, records for each the earlier
-// changed nodes among its E,N,W,S,NE (read after write) and SW (write after
-// read) neighbours, and processes nodes in rounds once those are done.
-constexpr int kReinitMax = 4096;  // changed nodes per step (dynamic shared memory)
-constexpr size_t kReinitSmem = (size_t)kReinitMax * (sizeof(unsigned long long) + 8 * sizeof(int) + 1) + 16;
+// state.  So a changed node waits for the earlier changed nodes among its
+// E,N,W,S,NE (read after write) and SW (write after read) neighbours; the
+// nodes that wait for none (almost all of them) are re-initialised at once by
+// the whole grid, the others by the grid's last block, in rounds.
+//
+// One warp per changed node: its lanes read what the update may need (the
+// species' 25 neighbour values, the neighbours' domains and marks, the boundary
+// slots, the velocity) in one go, and the arithmetic, which is the reference's
+// in its order, runs alike in every lane.  With a thread per node (75 loads
+// and 106 registers each) and the waiting nodes in a second one-block launch
+// the stage took 16.6 us for 150 changed nodes of 1024^2 and 4.2 us for none;
+// this form takes 11.1 (latency: five dependent reads, then those of the waiting
+// nodes) and 1.6 us.
+constexpr int kReinitMax = 4096;  // changed nodes per step
+struct SpeciesSet {
+    SpeciesConst s[kMaxSpecies];
+};
 
+// What a warp's lanes read for the re-initialisation of a node: lane 5 s + q
+// slot q of neighbour s (E, N, W, S, NE) of each species; the domains, boundary
+// slots and the velocity ride on lanes of their own.
 template <typename Real>
-__device__ void reinit_node(size_t n, uint32_t newDom, uint32_t* dom, Real* g, const Real* u, int nS,
-                            const SpeciesConst* sp, const double* srcTab, int nDomains, const uint32_t* ctypeTab,
-                            int cellTypesCopied, const CrossDev& c, int nx, int ny, size_t L, Status* st,
-                            unsigned iteration) {
-    // Every value the update may read is loaded before any is used (the
-    // neighbours' domains and distributions, the node's boundary slots and
-    // velocity), so that the loads overlap instead of forming a chain; the
-    // arithmetic below is the reference's, in its order.
-    const uint32_t oldDom = dom[n];
-    const int x = (int)(n % nx), y = (int)(n / nx);
+struct ReinitLoads {
+    Real gv[kMaxSpecies];
+    uint32_t dom;
+    bool bn;
+    double u;
+};
+
+// Neighbour s of (x, y): E, N, W, S, NE, then the other diagonals NW, SW, SE.
+__device__ __forceinline__ size_t reinit_neighbour(int x, int y, int nx, int ny, int s) {
     const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
     const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
-    const size_t nb[5] = {(size_t)y * nx + xp, (size_t)yp * nx + x, (size_t)y * nx + xm, (size_t)ym * nx + x,
-                          (size_t)yp * nx + xp};  // E, N, W, S, then NE
-    uint32_t dnb[5];
+    const int X = (s == 0 || s == 4 || s == 7) ? xp : ((s == 2 || s == 5 || s == 6) ? xm : x);
+    const int Y = (s == 1 || s == 4 || s == 5) ? yp : ((s == 3 || s == 6 || s == 7) ? ym : y);
+    return (size_t)Y * nx + X;
+}
+
+// The values other blocks may have written in this launch are read past the L1
+// cache.
+template <typename Real>
+__device__ __forceinline__ ReinitLoads<Real> reinit_load(size_t n, const uint32_t* dom, const Real* g, const Real* u,
+                                                         int nS, const CrossDev& c, int nx, int ny, size_t L) {
+    const int lane = threadIdx.x & 31;
+    const int x = (int)((uint32_t)n % (uint32_t)nx), y = (int)((uint32_t)n / (uint32_t)nx);
+    const int s5 = lane / 5, q5 = lane - 5 * s5;
+    const size_t nbv = reinit_neighbour(x, y, nx, ny, s5 < 5 ? s5 : 4);
+    ReinitLoads<Real> r;
 #pragma unroll
-    for (int s = 0; s < 5; ++s) dnb[s] = dom[nb[s]];
-    bool hasBN[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) hasBN[s] = c.bnDist[n * 4 + s] != kEmpty;
-    const double ux = (double)u[n], uy = (double)u[L + n];
-    dom[n] = newDom;
+    for (int k = 0; k < kMaxSpecies; ++k)
+        r.gv[k] = k < nS && lane < 25 ? __ldcg(g + ((size_t)k * 5 + q5) * L + nbv) : (Real)0;
+    r.dom = lane < 8 ? __ldcg(dom + reinit_neighbour(x, y, nx, ny, lane)) : (lane == 8 ? __ldcg(dom + n) : 0u);
+    r.bn = lane < 4 && __ldcg(c.bnDist + n * 4 + lane) != kEmpty;
+    r.u = lane < 2 ? (double)u[(size_t)lane * L + n] : 0.0;
+    return r;
+}
+
+// The warp re-initialises node n (all lanes take part).
+template <typename Real>
+__device__ __forceinline__ void reinit_node(const ReinitLoads<Real>& in, size_t n, uint32_t newDom, uint32_t* dom,
+                                            Real* g, int nS, const SpeciesConst* sp, const double* srcTab,
+                                            int nDomains, const uint32_t* ctypeTab, int cellTypesCopied, int nx,
+                                            int ny, size_t L, Status* st, unsigned iteration) {
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned hasBN = __ballot_sync(all, in.bn);
+    const unsigned same = __ballot_sync(all, lane < 8 && in.dom == newDom);  // bit s: neighbour s is of the new domain
+    const uint32_t oldDom = __shfl_sync(all, in.dom, 8);
+    const double ux = __shfl_sync(all, in.u, 0), uy = __shfl_sync(all, in.u, 1);
+    if (lane == 0) dom[n] = newDom;
     // boundaryNodes_[NE] aliases (domainIdentifier_, cellType_): null only if both are 0.
     const uint32_t ctype = cellTypesCopied ? (oldDom < (uint32_t)nDomains ? ctypeTab[oldDom] : 1u) : 0u;
     const bool neNull = newDom == 0 && ctype == 0;
-    double Cnew[kMaxSpecies] = {0.0, 0.0, 0.0};  // getC() of the species already re-initialised here
+    double Cnew[2] = {0.0, 0.0};  // getC() of the first two species once re-initialised here
     bool coupled = false;
     for (int k = 0; k < nS; ++k) coupled |= sp[k].partner >= 0;
+#pragma unroll 1
     for (int k = 0; k < nS; ++k) {
         const Real* gk = g + (size_t)k * 5 * L;
-        // the five slots of the four neighbours and NE, read unconditionally
-        Real gv[5][5];
-#pragma unroll
-        for (int s = 0; s < 5; ++s)
-#pragma unroll
-            for (int q = 0; q < 5; ++q) gv[s][q] = gk[(size_t)q * L + nb[s]];
-        // getC() in slot order after localSwap: T, W, S, E, N
-        auto cOf = [](const Real* v) {
-            double C = 0.0;
-            C += (double)v[0];
-            C += (double)v[3];
-            C += (double)v[4];
-            C += (double)v[1];
-            C += (double)v[2];
-            return C;
-        };
+        // getC() of neighbour s in slot order after localSwap (T, W, S, E, N),
+        // formed by lane s
+        const double v = (double)(k == 0 ? in.gv[0] : k == 1 ? in.gv[1] : in.gv[2]);
+        const int b = 5 * (lane < 5 ? lane : 0);
+        double Cs = 0.0;
+        Cs += __shfl_sync(all, v, b);
+        Cs += __shfl_sync(all, v, b + 3);
+        Cs += __shfl_sync(all, v, b + 4);
+        Cs += __shfl_sync(all, v, b + 1);
+        Cs += __shfl_sync(all, v, b + 2);
         const int style = sp[k].reinit;
         double sumC = 0.0;
         int counter = 0;
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            if (!hasBN[s] && newDom == dnb[s]) {
-                sumC += cOf(gv[s]);
+            const double Cn = __shfl_sync(all, Cs, s);
+            if (!((hasBN >> s) & 1u) && ((same >> s) & 1u)) {
+                sumC += Cn;
                 counter++;
             }
         }
-        if (counter == 0 && style != RI_DIAG && neNull && newDom == dnb[4]) {
-            sumC += cOf(gv[4]);
+        if (counter == 0 && style != RI_DIAG && neNull && ((same >> 4) & 1u)) {
+            sumC += __shfl_sync(all, Cs, 4);
             counter++;
-            atomicAdd(&st->nDiagReinit, 1);
+            if (lane == 0) atomicAdd(&st->nDiagReinit, 1);
         }
         if (counter == 0 && style == RI_DIAG) {
             // NE, NW, SW, SE of the same domain, no boundary-node test
-            const size_t dg[4] = {nb[4], (size_t)yp * nx + xm, (size_t)ym * nx + xm, (size_t)ym * nx + xp};
-            for (int s = 0; s < 4; ++s) {
-                if (dom[dg[s]] != newDom) continue;
-                Real v[5];
-                for (int q = 0; q < 5; ++q) v[q] = gk[(size_t)q * L + dg[s]];
-                sumC += cOf(v);
+            for (int s = 4; s < 8; ++s) {
+                if (!((same >> s) & 1u)) continue;
+                const size_t nd = reinit_neighbour((int)(n % nx), (int)(n / nx), nx, ny, s);
+                double C = 0.0;
+                C += (double)__ldcg(gk + nd);
+                C += (double)__ldcg(gk + 3 * L + nd);
+                C += (double)__ldcg(gk + 4 * L + nd);
+                C += (double)__ldcg(gk + 1 * L + nd);
+                C += (double)__ldcg(gk + 2 * L + nd);
+                sumC += C;
                 counter++;
             }
-            if (counter != 0) atomicAdd(&st->nDiagReinit, 1);
+            if (counter != 0 && lane == 0) atomicAdd(&st->nDiagReinit, 1);
         }
         if (counter == 0 && style == RI_ALL4) {
             // all of E, N, W, S whatever their domain
 #pragma unroll
             for (int s = 0; s < 4; ++s) {
-                sumC += cOf(gv[s]);
+                sumC += __shfl_sync(all, Cs, s);
                 counter++;
             }
         }
-        if (counter == 0) atomicAdd(&st->nFailedReinit, 1);
+        if (counter == 0 && lane == 0) atomicAdd(&st->nFailedReinit, 1);
         sumC /= static_cast<double>(counter);
         double gi[5];
         for (int q = 0; q < 5; ++q) gi[q] = style == RI_DIAG ? sumC / 4.0 : sumC / 5.0;
@@ -1240,142 +1285,128 @@ __device__ void reinit_node(size_t n, uint32_t newDom, uint32_t* dom, Real* g, c
         const int pj = sp[k].partner;
         if (pj >= 0 && pj < nS) {
             if (pj < k) {
-                Cp = Cnew[pj];
+                Cp = pj == 0 ? Cnew[0] : Cnew[1];
             } else {
-                Real v[5];
-                for (int q = 0; q < 5; ++q) v[q] = g[((size_t)pj * 5 + q) * L + n];
-                Cp = cOf(v);
+                const Real* gp = g + (size_t)pj * 5 * L + n;
+                Cp += (double)__ldcg(gp);
+                Cp += (double)__ldcg(gp + 3 * L);
+                Cp += (double)__ldcg(gp + 4 * L);
+                Cp += (double)__ldcg(gp + 1 * L);
+                Cp += (double)__ldcg(gp + 2 * L);
             }
         }
         collide_cde64(gi, ux, uy, sp[k], src, Cp, newDom, ctype, iteration);
-        if (coupled) Cnew[k] = sum5_swapped(gi);
-        Real* go = g + (size_t)k * 5 * L;
-        for (int q = 0; q < 5; ++q) go[(size_t)q * L + n] = (Real)gi[q];
+        if (coupled) {
+            const double C = sum5_swapped(gi);
+            if (k == 0) Cnew[0] = C;
+            else Cnew[1] = C;
+        }
+        const double out = lane == 0 ? gi[0] : lane == 1 ? gi[1] : lane == 2 ? gi[2] : lane == 3 ? gi[3] : gi[4];
+        if (lane < 5) g[((size_t)k * 5 + lane) * L + n] = (Real)out;
     }
 }
 
-// The earlier changed nodes a changed node n waits for: its E,N,W,S (read
-// after write: n reads their new state) and NE / SW neighbours (SW reads n's
-// old state through its NE fallback) with a smaller row-major index; with a
-// species that falls back on all four diagonals (RI_DIAG) also NW / SE; -1 none.
-constexpr int kReinitDeps = 8;
-__device__ __forceinline__ void reinit_deps(const CrossDev& c, size_t n, int nx, int ny, int* deps) {
-    const int x = (int)(n % nx), y = (int)(n / nx);
-    const int xm = x == 0 ? nx - 1 : x - 1, xp = x == nx - 1 ? 0 : x + 1;
-    const int ym = y == 0 ? ny - 1 : y - 1, yp = y == ny - 1 ? 0 : y + 1;
-    const size_t nbs[8] = {(size_t)y * nx + xp,  (size_t)yp * nx + x,  (size_t)y * nx + xm,  (size_t)ym * nx + x,
-                           (size_t)yp * nx + xp, (size_t)ym * nx + xm, (size_t)yp * nx + xm, (size_t)ym * nx + xp};
-#pragma unroll
-    for (int d = 0; d < 8; ++d) deps[d] = (d < 6 || c.diag8) && nbs[d] < n ? c.mark[nbs[d]] - 1 : -1;
+// Place + 1 in the changed list of the earlier changed node that lane d < 8
+// finds in direction d (0: none, or it is not waited for): E, N, W, S, NE, SW;
+// with a species that falls back on all four diagonals (RI_DIAG) also NW, SE.
+__device__ __forceinline__ int reinit_dep(const CrossDev& c, size_t n, int nx, int ny, int d) {
+    if (d >= 8 || (d >= 6 && !c.diag8)) return 0;
+    const int s = d == 5 ? 6 : d == 6 ? 5 : d;  // SW before NW
+    const size_t nb = reinit_neighbour((int)((uint32_t)n % (uint32_t)nx), (int)((uint32_t)n / (uint32_t)nx), nx, ny, s);
+    return nb < n ? c.mark[nb] : 0;
 }
 
-// (Each changed node's position in the list is marked where the crossings
-// append it, in cross_win_kernel; the block kernel clears the marks.)
-// Step 1, across the whole GPU: the nodes that wait for no other changed node
-// (almost all of them) are re-initialised at once.  No two such nodes read
-// each other (a changed neighbour in any of the six directions makes one of
-// the two wait for the other), so the order among them does not matter.
+// (Each changed node's place in the list is marked where the crossings append
+// it, in cross_win_kernel; the last block clears the marks.)  No two nodes that
+// wait for none read each other (a changed neighbour in any of the directions
+// makes one of the two wait for the other), so the order among them does not
+// matter.
+constexpr int kReinitBlock = 128;
 template <typename Real>
-__global__ void reinit_free_kernel(CrossDev c, uint32_t* dom, Real* g, const Real* u, int nS, SpeciesConst sp0,
-                                   SpeciesConst sp1, SpeciesConst sp2, const double* srcTab, int nDomains,
-                                   const uint32_t* ctypeTab, int nx, int ny, size_t L, Status* st) {
+__global__ void __launch_bounds__(kReinitBlock) reinit_kernel(CrossDev c, uint32_t* dom, Real* g, const Real* u, int nS,
+                                                              const __grid_constant__ SpeciesSet species,
+                                                              const double* srcTab, int nDomains,
+                                                              const uint32_t* ctypeTab, int nx, int ny, size_t L,
+                                                              Status* st) {
     pdl_wait();
     if (st->halt) return;
     const int cnt = st->nChanged;
-    if (cnt > kReinitMax || cnt > c.changedCap) return;  // reported by the block kernel
-    const SpeciesConst sp[3] = {sp0, sp1, sp2};
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += gridDim.x * blockDim.x) {
+    if (cnt == 0) return;
+    if (cnt > kReinitMax || cnt > c.changedCap) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(st, ERR_CAPACITY, cnt, ST_REINIT);
+        return;
+    }
+    const SpeciesConst* sp = species.s;
+    const unsigned iteration = st->iteration;
+    const int typesCopied = st->cellTypesCopied;
+    const int lane = threadIdx.x & 31, warps = kReinitBlock / 32, warp = threadIdx.x >> 5;
+    for (int k = blockIdx.x * warps + warp; k < cnt; k += gridDim.x * warps) {
         const size_t n = c.changedNode[k];
-        int deps[kReinitDeps];
-        reinit_deps(c, n, nx, ny, deps);
-        bool free = true;
-#pragma unroll
-        for (int d = 0; d < kReinitDeps; ++d) free &= deps[d] < 0;
-        if (!free) {
-            // listed for the one-block pass; the mark says where
-            const int w = atomicAdd(c.nWait, 1);
-            c.waitList[w] = k;
-            c.reinitDone[k] = 2 + w;
-        } else {
-            c.reinitDone[k] = 1;
+        const uint32_t newDom = c.changedDom[k];
+        // read with the marks, before it is known that the node may go ahead
+        const ReinitLoads<Real> in = reinit_load<Real>(n, dom, g, u, nS, c, nx, ny, L);
+        const bool free = !__any_sync(0xffffffffu, reinit_dep(c, n, nx, ny, lane) > 0);
+        if (lane == 0) {
+            int done = 1;
+            if (!free) {
+                // listed for the last block; the place says where
+                const int w = atomicAdd(&c.nWait[0], 1);
+                c.waitList[w] = k;
+                done = 2 + w;
+            }
+            c.reinitDone[k] = done;
         }
         if (free)
-            reinit_node<Real>(n, c.changedDom[k], dom, g, u, nS, sp, srcTab, nDomains, ctypeTab, st->cellTypesCopied,
-                              c, nx, ny, L, st, st->iteration);
+            reinit_node<Real>(in, n, newDom, dom, g, nS, sp, srcTab, nDomains, ctypeTab, typesCopied, nx, ny, L, st,
+                              iteration);
     }
-}
-
-template <typename Real>
-__global__ void __launch_bounds__(1024) reinit_kernel(CrossDev c, uint32_t* dom, Real* g, const Real* u, int nS,
-                                                      SpeciesConst sp0, SpeciesConst sp1, SpeciesConst sp2,
-                                                      const double* srcTab, int nDomains, const uint32_t* ctypeTab,
-                                                      int cellTypesCopied, int nx, int ny, size_t L, Status* st,
-                                                      unsigned iteration) {
-    pdl_wait();
-    const int cnt = st->nChanged;
-    if (st->halt || cnt == 0) {
-        if (threadIdx.x == 0) *c.nWait = 0;
-        return;
-    }
-    if (cnt > kReinitMax || cnt > c.changedCap) {
-        if (threadIdx.x == 0) {
-            raise_error(st, ERR_CAPACITY, cnt, ST_REINIT);
-            *c.nWait = 0;
-        }
-        return;
-    }
-    const SpeciesConst sp[3] = {sp0, sp1, sp2};
-    extern __shared__ __align__(16) unsigned char smem[];
-    unsigned long long* key = (unsigned long long*)smem;  // node << 32 | newDom
-    int(*deps)[kReinitDeps] = (int(*)[kReinitDeps])(key + kReinitMax);
-    unsigned char* done = (unsigned char*)(deps + kReinitMax);
-    __shared__ int remaining;
-    // Step 2, one block: only the nodes that wait for others (listed by the
-    // wide pass, usually few or none), in dependency rounds.  A dependency is
-    // done when the wide pass re-initialised it (reinitDone 1) or when this
-    // pass did (done[w] of its place w in the wait list, reinitDone 2 + w).
-    const int nw = min(*c.nWait, cnt);
-    if (threadIdx.x == 0) remaining = nw;
-    for (int w = threadIdx.x; w < nw; w += blockDim.x) {
-        const int k = c.waitList[w];
-        key[w] = (((unsigned long long)c.changedNode[k]) << 32) | c.changedDom[k];
-        reinit_deps(c, (size_t)c.changedNode[k], nx, ny, deps[w]);
-        done[w] = 0;
-    }
+    // the last block to finish: the waiting nodes, usually few or none.  A node
+    // waited for is done when the whole grid's pass did it (reinitDone 1) or
+    // when this one has (done[w] of its place w in the wait list).
+    __shared__ bool last;
+    __threadfence();
     __syncthreads();
-    int rounds = 0;
-    while (remaining > 0 && rounds < kReinitMax + 1) {
-        __shared__ int nowDone;
-        if (threadIdx.x == 0) nowDone = 0;
+    if (threadIdx.x == 0) last = atomicAdd((unsigned*)&c.nWait[1], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const int nw = __ldcg(&c.nWait[0]);
+    __shared__ unsigned char done[kReinitMax];
+    __shared__ int remaining;
+    for (int w = threadIdx.x; w < nw; w += kReinitBlock) done[w] = 0;
+    if (threadIdx.x == 0) remaining = nw;
+    __syncthreads();
+    // a round does every node whose earlier ones are done: at most nw rounds
+    for (int round = 0; round < nw && remaining > 0; ++round) {
         __syncthreads();
-        for (int w = threadIdx.x; w < nw; w += blockDim.x) {
+        for (int w = warp; w < nw; w += warps) {
             if (done[w]) continue;
-            bool ready = true;
-            for (int d = 0; d < kReinitDeps; ++d) {
-                const int p = deps[w][d];
-                if (p < 0) continue;
-                const int v = c.reinitDone[p];
-                if (v != 1 && done[v - 2] != 1) ready = false;
+            const size_t n = c.changedNode[__ldcg(&c.waitList[w])];
+            const int p = reinit_dep(c, n, nx, ny, lane);
+            bool waits = false;
+            if (p > 0) {
+                const int v = __ldcg(&c.reinitDone[p - 1]);
+                waits = v != 1 && done[v - 2] != 1;
             }
-            if (ready) done[w] = 2;  // processing this round
+            // marked only after the round's tests: no node of the round sees it done
+            if (!__any_sync(0xffffffffu, waits) && lane == 0) done[w] = 2;
         }
         __syncthreads();
-        for (int w = threadIdx.x; w < nw; w += blockDim.x) {
-            if (done[w] == 2) {
-                reinit_node<Real>((size_t)(key[w] >> 32), (uint32_t)(key[w] & 0xffffffffu), dom, g, u, nS, sp, srcTab,
-                                  nDomains, ctypeTab, st->cellTypesCopied, c, nx, ny, L, st, st->iteration);
-                atomicAdd(&nowDone, 1);
-            }
+        for (int w = warp; w < nw; w += warps) {
+            if (done[w] != 2) continue;
+            const int k = __ldcg(&c.waitList[w]);
+            const size_t n = c.changedNode[k];
+            reinit_node<Real>(reinit_load<Real>(n, dom, g, u, nS, c, nx, ny, L), n, c.changedDom[k], dom, g, nS, sp,
+                              srcTab, nDomains, ctypeTab, typesCopied, nx, ny, L, st, iteration);
+            if (lane == 0) atomicSub(&remaining, 1);
         }
         __syncthreads();
-        for (int w = threadIdx.x; w < nw; w += blockDim.x)
+        for (int w = threadIdx.x; w < nw; w += kReinitBlock)
             if (done[w] == 2) done[w] = 1;
-        if (threadIdx.x == 0) remaining -= nowDone;
         __syncthreads();
-        ++rounds;
     }
-    for (int k = threadIdx.x; k < cnt; k += blockDim.x) c.mark[(size_t)c.changedNode[k]] = 0;
-    if (threadIdx.x == 0) *c.nWait = 0;
+    for (int k = threadIdx.x; k < cnt; k += kReinitBlock) c.mark[(size_t)c.changedNode[k]] = 0;
+    if (threadIdx.x < 2) c.nWait[threadIdx.x] = 0;
 }
 
 template <typename Real>
@@ -1383,11 +1414,9 @@ void launch_reinit(CrossDev& c, uint32_t* dom, Real* g, const Real* u, int nS, c
                    const double* srcTab, int nDomains, const uint32_t* ctypeTab, int cellTypesCopied, int nx, int ny,
                    size_t L, Status* st, unsigned iteration, cudaStream_t s) {
     if (c.changedCap <= 0) return;
-    constexpr size_t smemBytes = kReinitSmem;
-    launch_pdl(reinit_free_kernel<Real>, 148, 256, 0, s, c, dom, g, u, nS, sp[0], sp[1], sp[2], srcTab, nDomains,
-               ctypeTab, nx, ny, L, st);
-    launch_pdl(reinit_kernel<Real>, 1, 1024, smemBytes, s, c, dom, g, u, nS, sp[0], sp[1], sp[2], srcTab, nDomains, ctypeTab,
-                                           cellTypesCopied, nx, ny, L, st, iteration);
+    const SpeciesSet species{{sp[0], sp[1], sp[2]}};
+    launch_pdl(reinit_kernel<Real>, 148, kReinitBlock, 0, s, c, dom, g, u, nS, species, srcTab, nDomains, ctypeTab, nx,
+               ny, L, st);
 }
 template void launch_reinit<double>(CrossDev&, uint32_t*, double*, const double*, int, const SpeciesConst*,
                                     const double*, int, const uint32_t*, int, int, int, size_t, Status*, unsigned,
@@ -1403,50 +1432,91 @@ template void launch_reinit<float>(CrossDev&, uint32_t*, float*, const float*, i
 // The kernel also resets the (node, slot) entries the step's crossings wrote
 // (every written key has a record), after the re-initialisation that read
 // them; that part runs on a halted step too.
-__global__ void __launch_bounds__(256) domain_fill_kernel(CrossDev c, uint32_t* dom, int nx, int ny, Status* st) {
+//
+// Each warp takes eight segments of 32 nodes, all loaded before the first is
+// used; the last mark at or before a node is a ballot and a shuffle, and the
+// warps' last marks meet in shared memory.  Rows without a mark now and after
+// the last fill, and without a changed node, hold the exterior throughout and
+// are left as they are.  With a run of consecutive nodes per thread (strided
+// access) and a block scan the kernel took 6.5 us for 1024^2 and 25 us for a
+// 2048^2 lattice with cells in its middle; this form takes 6.1 and 9.1 us.
+constexpr int kFillBlock = 128, kFillSeg = 8;
+__global__ void __launch_bounds__(kFillBlock) domain_fill_kernel(CrossDev c, uint32_t* dom, int nx, int ny,
+                                                                 Status* st) {
     pdl_wait();
-    const int nrec = min(st->pad[2], c.recCap);
+    const int y = blockIdx.x;
+    const size_t row = (size_t)y * nx;
+    // everything the block's course depends on, read at once
+    const int nrec = min(st->pad[2], c.recCap), halt = st->halt;
+    const bool marked = c.rowNow[y] | c.rowHad[y];
+    const uint32_t left = dom[row];
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nrec; k += gridDim.x * blockDim.x) {
         const uint32_t key = c.recKey[k];
         c.bnDist[key] = kEmpty;
         c.bnConn[key] = ~0u;
     }
-    if (st->halt) return;
-    const int y = blockIdx.x;
-    const size_t row = (size_t)y * nx;
-    const uint32_t left = dom[row];
+    if (halt || !marked) return;
     if (left != 0) {
         if (threadIdx.x == 0) raise_error(st, ERR_LEFT_DOMAIN, y, ST_DOMAIN);
         return;
     }
-    const int chunk = (nx + blockDim.x - 1) / blockDim.x;
-    const int xb = threadIdx.x * chunk;
-    const int xe = min(nx, xb + chunk);
-    // last W mark in this thread's chunk (x >= 1): (x << 32 | value)
-    unsigned long long last = 0;
-    for (int x = max(xb, 1); x < xe; ++x) {
-        const uint32_t w = c.wDom[row + x];
-        if (w) last = ((unsigned long long)(x + 1) << 32) | (w - 1);
-    }
-    typedef cub::BlockScan<unsigned long long, 256> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    unsigned long long carry;
-    Scan(tmp).ExclusiveScan(last, carry, 0ull, cub::Max());
-    uint32_t cur = carry ? (uint32_t)(carry & 0xffffffffu) : left;
-    for (int x = max(xb, 1); x < xe; ++x) {
-        const uint32_t w = c.wDom[row + x];
-        if (w) {
-            cur = w - 1;
-            c.wDom[row + x] = 0;
+    constexpr int warps = kFillBlock / 32;
+    __shared__ uint32_t lastOf[warps];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;  // the last mark before this pass (domain + 1, 0: none)
+    bool any = false;
+    for (int x0 = 0; x0 < nx; x0 += warps * kFillSeg * 32) {
+        const int xw = x0 + warp * kFillSeg * 32 + lane;
+        uint32_t w[kFillSeg];
+#pragma unroll
+        for (int j = 0; j < kFillSeg; ++j) {
+            const int x = xw + 32 * j;
+            w[j] = x >= 1 && x < nx ? c.wDom[row + x] : 0u;
         }
-        dom[row + x] = cur;
+        uint32_t lastMark = 0;
+#pragma unroll
+        for (int j = 0; j < kFillSeg; ++j) {
+            const unsigned bal = __ballot_sync(0xffffffffu, w[j] != 0);
+            const uint32_t v = __shfl_sync(0xffffffffu, w[j], bal ? 31 - __clz(bal) : 0);
+            if (bal) lastMark = v;
+        }
+        if (lane == 0) lastOf[warp] = lastMark;
+        __syncthreads();
+        uint32_t cur = carry;
+#pragma unroll
+        for (int q = 0; q < warps; ++q) {
+            const uint32_t v = lastOf[q];
+            if (v) {
+                if (q < warp) cur = v;
+                carry = v;
+                any = true;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kFillSeg; ++j) {
+            const int x = xw + 32 * j;
+            const unsigned bal = __ballot_sync(0xffffffffu, w[j] != 0);
+            const unsigned own = bal & (0xffffffffu >> (31 - lane));
+            const uint32_t v = __shfl_sync(0xffffffffu, w[j], own ? 31 - __clz(own) : lane);
+            const uint32_t e = __shfl_sync(0xffffffffu, w[j], bal ? 31 - __clz(bal) : 0);
+            const uint32_t mark = own ? v : cur;
+            if (x >= 1 && x < nx) {
+                dom[row + x] = mark ? mark - 1u : 0u;
+                if (w[j]) c.wDom[row + x] = 0;
+            }
+            if (bal) cur = e;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        c.rowHad[y] = any;
+        c.rowNow[y] = 0;
     }
 }
 
-
 void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, size_t L, Status* st, unsigned iteration,
                         cudaStream_t s) {
-    launch_pdl(domain_fill_kernel, ny, 256, 0, s, c, dom, nx, ny, st);
+    launch_pdl(domain_fill_kernel, ny, kFillBlock, 0, s, c, dom, nx, ny, st);
 }
 
 
@@ -1913,8 +1983,6 @@ void launch_motion_adjoint(const double* X, const double* Y, const double* fx, c
 namespace lbib {
 
 void init_kernel_attributes() {
-    cudaFuncSetAttribute(reinit_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReinitSmem);
-    cudaFuncSetAttribute(reinit_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kReinitSmem);
     init_kernel_attributes_topology();
 }
 

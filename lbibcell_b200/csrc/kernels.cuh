@@ -88,10 +88,12 @@ struct CrossDev {
     uint32_t* bnConn;            // 4*L, ~0u
     uint32_t* bnDom;             // 4*L
     uint32_t* wDom;              // L, W-slot winner domain + 1 (0: none)
+    uint8_t* rowNow;             // ny: the row has a W-slot winner or a changed node this step
+    uint8_t* rowHad;             // ny: it had W-slot winners at its last fill
     int* mark;                   // L, position + 1 of a node in this step's changed list (0: none)
     int* reinitDone;             // changedCap: 1 = re-initialised by the wide pass, 2 + w = waiting at waitList[w]
     int* waitList;               // changedCap: list positions of the nodes that wait for another
-    int* nWait;                  // entries of waitList
+    int* nWait;                  // [0] entries of waitList, [1] blocks of the re-initialisation that are through
     uint32_t* changedNode;       // capacity: nodes whose domain changes
     uint32_t* changedDom;
     int changedCap;

@@ -455,7 +455,7 @@ Handle::~Handle() {
     fr(m.ringStart); fr(m.ringNode); fr(m.ringDom);
     fr(outPos); fr(inPos); fr(target); fr(areaAcc);  // area lives in the status allocation
     fr(tiles.count); fr(tiles.active); fr(tiles.slots);
-    fr(cross.bnDist); fr(cross.bnConn); fr(cross.bnDom); fr(cross.wDom); fr(cross.mark);
+    fr(cross.bnDist); fr(cross.bnConn); fr(cross.bnDom); fr(cross.wDom); fr(cross.rowNow); fr(cross.rowHad); fr(cross.mark);
     fr(cross.changedNode); fr(cross.changedDom); fr(cross.perturbList); fr(cross.reinitDone); fr(cross.waitList);
     fr(cross.nWait);
     fr(cross.recKey); fr(cross.recConn); fr(cross.recDom); fr(cross.recDist); fr(cross.nfKeys); fr(cross.nfD);
@@ -1200,8 +1200,8 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
         h.cross.reinitDone = dalloc<int>(h.cross.changedCap);
         h.cross.waitList = dalloc<int>(h.cross.changedCap);
         if (!h.cross.nWait) {
-            h.cross.nWait = dalloc<int>(1);
-            CK(cudaMemsetAsync(h.cross.nWait, 0, sizeof(int), h.stream));
+            h.cross.nWait = dalloc<int>(2);
+            CK(cudaMemsetAsync(h.cross.nWait, 0, 2 * sizeof(int), h.stream));
         }
         h.cross.changedDom = dalloc<uint32_t>(h.cross.changedCap);
     }
@@ -1442,7 +1442,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
         for (int k = 0; k < h.S; ++k) spc[k] = h.sp[k].c;
         launch_reinit<Real>(h.cross, h.dom, gcur, (const Real*)h.u, h.S, spc, h.srcTab, h.nDomains, h.ctypeTab, 0,
                             h.nx, h.ny, h.L, h.st, it, s);
-        nl += 2;
+        nl += 1;
     }
     if (fromStage <= ST_DOMAIN) {
         launch_domain_fill(h.cross, h.dom, h.nx, h.ny, h.L, h.st, it, s);
@@ -2088,6 +2088,10 @@ static void create(Handle& h, const std::string& params, const std::string& geom
     h.cross.bnConn = dalloc<uint32_t>(4 * h.L);
     h.cross.bnDom = dalloc<uint32_t>(4 * h.L);
     h.cross.wDom = dalloc<uint32_t>(h.L);
+    h.cross.rowNow = dalloc<uint8_t>(h.ny);
+    h.cross.rowHad = dalloc<uint8_t>(h.ny);
+    CK(cudaMemsetAsync(h.cross.rowNow, 0, h.ny, h.stream));
+    CK(cudaMemsetAsync(h.cross.rowHad, 0, h.ny, h.stream));
     h.cross.mark = dalloc<int>(h.L);
     CK(cudaMemsetAsync(h.cross.mark, 0, sizeof(int) * h.L, h.stream));
     CK(cudaMemsetAsync(h.cross.bnDist, 0xff, sizeof(unsigned long long) * 4 * h.L, h.stream));
