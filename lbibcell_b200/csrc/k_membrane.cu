@@ -24,10 +24,13 @@
 //                    (PhysicalNode.cpp:109-124, CDESolverD2Q5.cpp:156-228) in
 //                    row-major order semantics, processed in dependency rounds.
 //   domain_fill      GeometryHandler::updateAllDomainIdentifiers (GeometryHandler.cpp:68-85).
+#include <algorithm>
+
 #include <cub/cub.cuh>
 
 #include "kernels.cuh"
 #include "lattice_math.cuh"
+#include "remesh.cuh"
 
 namespace lbib {
 
@@ -978,9 +981,13 @@ __device__ __forceinline__ void edge_check_node(const MembraneDev& m, int i, int
 
 // Pass 1: among records at the closest distance, the earliest connection.
 // And, over the same grid, GeometryHandler::connectGeometryNodesToPhysicalNodes'
-// edge test of the moved nodes.  The kernel first raises the halt for the
-// connections that pass 0 listed for the host's perturbation.
-__global__ void cross_tie_kernel(CrossDev c, MembraneDev m, int nx, int ny, Status* st) {
+// edge test of the moved nodes, and the count of the connections that the
+// remeshing pass will split (remesh.cuh; a kernel of its own, with the pass's
+// decision in its last block, took 6.3 us at 150k connections).  The kernel
+// first raises the halt for the connections that pass 0 listed for the host's
+// perturbation.
+__global__ void __launch_bounds__(kRemeshBlock) cross_tie_kernel(CrossDev c, MembraneDev m, TopoDev t, int nx, int ny,
+                                                                 Status* st) {
     pdl_wait();
     if (st->halt) return;
     if (st->nPerturbConn > 0) {
@@ -989,6 +996,7 @@ __global__ void cross_tie_kernel(CrossDev c, MembraneDev m, int nx, int ny, Stat
     }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.topo->M; i += gridDim.x * blockDim.x)
         edge_check_node(m, i, nx, ny, st, ST_CROSSINGS);
+    if (t.flag != nullptr) remesh_count_block(m, t);  // (not at set-up)
     const int n = min(st->pad[2], c.recCap);
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
         const uint32_t key = c.recKey[r];
@@ -1109,7 +1117,7 @@ __global__ void edge_check_kernel(MembraneDev m, int nx, int ny, Status* st, int
 
 template <typename Real>
 void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, size_t L, Status* st,
-                      unsigned iteration, cudaStream_t s, bool check, int* perturb, int perturbCap) {
+                      const TopoDev* remesh, cudaStream_t s, bool check, int* perturb, int perturbCap) {
     const int blocks = (m.Ccap + kCrossBlock - 1) / kCrossBlock;
     if (m.Ccap == 0) {  // nodes without connections: the halt of the listed nodes alone
         if (check && m.Mcap > 0)
@@ -1124,13 +1132,14 @@ void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, in
     // grid-stride over the step's records (their count is known on the device
     // only): 8 blocks per SM, so that each thread's chain of dependent loads
     // overlaps many others
-    launch_pdl(cross_tie_kernel, 148 * 8, 256, 0, s, c, m, nx, ny, st);
+    launch_pdl(cross_tie_kernel, std::max(148 * 8, (m.Ccap + kRemeshBlock - 1) / kRemeshBlock), kRemeshBlock, 0, s, c, m,
+               remesh ? *remesh : TopoDev{}, nx, ny, st);
     launch_pdl(cross_win_kernel, 148 * 8, 256, 0, s, c, m, dom, nx, ny, st);
 }
 template void launch_crossings<double>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
-                                       unsigned, cudaStream_t, bool, int*, int);
+                                       const TopoDev*, cudaStream_t, bool, int*, int);
 template void launch_crossings<float>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
-                                      unsigned, cudaStream_t, bool, int*, int);
+                                      const TopoDev*, cudaStream_t, bool, int*, int);
 
 void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s) {
     if (m.Mcap == 0) return;
@@ -1636,7 +1645,6 @@ __global__ void __launch_bounds__(256) areas_kernel(MembraneDev m, double* area,
 // cells of type 1 get maxsource whatever their area.
 // acc != nullptr (FP32-shifted runs): the cell's area is first formed from
 // its fixed-point sum, which is reset for the next step (on a halted step too).
-constexpr double kAreaFix = 16777216.0;  // 2^24: the fixed-point scale of the shoelace terms
 __global__ void area_regulator_kernel(MembraneDev m, double* area, double* target, double* massTab,
                                       int nDomains, double factor, double strength, double maxsource,
                                       const uint32_t* ctypeTab, unsigned long long* acc, const Status* st) {
@@ -1740,24 +1748,7 @@ template void launch_growth<float>(const float*, const uint32_t*, size_t, int, i
 // the order; no ring ranking is needed.  FP64 runs keep the ring-ordered sum.
 __global__ void areas_fixed_kernel(MembraneDev m, const int* cellOfDom, int nDomains, unsigned long long* acc) {
     pdl_wait();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    int cell = -1;
-    long long v = 0;
-    if (c < m.topo->C) {
-        const int a = m.ca[c], b = m.cb[c];
-        const uint32_t d = m.cdom[c];
-        if (d < (uint32_t)nDomains) cell = cellOfDom[d];
-        v = __double2ll_rn((m.x[a] * m.y[b] - m.x[b] * m.y[a]) * kAreaFix);
-    }
-    // one atomic per run of equal cells in the warp (connections of a cell are mostly contiguous)
-    const unsigned peers = __match_any_sync(0xffffffffu, cell);
-    long long sum = 0;
-    for (int l = 0; l < 32; ++l) {
-        const long long t = __shfl_sync(0xffffffffu, v, l);
-        if ((peers >> l) & 1u) sum += t;
-    }
-    if (cell >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1)
-        atomicAdd(acc + cell, (unsigned long long)sum);
+    area_terms_fixed(m, blockIdx.x * blockDim.x + threadIdx.x, m.topo->C, m.ca, m.cb, m.cdom, cellOfDom, nDomains, acc);
 }
 
 void launch_areas(const MembraneDev& m, double* area, Status* st, cudaStream_t s) {
@@ -1801,9 +1792,10 @@ void launch_area_regulator(const MembraneDev& m, double* area, double* target, d
 
 void launch_area_regulator_fixed(const MembraneDev& m, const int* cellOfDom, unsigned long long* acc, double* area,
                                  double* target, double* massTab, int nDomains, double factor, double strength,
-                                 double maxsource, const uint32_t* ctypeTab, const Status* st, cudaStream_t s) {
+                                 double maxsource, const uint32_t* ctypeTab, const Status* st, cudaStream_t s,
+                                 bool summed) {
     if (m.nCells == 0 || m.Ccap == 0) return;
-    launch_pdl(areas_fixed_kernel, (m.Ccap + 255) / 256, 256, 0, s, m, cellOfDom, nDomains, acc);
+    if (!summed) launch_pdl(areas_fixed_kernel, (m.Ccap + 255) / 256, 256, 0, s, m, cellOfDom, nDomains, acc);
     launch_pdl(area_regulator_kernel, (m.nCells + 127) / 128, 128, 0, s, m, area, target, massTab, nDomains, factor,
                strength, maxsource, ctypeTab, acc, st);
 }

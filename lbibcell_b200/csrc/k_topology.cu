@@ -23,9 +23,12 @@
 //   rings     the node order of GeometryHandler::computeAreas (first connection
 //             of each domain in vector order, then the second node's outgoing
 //             connection) by pointer jumping, one block per cell.
+#include <algorithm>
+
 #include <cub/cub.cuh>
 
 #include "kernels.cuh"
+#include "remesh.cuh"
 
 namespace lbib {
 
@@ -35,11 +38,6 @@ size_t topo_scan_bytes(int n) {
     return b;
 }
 
-// |d| < MAXLENGTH and |d| > MAXLENGTH for a squared length d2, as the
-// reference tests them (the correctly rounded sqrt, Connection::getLength,
-// Connection.cpp:389-394), with the root taken only within a few ulps of
-// MAXLENGTH^2: the rounded root is monotonic, so well below it is below
-// MAXLENGTH and at or above it is not (and the other way round).
 // Position of the n-th (from 0) set bit of w; w has more than n set bits.
 __device__ __forceinline__ int nth_set_bit(unsigned w, int n) {
     int base = 0;
@@ -58,28 +56,13 @@ __device__ __forceinline__ int nth_set_bit(unsigned w, int n) {
     return base;
 }
 
+// |d| < MAXLENGTH for a squared length d2 (longer_than_max's other side).
 __device__ __forceinline__ bool shorter_than_max(double d2) {
     constexpr double m2 = kMAXLENGTH * kMAXLENGTH;
     if (d2 < m2 * (1.0 - 1e-12)) return true;
     if (d2 >= m2) return false;
     return sqrt(d2) < kMAXLENGTH;
 }
-__device__ __forceinline__ bool longer_than_max(double d2) {
-    constexpr double m2 = kMAXLENGTH * kMAXLENGTH;
-    if (d2 > m2 * (1.0 + 1e-12)) return true;
-    if (d2 <= m2) return false;
-    return sqrt(d2) > kMAXLENGTH;
-}
-
-// Perturbation tests of a new node (GeometryNode.cpp:160, 174, 189, 202).
-__device__ __forceinline__ bool new_node_needs_rng(double X, double Y) {
-    if (fabs((double)(int)X - X) <= kEPSILON) return true;
-    if (fabs((double)(int)Y - Y) <= kEPSILON) return true;
-    if (fabs(Y - floor(Y) - (X - floor(X))) <= kEPSILON) return true;
-    if (fabs(ceil(Y) - Y - (X - floor(X))) <= kEPSILON) return true;
-    return false;
-}
-
 // Warp-aggregated atomics: lanes with the same key share one atomic.
 __device__ __forceinline__ int agg_add(int* addr, int key) {
     const unsigned act = __activemask();
@@ -103,77 +86,18 @@ __device__ __forceinline__ void agg_min(int* addr, int key, int v) {
 // ---------------------------------------------------------------------------
 // Remesh
 
-constexpr int kRemeshBlock = 256;  // connections per block of the count and apply kernels
-
-// Connection c is split: longer than MAXLENGTH (Connection::getLength,
-// Connection.cpp:389-394).  `rng`: its new node needs the random perturbation.
-__device__ __forceinline__ bool remesh_split(const MembraneDev& m, int c, bool& rng) {
-    const int a = m.ca[c], b = m.cb[c];
-    const double x1 = m.x[a], y1 = m.y[a], x2 = m.x[b], y2 = m.y[b];
-    const bool split = longer_than_max((x1 - x2) * (x1 - x2) + (y1 - y2) * (y1 - y2));
-    rng = split && new_node_needs_rng((x1 + x2) / 2, (y1 + y2) / 2);
-    return split;
+// The pass was counted with the crossings' ties (remesh_count_block): K
+// connections to split.  It runs unless it would overflow a buffer (the host
+// runs it then; so it does a third pass, remesh_commit_kernel).  New nodes that
+// need the random perturbation are made on the device all the same and listed
+// for the host, which perturbs them before the pass is committed.
+__device__ __forceinline__ bool remesh_fits(const MembraneDev& m, int K, int M, int C) {
+    return M + K <= m.Mcap && C + K <= m.Ccap;
 }
 
-// Pass decision.  Each block counts its connections to split (t.flag[block])
-// and the new nodes that need the random generator (T->nRng); the last block
-// to finish forms the exclusive prefix of the block counts (t.rank[block]),
-// and decides: K = the total, or 0 with a halt when the pass would overflow a
-// buffer (the host runs it then; so it does a third pass,
-// remesh_commit_kernel).  New nodes that need the random perturbation are
-// made on the device all the same and listed for the host, which perturbs
-// them before the pass is committed (remesh_commit_kernel).
-__global__ void __launch_bounds__(kRemeshBlock) remesh_count_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    // a halted step leaves the counts alone (a pass may wait for the host's
-    // perturbation of its new nodes); no block of this kernel raises a halt
-    // before every block has read it, so all blocks return together
-    if (st->halt) return;
-    Topo* T = m.topo;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    bool f = false, rng = false;
-    if (c < T->C) f = remesh_split(m, c, rng);
-    const int cnt = __syncthreads_count(f);
-    const int nr = __syncthreads_count(rng);
-    __shared__ bool last;
-    if (threadIdx.x == 0) {
-        t.flag[blockIdx.x] = cnt;
-        if (nr) atomicAdd(&T->nRng, nr);
-        __threadfence();
-        last = atomicAdd(&T->done, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    // each thread sums a run of consecutive block counts, one block-wide scan
-    // of the runs, then each thread writes its run's prefixes
-    typedef cub::BlockScan<int, kRemeshBlock> Scan;
-    __shared__ typename Scan::TempStorage tmp;
-    const int nb = (int)gridDim.x;
-    const int per = (nb + kRemeshBlock - 1) / kRemeshBlock;
-    const int beg = threadIdx.x * per, end = min(beg + per, nb);
-    int local = 0;
-    for (int b = beg; b < end; ++b) local += __ldcg(&t.flag[b]);
-    int ex, carry;
-    Scan(tmp).ExclusiveSum(local, ex, carry);
-    for (int b = beg; b < end; ++b) {
-        t.rank[b] = ex;
-        ex += __ldcg(&t.flag[b]);
-    }
-    if (threadIdx.x == 0) {
-        const int K = carry, C = T->C, M = T->M;
-        const bool run = K > 0 && M + K <= m.Mcap && C + K <= m.Ccap;
-        T->K = run ? K : 0;
-        if (!run) T->nRng = 0;  // kept for the apply and commit kernels of a pass that runs
-        T->rngFill = 0;
-        T->done = 0;
-        if (K > 0 && !run) raise_halt(st, ST_REMESH);
-    }
-}
-
-// Applies the pass: connection c's rank among the split ones is its block's
-// prefix plus the split connections before it in the block (the same test
-// on the same positions as the count).
+// Applies the pass: connection c's rank among the split ones is the sum of the
+// block counts before its block plus the split connections before it in the
+// block (the same test on the same positions as the count).
 __global__ void __launch_bounds__(kRemeshBlock) remesh_apply_kernel(MembraneDev m, TopoDev t, Status* st) {
     pdl_wait();
     if (st->halt) return;
@@ -181,17 +105,29 @@ __global__ void __launch_bounds__(kRemeshBlock) remesh_apply_kernel(MembraneDev 
     const int K = T->K;
     if (K == 0) return;
     const int C = T->C, M = T->M;
+    if (!remesh_fits(m, K, M, C)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_REMESH);
+        return;
+    }
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     bool rng = false;
     const bool f = c < C && remesh_split(m, c, rng);
     const unsigned bal = __ballot_sync(0xffffffffu, f);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    __shared__ int wsum[kRemeshBlock / 32];
-    if (lane == 0) wsum[w] = __popc(bal);
+    __shared__ int wsum[kRemeshBlock / 32], wbefore[kRemeshBlock / 32];
+    int before = 0;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += kRemeshBlock) before += t.flag[b];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) {
+        wsum[w] = __popc(bal);
+        wbefore[w] = before;
+    }
     __syncthreads();
     if (c >= C) return;
-    int r = t.rank[blockIdx.x] + __popc(bal & ((1u << lane) - 1u));
+    int r = __popc(bal & ((1u << lane) - 1u));
     for (int i = 0; i < w; ++i) r += wsum[i];
+#pragma unroll
+    for (int i = 0; i < kRemeshBlock / 32; ++i) r += wbefore[i];
     if (!f) {
         const int dst = c - r;
         t.ca2[dst] = m.ca[c]; t.cb2[dst] = m.cb[c]; t.cdom2[dst] = m.cdom[c]; t.cdesc2[dst] = m.cdesc[c];
@@ -228,11 +164,29 @@ __global__ void __launch_bounds__(kRemeshBlock) remesh_apply_kernel(MembraneDev 
 //    by the host where needed) and the edge test of connectGeometryNodesToPhysicalNodes
 //    (GeometryHandler.cpp:618-644).  The nodes that existed before the pass
 //    were bound, and tested, by the crossing stage from the same positions.
-__global__ void remesh_commit_kernel(MembraneDev m, TopoDev t, int nx, int ny, Status* st) {
+// areaAcc != nullptr (FP32-shifted steps without coarsening): the kernel also
+// adds the shoelace terms of the final connection list to the cells'
+// fixed-point sums (a kernel of its own otherwise: 3.9 us at 150k connections).
+__global__ void __launch_bounds__(256) remesh_commit_kernel(MembraneDev m, TopoDev t, int nx, int ny, Status* st,
+                                                            unsigned long long* areaAcc) {
     pdl_wait();
     Topo* T = m.topo;
     const int K = T->K;
-    if (K == 0) return;
+    const int stage = st->halt ? st->haltStage : 0;
+    if (K == 0) {
+        if (areaAcc != nullptr && stage == 0)
+            area_terms_fixed(m, blockIdx.x * blockDim.x + threadIdx.x, T->C, m.ca, m.cb, m.cdom, t.cellOfDom,
+                             t.nDomains, areaAcc);
+        return;
+    }
+    if ((stage != 0 && stage < ST_REMESH) || !remesh_fits(m, K, T->M, T->C)) {
+        // halted before the pass was applied, or handed to the host: not run
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            T->K = 0;
+            T->nRng = 0;
+        }
+        return;
+    }
     if (T->nRng > 0) {
         // new nodes wait for the host's perturbation; the step resumes here
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_REMESH_RNG);
@@ -256,6 +210,7 @@ __global__ void remesh_commit_kernel(MembraneDev m, TopoDev t, int nx, int ny, S
         else if (X + 2.0 > nx) raise_error(st, ERR_EDGE_E, i, ST_REMESH);
         else if (Y + 2.0 > ny) raise_error(st, ERR_EDGE_N, i, ST_REMESH);
     }
+    if (areaAcc != nullptr) area_terms_fixed(m, c, C + K, t.ca2, t.cb2, t.cdom2, t.cellOfDom, t.nDomains, areaAcc);
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -270,18 +225,17 @@ __global__ void remesh_commit_kernel(MembraneDev m, TopoDev t, int nx, int ny, S
     }
 }
 
-int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly) {
+int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly,
+                  unsigned long long* areaAcc) {
     if (m.Ccap == 0) return 0;
     int n = 0;
     if (!commitOnly) {
         // the count and the apply kernel partition the connections alike
-        const int cb = (m.Ccap + kRemeshBlock - 1) / kRemeshBlock;
-        launch_pdl(remesh_count_kernel, cb, kRemeshBlock, 0, s, m, t, st);
-        launch_pdl(remesh_apply_kernel, cb, kRemeshBlock, 0, s, m, t, st);
-        n = 2;
+        launch_pdl(remesh_apply_kernel, (m.Ccap + kRemeshBlock - 1) / kRemeshBlock, kRemeshBlock, 0, s, m, t, st);
+        n = 1;
     }
     // a pass runs only when C + K <= Ccap: this grid covers the new list
-    launch_pdl(remesh_commit_kernel, (m.Ccap + 255) / 256, 256, 0, s, m, t, nx, ny, st);
+    launch_pdl(remesh_commit_kernel, (m.Ccap + 255) / 256, 256, 0, s, m, t, nx, ny, st, areaAcc);
     return n + 1;
 }
 
@@ -630,87 +584,144 @@ int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
 // ---------------------------------------------------------------------------
 // Rings
 
-__global__ void ring_first_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (!m.topo->changed) return;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.topo->C) return;
-    t.outConn[m.ca[c]] = c;
-    agg_min(&t.firstConn[m.cdom[c]], (int)m.cdom[c], c);
-}
-
-__global__ void ring_count_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (!m.topo->changed) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.topo->M) return;
-    const int cell = t.cellOfDom[m.cdom[t.outConn[i]]];
-    agg_add(&t.cellCount[cell], cell);
-}
-
-__global__ void ring_fill_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (!m.topo->changed) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.topo->M) return;
-    const uint32_t d = m.cdom[t.outConn[i]];
-    const int cell = t.cellOfDom[d];
-    const int k = agg_add(&t.cellFill[cell], cell);
-    t.members[t.cellStart[cell] + k] = i;
-    const int start = m.cb[t.firstConn[d]];
-    // break the ring before its start node: the node whose successor is the start is last
-    t.succ[i] = m.next[i] == start ? -1 : m.next[i];
-    t.dist[i] = m.next[i] == start ? 0 : 1;
-}
-
 constexpr int kRingPerThread = 16;  // 256 threads x 16 = 4096 nodes per ring
+constexpr int kRingMax = 256 * kRingPerThread;
+constexpr int kRingBlocks = 296;
 
-__global__ void __launch_bounds__(256) ring_rank_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (!m.topo->changed) return;
-    const int cell = blockIdx.x;
-    const int b = t.cellStart[cell], len = t.cellCount[cell];
-    if (len > 256 * kRingPerThread) {
-        if (threadIdx.x == 0) raise_error(st, ERR_CAPACITY, cell, ST_BIO);
-        return;
-    }
-    int ns[kRingPerThread], nd[kRingPerThread];
-    for (int round = 0; (1 << round) < len; ++round) {
-        for (int k = 0; k < kRingPerThread; ++k) {
-            const int idx = threadIdx.x + k * 256;
-            if (idx >= len) break;
-            const int i = t.members[b + idx];
-            const int sc = t.succ[i];
-            if (sc >= 0) { nd[k] = t.dist[i] + t.dist[sc]; ns[k] = t.succ[sc]; }
-            else { nd[k] = t.dist[i]; ns[k] = -1; }
+// All blocks of the launch meet (a cooperative launch: they are resident).
+// The wait is bounded; a block that gives up raises the error and goes on.
+__device__ void ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        meet += gridDim.x;
+        __threadfence();
+        atomicAdd(t.ringMeet, 1u);
+        unsigned tries = 0;
+        while ((int)(*(volatile unsigned*)t.ringMeet - meet) < 0) {
+            __nanosleep(64);
+            if (++tries > 4000000u) {
+                raise_error(st, ERR_STATE, (int)blockIdx.x, ST_BIO);
+                break;
+            }
         }
-        __syncthreads();
-        for (int k = 0; k < kRingPerThread; ++k) {
-            const int idx = threadIdx.x + k * 256;
-            if (idx >= len) break;
-            const int i = t.members[b + idx];
-            t.succ[i] = ns[k];
-            t.dist[i] = nd[k];
-        }
-        __syncthreads();
+        __threadfence();
     }
-    for (int k = 0; k < kRingPerThread; ++k) {
-        const int idx = threadIdx.x + k * 256;
-        if (idx >= len) break;
-        const int i = t.members[b + idx];
-        const int d = t.dist[i];
-        if (d >= 0 && d < len) m.ringNode[b + (len - 1 - d)] = i;
-        else raise_error(st, ERR_STATE, i, ST_BIO);
-    }
-    if (threadIdx.x == 0) m.ringStart[cell] = b;
-    if (threadIdx.x == 0 && cell == gridDim.x - 1) m.ringStart[cell + 1] = b + len;
+    __syncthreads();
 }
 
-__global__ void ring_done_kernel(MembraneDev m, TopoDev t) {
-    pdl_wait();
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d < t.nDomains) t.firstConn[d] = 0x7fffffff;
-    if (d == 0) m.topo->changed = 0;
+// The ring order after a topology change, in one launch: a step whose topology
+// did not change (the usual one) costs one short kernel (1.1 us) instead of
+// seven and two memsets (14 us of an FP64 step).  The ranks are formed in
+// shared memory, over the cell's own places; with the links in global memory a
+// change cost 75 us at 390 cells of 380 nodes (the seven launches 25 us), now
+// 26 us.  Values that other blocks wrote in this launch are read past the L1
+// cache.
+__global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, int nCells, Status* st) {
+    if (!m.topo->changed) return;
+    const int M = m.topo->M, C = m.topo->C;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
+    unsigned meet = *(volatile unsigned*)&t.ringMeet[1];  // arrivals of the launches before this one
+    for (int c = tid; c <= nCells; c += all) {
+        t.cellCount[c] = 0;
+        if (c < nCells) t.cellFill[c] = 0;
+    }
+    // a node's outgoing connection, and each domain's first connection
+    for (int c0 = blockIdx.x * blockDim.x; c0 < C; c0 += all) {
+        const int c = c0 + threadIdx.x;
+        if (c < C) {
+            t.outConn[m.ca[c]] = c;
+            agg_min(&t.firstConn[m.cdom[c]], (int)m.cdom[c], c);
+        }
+    }
+    ring_barrier(t, meet, st);
+    for (int i0 = blockIdx.x * blockDim.x; i0 < M; i0 += all) {
+        const int i = i0 + threadIdx.x;
+        if (i < M) {
+            const int cell = t.cellOfDom[m.cdom[__ldcg(&t.outConn[i])]];
+            agg_add(&t.cellCount[cell], cell);
+        }
+    }
+    ring_barrier(t, meet, st);
+    if (blockIdx.x == 0) {  // the cells' places: an exclusive prefix of their counts
+        typedef cub::BlockScan<int, 256> Scan;
+        __shared__ typename Scan::TempStorage tmp;
+        const int per = (nCells + 1 + 255) / 256;
+        const int beg = min((int)threadIdx.x * per, nCells + 1), end = min(beg + per, nCells + 1);
+        int local = 0, ex;
+        for (int c = beg; c < end; ++c) local += __ldcg(&t.cellCount[c]);
+        Scan(tmp).ExclusiveSum(local, ex);
+        for (int c = beg; c < end; ++c) {
+            t.cellStart[c] = ex;
+            ex += __ldcg(&t.cellCount[c]);
+        }
+    }
+    ring_barrier(t, meet, st);
+    for (int i0 = blockIdx.x * blockDim.x; i0 < M; i0 += all) {
+        const int i = i0 + threadIdx.x;
+        if (i < M) {
+            const uint32_t d = m.cdom[__ldcg(&t.outConn[i])];
+            const int cell = t.cellOfDom[d];
+            const int k = agg_add(&t.cellFill[cell], cell);
+            t.members[__ldcg(&t.cellStart[cell]) + k] = i;
+            const int start = m.cb[__ldcg(&t.firstConn[d])];
+            // break the ring before its start node: the node whose successor is the start is last
+            t.succ[i] = m.next[i] == start ? -1 : m.next[i];
+            t.dist[i] = k;  // the node's place among its cell's members
+        }
+    }
+    ring_barrier(t, meet, st);
+    // each ring's ranks by pointer jumping, one block per cell
+    __shared__ int sNext[kRingMax], sDist[kRingMax];  // by place: the next node's place (-1: none), the links to the end
+    for (int cell = blockIdx.x; cell < nCells; cell += gridDim.x) {
+        const int b = __ldcg(&t.cellStart[cell]), len = __ldcg(&t.cellCount[cell]);
+        if (len > kRingMax) {
+            if (threadIdx.x == 0) raise_error(st, ERR_CAPACITY, cell, ST_BIO);
+            continue;
+        }
+        __syncthreads();
+        for (int p = threadIdx.x; p < len; p += 256) {
+            const int next = __ldcg(&t.succ[__ldcg(&t.members[b + p])]);
+            const int q = next >= 0 ? __ldcg(&t.dist[next]) : -1;
+            // a ring that leaves its cell has no order: its nodes' ranks fall outside and are reported
+            const bool own = next < 0 || t.cellOfDom[m.cdom[__ldcg(&t.outConn[next])]] == cell;
+            sNext[p] = own && q < len ? q : -1;
+            sDist[p] = own ? (next >= 0 ? 1 : 0) : kRingMax;
+        }
+        __syncthreads();
+        for (int round = 0; (1 << round) < len; ++round) {
+            int ns[kRingPerThread], nd[kRingPerThread];
+#pragma unroll
+            for (int k = 0; k < kRingPerThread; ++k) {
+                const int p = threadIdx.x + k * 256;
+                if (p >= len) break;
+                const int q = sNext[p];
+                nd[k] = sDist[p] + (q >= 0 ? sDist[q] : 0);
+                ns[k] = q >= 0 ? sNext[q] : -1;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kRingPerThread; ++k) {
+                const int p = threadIdx.x + k * 256;
+                if (p >= len) break;
+                sNext[p] = ns[k];
+                sDist[p] = nd[k];
+            }
+            __syncthreads();
+        }
+        for (int p = threadIdx.x; p < len; p += 256) {
+            const int i = __ldcg(&t.members[b + p]);
+            const int d = sDist[p];
+            if (d >= 0 && d < len) m.ringNode[b + (len - 1 - d)] = i;
+            else raise_error(st, ERR_STATE, i, ST_BIO);
+        }
+        if (threadIdx.x == 0) m.ringStart[cell] = b;
+        if (threadIdx.x == 0 && cell == nCells - 1) m.ringStart[cell + 1] = b + len;
+    }
+    for (int d = tid; d < t.nDomains; d += all) t.firstConn[d] = 0x7fffffff;
+    if (tid == 0) {
+        t.ringMeet[1] = meet;
+        m.topo->changed = 0;  // every block has read it: it met the others since
+    }
 }
 
 // The listed connections to perturb (crossings_kernel, t.rngList), each
@@ -754,16 +765,19 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
 int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
     const int nCells = t.nCellsCap;
     if (m.Mcap == 0 || nCells == 0) return 0;
-    const int mb = (m.Mcap + 255) / 256, cbk = (m.Ccap + 255) / 256;
-    cudaMemsetAsync(t.cellCount, 0, sizeof(int) * (nCells + 1), s);
-    cudaMemsetAsync(t.cellFill, 0, sizeof(int) * nCells, s);
-    launch_pdl(ring_first_kernel, cbk, 256, 0, s, m, t, st);
-    launch_pdl(ring_count_kernel, mb, 256, 0, s, m, t, st);
-    cub::DeviceScan::ExclusiveSum(t.scanTmp, t.scanTmpBytes, t.cellCount, t.cellStart, nCells + 1, s);
-    launch_pdl(ring_fill_kernel, mb, 256, 0, s, m, t, st);
-    launch_pdl(ring_rank_kernel, nCells, 256, 0, s, m, t, st);
-    launch_pdl(ring_done_kernel, (t.nDomains + 255) / 256, 256, 0, s, m, t);
-    return 7;
+    // two blocks per SM at most: never more than are resident together
+    const int blocks = std::min(kRingBlocks, std::max(nCells, (std::max(m.Mcap, m.Ccap) + 255) / 256));
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, rings_kernel, m, t, nCells, st);
+    return 1;
 }
 
 }  // namespace lbib

@@ -12,10 +12,10 @@ struct Topo {
     int C;            // connections
     unsigned maxId;   // id of the last node (ids ascend with the index)
     int changed;      // the topology changed: rings must be rebuilt
-    int K;            // connections split by the current remesh pass
+    int K;            // connections that the current remesh pass splits (counted with the crossings)
     int removed;      // nodes removed by the current coarsening
     int nCand;        // coarsening candidates
-    unsigned done;    // blocks of the remesh count / copy that have finished (the last one decides / commits)
+    unsigned done;    // blocks of the remesh copy that have finished (the last one commits)
     int nRng;         // new nodes of the remesh pass that need the random perturbation
     int rngFill;      // entries of TopoDev::rngList (those nodes' indices)
 };
@@ -156,6 +156,7 @@ struct TopoDev {
     int* succ; int* dist;                                 // Mcap
     int* rngList;       // Mcap: new nodes of a remesh pass that need the host's random perturbation
     int* startNode;     // nCells
+    unsigned* ringMeet; // rings_kernel: [0] arrivals at its barriers, ever; [1] those of the launches that are through
     void* scanTmp; size_t scanTmpBytes;
     int nDomains;
 };
@@ -188,11 +189,12 @@ void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny
 template <typename Real>
 void launch_interp_move(const MembraneDev& m, const Real* u, int nx, int ny, size_t L, CrossDev& c, Status* st,
                         unsigned iteration, cudaStream_t s);
+// The crossings, and (remesh != nullptr) the count of the step's remeshing pass.
 // `check`: first raise the halts of the move's listed nodes and of connections
 // that need the host's perturbation (listed in perturb[0..perturbCap)).
 template <typename Real>
 void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, size_t L, Status* st,
-                      unsigned iteration, cudaStream_t s, bool check = false, int* perturb = nullptr,
+                      const TopoDev* remesh, cudaStream_t s, bool check = false, int* perturb = nullptr,
                       int perturbCap = 0);
 template <typename Real>
 void launch_reinit(CrossDev& c, uint32_t* dom, Real* g, const Real* u, int nS, const SpeciesConst* sp,
@@ -242,9 +244,11 @@ void launch_areas_fixed(const MembraneDev& m, const int* cellOfDom, int nDomains
                         double* area, cudaStream_t s);
 // FP32-shifted runs: areas from the connections in fixed point (no ring order
 // needed), then the regulator.  acc (nCells) must start at zero; it is left zero.
+// summed: the remeshing commit formed the sums already.
 void launch_area_regulator_fixed(const MembraneDev& m, const int* cellOfDom, unsigned long long* acc, double* area,
                                  double* target, double* massTab, int nDomains, double factor, double strength,
-                                 double maxsource, const uint32_t* ctypeTab, const Status* st, cudaStream_t s);
+                                 double maxsource, const uint32_t* ctypeTab, const Status* st, cudaStream_t s,
+                                 bool summed = false);
 // massNode[n] = massTab[dom[n]] (0 outside cells).
 void launch_mass_expand(const uint32_t* dom, size_t L, const double* massTab, int nDomains, double* massNode,
                         const Status* st, cudaStream_t s);
@@ -273,9 +277,11 @@ struct ConnPerturbRec {
 };
 void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, ConnPerturbRec* out, cudaStream_t s);
 
-// A remesh pass (count, apply, commit); commitOnly: the commit alone, after
-// the host perturbed the pass's new nodes (halt ST_REMESH_RNG).
-int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly = false);
+// A remesh pass, counted with the crossings (apply, commit); commitOnly: the
+// commit alone, after the host perturbed the pass's new nodes (halt
+// ST_REMESH_RNG).  areaAcc: also add the shoelace terms of the final list.
+int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly = false,
+                  unsigned long long* areaAcc = nullptr);
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
 int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
 size_t topo_scan_bytes(int n);

@@ -466,7 +466,7 @@ Handle::~Handle() {
     fr(td.dalt); fr(td.id2); fr(td.prev2); fr(td.next2); fr(td.inConn); fr(td.outConn); fr(td.removed);
     fr(td.connAlive); fr(td.ncA); fr(td.ncB); fr(td.ncDom); fr(td.ncDesc); fr(td.ncAlive); fr(td.cellOfDom);
     fr(td.firstConn); fr(td.cellCount); fr(td.cellStart); fr(td.cellFill); fr(td.members); fr(td.succ); fr(td.rngList);
-    fr(td.dist); fr(td.startNode); fr(td.scanTmp);
+    fr(td.dist); fr(td.startNode); fr(td.scanTmp); fr(td.ringMeet);
     fr(st);
     if (stHost) cudaFreeHost(stHost);  // topoHost lives in the same block
     if (evA) cudaEventDestroy(evA);
@@ -1433,7 +1433,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
     }
     if (fromStage <= ST_CROSSINGS) {
         // ST_PERTURB_CONN: the test runs with the crossings
-        launch_crossings<Real>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, it, s, fromStage <= ST_PERTURB_CONN,
+        launch_crossings<Real>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, &h.td, s, fromStage <= ST_PERTURB_CONN,
                                h.td.rngList, h.Mcap);
         nl += hasM ? 3 : 0;
     }
@@ -1448,8 +1448,13 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
         launch_domain_fill(h.cross, h.dom, h.nx, h.ny, h.L, h.st, it, s);
         nl += 1;
     }
+    // the FP32-shifted area sums ride on the remeshing commit, whose list is
+    // the step's last unless it coarsens
+    const bool area = std::find(h.bio.begin(), h.bio.end(), 2) != h.bio.end();
+    const bool summed = sizeof(Real) == 4 && area && h.m.nCells > 0 && !coarsenStep && fromStage <= ST_REMESH_COMMIT;
     if (fromStage <= ST_REMESH_COMMIT)
-        nl += launch_remesh(h.m, h.td, h.nx, h.ny, h.st, s, fromStage == ST_REMESH_COMMIT);
+        nl += launch_remesh(h.m, h.td, h.nx, h.ny, h.st, s, fromStage == ST_REMESH_COMMIT,
+                            summed ? h.areaAcc : nullptr);
     if (fromStage <= ST_COARSEN && coarsenStep) {
         // SimulationRunner.cpp:84-87: ForceSolver::deleteAllForces, then coarsenBoundary
         launch_clear_forces(h.m, s);
@@ -1471,8 +1476,8 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
                     nl += h.m.nCells > 0 ? 2 : 0;
                 } else {
                     launch_area_regulator_fixed(h.m, h.td.cellOfDom, h.areaAcc, h.area, h.target, h.massTab,
-                                                h.nDomains, h.areaFactor, h.areaStrength, h.areaMax, ct, h.st, s);
-                    nl += h.m.nCells > 0 ? 2 : 0;
+                                                h.nDomains, h.areaFactor, h.areaStrength, h.areaMax, ct, h.st, s, summed);
+                    nl += h.m.nCells > 0 ? (summed ? 1 : 2) : 0;
                 }
                 if (h.massNode != nullptr) {
                     launch_mass_expand(h.dom, h.L, h.massTab, h.nDomains, h.massNode, h.st, s);
@@ -2083,6 +2088,9 @@ static void create(Handle& h, const std::string& params, const std::string& geom
     CK(cudaMemsetAsync(h.tiles.count, 0, sizeof(int) * h.tiles.nTiles, h.stream));
     CK(cudaMemsetAsync(h.tiles.active, 0, sizeof(int) * h.tiles.nTiles, h.stream));
 
+    h.td.ringMeet = dalloc<unsigned>(2);
+    CK(cudaMemsetAsync(h.td.ringMeet, 0, 2 * sizeof(unsigned), h.stream));
+
     // crossing planes
     h.cross.bnDist = dalloc<unsigned long long>(4 * h.L);
     h.cross.bnConn = dalloc<uint32_t>(4 * h.L);
@@ -2292,8 +2300,8 @@ static void cure_lattice(Handle& h, HostMembrane& hm) {
     std::memset(h.stHost, 0, sizeof(Status));
     write_status(h);
     launch_edge_check(h.m, h.nx, h.ny, h.st, 0, h.stream);
-    if (h.precision == LBIB_FP64) launch_crossings<double>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, 0, h.stream);
-    else launch_crossings<float>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, 0, h.stream);
+    if (h.precision == LBIB_FP64) launch_crossings<double>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, nullptr, h.stream);
+    else launch_crossings<float>(h.m, h.cross, h.dom, h.nx, h.ny, h.L, h.st, nullptr, h.stream);
     launch_domain_fill(h.cross, h.dom, h.nx, h.ny, h.L, h.st, 0, h.stream);
     // the crossings mark the nodes whose domain they change; at set-up no
     // re-initialisation follows to clear the marks
