@@ -62,79 +62,133 @@ __device__ __forceinline__ double dirac(const double dx, const double dy) {
 
 // ---------------------------------------------------------------------------
 // Force evaluation
-__device__ __forceinline__ int tile_agg_add(int* arr, int tile, bool valid);
-__device__ void tile_slot_node(const MembraneDev& m, TileDev& t, int i, bool ok, int nx, int ny, Status* st);
+
+// The force of one record on the node at (x1, y1) (ForceStructs.hpp:49-588),
+// added to (Fx, Fy); p0 is the record's first parameter, p its four, (x2, y2)
+// the partner's position (types 0, 5, 6, 7).
+__device__ __forceinline__ void add_force(int type, double p0, const double* p, double x1, double y1, double x2,
+                                          double y2, double& Fx, double& Fy) {
+    switch (type) {
+        case 0: case 7: {  // spring between two nodes: f = k(|d| - l0), along d
+            const double dist = sqrt((x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1));
+            const double f = p0 * (dist - p[1]);
+            Fx += ((x2 - x1) * f) / dist;
+            Fy += ((y2 - y1) * f) / dist;
+            break;
+        }
+        case 1: {  // anchor spring to (x, y)
+            const double tx = p0, ty = p[1];
+            const double dist = sqrt((tx - x1) * (tx - x1) + (ty - y1) * (ty - y1));
+            const double f = p[2] * (dist - p[3]);
+            if (dist != 0.0) {
+                Fx += ((tx - x1) * f) / dist;
+                Fy += ((ty - y1) * f) / dist;
+            }
+            break;
+        }
+        case 2:  // constant force
+            Fx += p0;
+            Fy += p[1];
+            break;
+        case 3: {  // horizontal slider at y
+            const double dist = sqrt((x1 - x1) * (x1 - x1) + (p0 - y1) * (p0 - y1));
+            const double f = p[1] * (dist - p[2]);
+            Fx += 0.0;
+            Fy += (y1 < p0) ? f : -f;
+            break;
+        }
+        case 4: {  // vertical slider at x
+            const double dist = sqrt((p0 - x1) * (p0 - x1) + (y1 - y1) * (y1 - y1));
+            const double f = p[1] * (dist - p[2]);
+            Fx += (x1 < p0) ? f : -f;
+            Fy += 0.0;
+            break;
+        }
+        default: {  // 5, 6: constant-magnitude pull toward the partner
+            const double dist = sqrt((x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1));
+            Fx += ((x2 - x1) * p0) / dist;
+            Fy += ((y2 - y1) * p0) / dist;
+            break;
+        }
+    }
+}
+
+// A node's entries in the slot lists of the (up to 2 x 2) tiles its stencil
+// covers.  The lanes of a warp that enter the same tile share one atomic;
+// tile_slots_take issues the four rounds' atomics, tile_slots_put, which
+// waits for them, stores the entries: what stands between the two hides the
+// round trips.  All lanes of the warp take part in both.
+struct TileSlots {
+    int tile[4];
+    int base[4];
+    unsigned group[4];
+};
+__device__ __forceinline__ TileSlots tile_slots_take(const MembraneDev& m, const TileDev& t, int i, bool ok, int nx, int ny,
+                                     Status* st);
+__device__ __forceinline__ void tile_slots_put(const TileDev& t, const TileSlots& s, int i, Status* st);
 
 // `begin`: the first kernel of a step (begin_step).
 // `slots`: also enter the node in the per-tile lists of the spread (which left
 // the tile counts at zero).
-__global__ void force_eval_kernel(MembraneDev m, Status* st, unsigned iteration, int begin, TileDev t, int nx,
-                                  int ny, int slots) {
+// Two records are read ahead (a membrane node has two tension records), and the
+// slot lists' atomics are under way meanwhile: 5.5 -> 4.0 us for one cell, 8.3 ->
+// 6.3 us for 150k nodes.
+__global__ void __launch_bounds__(128) force_eval_kernel(MembraneDev m, Status* st, unsigned iteration, int begin,
+                                                         TileDev t, int nx, int ny, int slots) {
     pdl_wait();
     if (st->halt) return;
     if (begin && blockIdx.x == 0 && threadIdx.x == 0) begin_step(st);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.topo->M) return;
-    const double x1 = m.x[i], y1 = m.y[i];
-    double Fx = 0.0, Fy = 0.0;
-    const int r0 = m.foff[i], r1 = m.foff[i + 1];
-    for (int r = r0; r < r1; ++r) {
-        const int type = m.ftype[r];
-        const double* p = m.fpar + 4 * (size_t)r;
-        const int j = m.fpartner[r];
-        if ((type == 0 || type == 7 || type == 5 || type == 6) && (j < 0 || j >= m.topo->M)) {
-            raise_error(st, ERR_FORCE_NODE, i, ST_FORCE);
-            return;
-        }
-        switch (type) {
-            case 0: case 7: {  // spring between two nodes: f = k(|d| - l0), along d
-                const double x2 = m.x[j], y2 = m.y[j];
-                const double dist = sqrt((x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1));
-                const double f = p[0] * (dist - p[1]);
-                Fx += ((x2 - x1) * f) / dist;
-                Fy += ((y2 - y1) * f) / dist;
-                break;
-            }
-            case 1: {  // anchor spring to (x, y)
-                const double tx = p[0], ty = p[1];
-                const double dist = sqrt((tx - x1) * (tx - x1) + (ty - y1) * (ty - y1));
-                const double f = p[2] * (dist - p[3]);
-                if (dist != 0.0) {
-                    Fx += ((tx - x1) * f) / dist;
-                    Fy += ((ty - y1) * f) / dist;
-                }
-                break;
-            }
-            case 2:  // constant force
-                Fx += p[0];
-                Fy += p[1];
-                break;
-            case 3: {  // horizontal slider at y
-                const double dist = sqrt((x1 - x1) * (x1 - x1) + (p[0] - y1) * (p[0] - y1));
-                const double f = p[1] * (dist - p[2]);
-                Fx += 0.0;
-                Fy += (y1 < p[0]) ? f : -f;
-                break;
-            }
-            case 4: {  // vertical slider at x
-                const double dist = sqrt((p[0] - x1) * (p[0] - x1) + (y1 - y1) * (y1 - y1));
-                const double f = p[1] * (dist - p[2]);
-                Fx += (x1 < p[0]) ? f : -f;
-                Fy += 0.0;
-                break;
-            }
-            default: {  // 5, 6: constant-magnitude pull toward the partner
-                const double x2 = m.x[j], y2 = m.y[j];
-                const double dist = sqrt((x2 - x1) * (x2 - x1) + (y2 - y1) * (y2 - y1));
-                Fx += ((x2 - x1) * p[0]) / dist;
-                Fy += ((y2 - y1) * p[0]) / dist;
-                break;
-            }
-        }
+    const int M = m.topo->M;
+    if (i - (int)(threadIdx.x & 31) >= M) return;  // the whole warp
+    bool live = i < M;
+    int r0 = 0, r1 = 0;
+    double x1 = 0.0, y1 = 0.0;
+    if (live) {
+        x1 = m.x[i];
+        y1 = m.y[i];
+        r0 = m.foff[i];
+        r1 = m.foff[i + 1];
     }
-    m.fx[i] = Fx;
-    m.fy[i] = Fy;
-    if (slots) tile_slot_node(m, t, i, true, nx, ny, st);
+    TileSlots ts;
+    if (slots) ts = tile_slots_take(m, t, i, live, nx, ny, st);
+    double Fx = 0.0, Fy = 0.0;
+    for (int r = r0; r < r1; r += 2) {
+        int type[2], j[2];
+        double p0[2], x2[2] = {0.0, 0.0}, y2[2] = {0.0, 0.0};
+        bool pair[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int rq = r + q < r1 ? r + q : r;
+            type[q] = m.ftype[rq];
+            j[q] = m.fpartner[rq];
+            p0[q] = m.fpar[4 * (size_t)rq];
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            pair[q] = type[q] == 0 || type[q] == 7 || type[q] == 5 || type[q] == 6;
+            if (pair[q] && j[q] >= 0 && j[q] < M) {
+                x2[q] = m.x[j[q]];
+                y2[q] = m.y[j[q]];
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            if (!live || r + q >= r1) break;
+            if (pair[q] && (j[q] < 0 || j[q] >= M)) {
+                raise_error(st, ERR_FORCE_NODE, i, ST_FORCE);
+                live = false;
+                break;
+            }
+            add_force(type[q], p0[q], m.fpar + 4 * (size_t)(r + q), x1, y1, x2[q], y2[q], Fx, Fy);
+        }
+        if (!live) break;
+    }
+    if (live) {
+        m.fx[i] = Fx;
+        m.fy[i] = Fy;
+    }
+    if (slots) tile_slots_put(t, ts, i, st);
 }
 
 // dL/d of every force record's parameters from dL/dF of the node forces
@@ -273,36 +327,37 @@ __device__ __forceinline__ void stencil_slot(const Stencil& s, int k, int& xk, i
             if (((4 * x + y) & 15) == k) { xk = x; yk = y; }
 }
 
-// Lanes with the same tile share one atomic.
-__device__ __forceinline__ int tile_agg_add(int* arr, int tile, bool valid) {
-    const unsigned act = __activemask();
-    const unsigned grp = __match_any_sync(act, valid ? tile : -1);
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(grp) - 1;
-    int base = 0;
-    if (valid && lane == leader) base = atomicAdd(&arr[tile], __popc(grp));
-    base = __shfl_sync(grp, base, leader);
-    return base + __popc(grp & ((1u << lane) - 1u));
-}
-
-// Node i into the fixed-size slot lists of the (up to 2 x 2) tiles its stencil
-// covers.
-__device__ void tile_slot_node(const MembraneDev& m, TileDev& t, int i, bool ok, int nx, int ny, Status* st) {
+__device__ __forceinline__ TileSlots tile_slots_take(const MembraneDev& m, const TileDev& t, int i, bool ok, int nx,
+                                                     int ny, Status* st) {
     Stencil sc{0, 0, 0, 0};
     if (ok && !stencil_range(m.bx[i], m.by[i], nx, ny, sc)) {
         raise_error(st, ERR_STENCIL, i, ST_SPREAD);
         ok = false;
     }
     const int tx0 = sc.x0 / kTile, tx1 = sc.x1 / kTile, ty0 = sc.y0 / kTile, ty1 = sc.y1 / kTile;
+    const int lane = threadIdx.x & 31;
+    TileSlots s;
+#pragma unroll
     for (int j = 0; j < 4; ++j) {
         const int tx = tx0 + (j & 1), ty = ty0 + (j >> 1);
-        const bool v = ok && tx <= tx1 && ty <= ty1;
-        const int tile = v ? ty * t.tilesX + tx : -1;
-        const int slot = tile_agg_add(t.count, tile, v);
-        if (v) {
-            if (slot < kTileSlots) t.slots[(size_t)tile * kTileSlots + slot] = i;
-            else raise_error(st, ERR_CAPACITY, tile, ST_SPREAD);
-        }
+        s.tile[j] = ok && tx <= tx1 && ty <= ty1 ? ty * t.tilesX + tx : -1;
+        s.group[j] = __match_any_sync(0xffffffffu, s.tile[j]);
+        s.base[j] = 0;
+        if (s.tile[j] >= 0 && lane == __ffs(s.group[j]) - 1)
+            s.base[j] = atomicAdd(&t.count[s.tile[j]], __popc(s.group[j]));
+    }
+    return s;
+}
+
+__device__ __forceinline__ void tile_slots_put(const TileDev& t, const TileSlots& s, int i, Status* st) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int slot = __shfl_sync(0xffffffffu, s.base[j], __ffs(s.group[j]) - 1) +
+                         __popc(s.group[j] & ((1u << lane) - 1u));
+        if (s.tile[j] < 0) continue;
+        if (slot < kTileSlots) t.slots[(size_t)s.tile[j] * kTileSlots + slot] = i;
+        else raise_error(st, ERR_CAPACITY, s.tile[j], ST_SPREAD);
     }
 }
 
@@ -310,7 +365,7 @@ __global__ void tile_slot_kernel(MembraneDev m, TileDev t, int nx, int ny, Statu
     pdl_wait();
     if (st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    tile_slot_node(m, t, i, i < m.topo->M, nx, ny, st);
+    tile_slots_put(t, tile_slots_take(m, t, i, i < m.topo->M, nx, ny, st), i, st);
 }
 
 // Per-tile entry: the stencil origin relative to the tile (+4) and the stencil
@@ -1130,11 +1185,13 @@ void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, in
     // word before a run and by the first kernel of each step
     launch_pdl(crossings_kernel, blocks, kCrossBlock, 0, s, m, c, nx, ny, st, check ? 1 : 0, perturb, perturbCap);
     // grid-stride over the step's records (their count is known on the device
-    // only): 8 blocks per SM, so that each thread's chain of dependent loads
-    // overlaps many others
-    launch_pdl(cross_tie_kernel, std::max(148 * 8, (m.Ccap + kRemeshBlock - 1) / kRemeshBlock), kRemeshBlock, 0, s, c, m,
+    // only): up to 8 blocks per SM, so that each thread's chain of dependent
+    // loads overlaps many others, and no more than 4 records per connection
+    // fill
+    const int recBlocks = std::min(148 * 8, (4 * m.Ccap + 255) / 256);
+    launch_pdl(cross_tie_kernel, std::max(recBlocks, (m.Ccap + kRemeshBlock - 1) / kRemeshBlock), kRemeshBlock, 0, s, c, m,
                remesh ? *remesh : TopoDev{}, nx, ny, st);
-    launch_pdl(cross_win_kernel, 148 * 8, 256, 0, s, c, m, dom, nx, ny, st);
+    launch_pdl(cross_win_kernel, recBlocks, 256, 0, s, c, m, dom, nx, ny, st);
 }
 template void launch_crossings<double>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
                                        const TopoDev*, cudaStream_t, bool, int*, int);
