@@ -123,8 +123,8 @@ struct TileSlots {
     int base[4];
     unsigned group[4];
 };
-__device__ __forceinline__ TileSlots tile_slots_take(const MembraneDev& m, const TileDev& t, int i, bool ok, int nx, int ny,
-                                     Status* st);
+__device__ __forceinline__ TileSlots tile_slots_take(double bx, double by, const TileDev& t, int i, bool ok, int nx,
+                                                     int ny, Status* st);
 __device__ __forceinline__ void tile_slots_put(const TileDev& t, const TileSlots& s, int i, Status* st);
 
 // `begin`: the first kernel of a step (begin_step).
@@ -136,22 +136,18 @@ __device__ __forceinline__ void tile_slots_put(const TileDev& t, const TileSlots
 __global__ void __launch_bounds__(128) force_eval_kernel(MembraneDev m, Status* st, unsigned iteration, int begin,
                                                          TileDev t, int nx, int ny, int slots) {
     pdl_wait();
-    if (st->halt) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, ic = min(i, m.Mcap - 1);
+    int halt = st->halt, M = m.topo->M;
+    double x1 = m.x[ic], y1 = m.y[ic], bx = m.bx[ic], by = m.by[ic];
+    int r0 = m.foff[ic], r1 = m.foff[ic + 1];
+    read_ahead(halt, M, x1, y1, bx, by, r0, r1);
+    if (halt) return;
     if (begin && blockIdx.x == 0 && threadIdx.x == 0) begin_step(st);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int M = m.topo->M;
     if (i - (int)(threadIdx.x & 31) >= M) return;  // the whole warp
     bool live = i < M;
-    int r0 = 0, r1 = 0;
-    double x1 = 0.0, y1 = 0.0;
-    if (live) {
-        x1 = m.x[i];
-        y1 = m.y[i];
-        r0 = m.foff[i];
-        r1 = m.foff[i + 1];
-    }
+    if (!live) r0 = r1 = 0;
     TileSlots ts;
-    if (slots) ts = tile_slots_take(m, t, i, live, nx, ny, st);
+    if (slots) ts = tile_slots_take(bx, by, t, i, live, nx, ny, st);
     double Fx = 0.0, Fy = 0.0;
     for (int r = r0; r < r1; r += 2) {
         int type[2], j[2];
@@ -327,10 +323,10 @@ __device__ __forceinline__ void stencil_slot(const Stencil& s, int k, int& xk, i
             if (((4 * x + y) & 15) == k) { xk = x; yk = y; }
 }
 
-__device__ __forceinline__ TileSlots tile_slots_take(const MembraneDev& m, const TileDev& t, int i, bool ok, int nx,
+__device__ __forceinline__ TileSlots tile_slots_take(double bx, double by, const TileDev& t, int i, bool ok, int nx,
                                                      int ny, Status* st) {
     Stencil sc{0, 0, 0, 0};
-    if (ok && !stencil_range(m.bx[i], m.by[i], nx, ny, sc)) {
+    if (ok && !stencil_range(bx, by, nx, ny, sc)) {
         raise_error(st, ERR_STENCIL, i, ST_SPREAD);
         ok = false;
     }
@@ -365,7 +361,8 @@ __global__ void tile_slot_kernel(MembraneDev m, TileDev t, int nx, int ny, Statu
     pdl_wait();
     if (st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    tile_slots_put(t, tile_slots_take(m, t, i, i < m.topo->M, nx, ny, st), i, st);
+    const bool live = i < m.topo->M;
+    tile_slots_put(t, tile_slots_take(live ? m.bx[i] : 0.0, live ? m.by[i] : 0.0, t, i, live, nx, ny, st), i, st);
 }
 
 // Per-tile entry: the stencil origin relative to the tile (+4) and the stencil
@@ -377,14 +374,17 @@ __device__ __forceinline__ int pack_stencil(const Stencil& s, int tileX0, int ti
 // The tile's list as the spread takes it: its length, noted for the readers of
 // the force field, and the counter left at zero for the next step's lists (a
 // memset node between two kernels of the step cost 3.5 us).
-__device__ __forceinline__ int take_tile_count(const TileDev& t, int tile) {
-    __shared__ int count;
+// -1 on a halted step.  `first`: entry threadIdx.x of the list, if it has one.
+__device__ __forceinline__ int take_tile_count(const TileDev& t, int tile, const Status* st, int& first) {
+    int halt = st->halt, count = t.count[tile];
+    first = t.slots[(size_t)tile * kTileSlots + threadIdx.x];
+    read_ahead(halt, count, first);
+    if (halt) return -1;
+    __syncthreads();
     if (threadIdx.x == 0) {
-        count = t.count[tile];
         t.active[tile] = count;
         if (count != 0) t.count[tile] = 0;
     }
-    __syncthreads();
     return count;
 }
 
@@ -410,10 +410,10 @@ template <typename Real>
 __global__ void __launch_bounds__(256) spread_kernel(MembraneDev m, TileDev t, Real* force, int nx, int ny, size_t L,
                                                      Status* st) {
     pdl_wait();
-    if (st->halt) return;
     const int tile = blockIdx.x;
-    const int cnt = take_tile_count(t, tile);
-    if (cnt == 0) return;
+    int first;
+    const int cnt = take_tile_count(t, tile, st, first);
+    if (cnt <= 0) return;
     if (cnt > kSpreadMax) {
         if (threadIdx.x == 0) raise_error(st, ERR_CAPACITY, tile, ST_SPREAD);
         return;
@@ -428,7 +428,8 @@ __global__ void __launch_bounds__(256) spread_kernel(MembraneDev m, TileDev t, R
         static_assert(sizeof(fac) >= (kSpreadMax + 3) * sizeof(int), "the unsorted list fits the factors' place");
         const int* list = t.slots + (size_t)tile * kTileSlots;
         const int cnt4 = (cnt + 3) & ~3;
-        for (int k = threadIdx.x; k < cnt4; k += blockDim.x) raw[k] = k < cnt ? list[k] : 0x7fffffff;
+        for (int k = threadIdx.x; k < cnt4; k += blockDim.x)
+            raw[k] = k < cnt ? (k < (int)blockDim.x ? first : list[k]) : 0x7fffffff;
         __syncthreads();
         for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
             const int v = raw[k];
@@ -536,10 +537,10 @@ constexpr int kScatterChunk = 256;
 __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDev t, float* force, int nx, int ny,
                                                            size_t L, Status* st) {
     pdl_wait();
-    if (st->halt) return;
     const int tile = blockIdx.x;
-    const int cnt = min(take_tile_count(t, tile), kTileSlots);
-    if (cnt == 0) return;
+    int first;
+    const int cnt = min(take_tile_count(t, tile, st, first), kTileSlots);
+    if (cnt <= 0) return;
     // each 64-bit fixed-point sum is kept as a signed high part (bits 22..63)
     // and an unsigned low part (bits 0..21), each summed with 32-bit integer
     // atomics: the low parts of up to 1024 contributions cannot overflow
@@ -560,7 +561,7 @@ __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDe
         const int nc = min(kScatterChunk, cnt - c0);
         __syncthreads();
         for (int e = threadIdx.x; e < nc; e += blockDim.x) {
-            const int i = list[c0 + e];
+            const int i = c0 == 0 ? first : list[c0 + e];  // (a chunk is a block's threads)
             const double X = m.x[i], Y = m.y[i];
             Stencil sc;
             stencil_range(m.bx[i], m.by[i], nx, ny, sc);
@@ -676,20 +677,16 @@ __global__ void __launch_bounds__(kInterpBlock) interp_move_kernel(MembraneDev m
                                                                    size_t L, CrossDev c, Status* st,
                                                                    unsigned iteration) {
     pdl_wait();
-    if (st->halt) return;
     __shared__ double2 prod[kInterpBlock / 32][16 * 8];
-    const int M = m.topo->M;
     const int lane = threadIdx.x & 31, col = lane & 3, e = lane >> 2;
     double2* p = prod[threadIdx.x >> 5];
-    const int i = blockIdx.x * kInterpNodes + (int)(threadIdx.x >> 2);
-    if (i - e >= M) return;  // the whole warp
+    const int i = blockIdx.x * kInterpNodes + (int)(threadIdx.x >> 2), ic = min(i, m.Mcap - 1);
+    int halt = st->halt, M = m.topo->M;
+    double X = m.x[ic], Y = m.y[ic], bind = (col < 2 ? m.bx : m.by)[ic];
+    read_ahead(halt, M, X, Y, bind);
+    if (halt || i - e >= M) return;  // the whole warp
     const bool live = i < M;
-    double X = 0.0, Y = 0.0, bind = 32.0;
-    if (live) {
-        X = m.x[i];
-        Y = m.y[i];
-        bind = col < 2 ? m.bx[i] : m.by[i];
-    }
+    if (!live) X = Y = bind = 32.0;
     // stencil_range, one of its four bounds per lane
     const int bound = (col & 1) ? (int)floor(bind + 2.0) : (int)ceil(bind - 2.0);
     Stencil sc;
@@ -921,19 +918,21 @@ constexpr int kCrossBlock = 128;
 __global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, CrossDev c, int nx, int ny, Status* st,
                                                                 int check, int* perturb, int perturbCap) {
     pdl_wait();
-    if (st->halt) return;
-    if (check && st->nPerturbNode > 0) {
+    const int cn = blockIdx.x * kCrossBlock + threadIdx.x, cc = min(cn, max(m.Ccap, 1) - 1);
+    const bool any = m.Ccap > 0;  // there are buffers to read from
+    int halt = st->halt, nodes = st->nPerturbNode, C = m.topo->C, a = any ? m.ca[cc] : 0, b = any ? m.cb[cc] : 0;
+    uint32_t D = any ? m.cdom[cc] : 0u;
+    read_ahead(halt, nodes, C, a, b, D);
+    if (halt) return;
+    if (check && nodes > 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
         return;
     }
-    const int cn = blockIdx.x * kCrossBlock + threadIdx.x;
     int nrec = 0;
     bool simple = false;
     CrossRec r[4];
     bool have[4] = {false, false, false, false};
-    if (cn < m.topo->C) {
-        const int a = m.ca[cn], b = m.cb[cn];
-        const uint32_t D = m.cdom[cn];
+    if (cn < C) {
         const double x1 = m.x[a], y1 = m.y[a], x2 = m.x[b], y2 = m.y[b];
         if (check && (fabs(x1 - x2) < kEPSILON || fabs(y1 - y2) < kEPSILON)) {
             const int k = atomicAdd(&st->nPerturbConn, 1);
@@ -1044,19 +1043,28 @@ __device__ __forceinline__ void edge_check_node(const MembraneDev& m, int i, int
 __global__ void __launch_bounds__(kRemeshBlock) cross_tie_kernel(CrossDev c, MembraneDev m, TopoDev t, int nx, int ny,
                                                                  Status* st) {
     pdl_wait();
-    if (st->halt) return;
-    if (st->nPerturbConn > 0) {
+    const int tid = blockIdx.x * kRemeshBlock + threadIdx.x, all = gridDim.x * kRemeshBlock;
+    const int rc = min(tid, c.recCap - 1);
+    int halt = st->halt, conns = st->nPerturbConn, n = st->pad[2], M = m.topo->M;
+    uint32_t key = c.recKey[rc], conn = c.recConn[rc];
+    unsigned long long dist = c.recDist[rc];
+    read_ahead(halt, conns, n, M, key, conn, dist);
+    if (halt) return;
+    if (conns > 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_PERTURB_CONN);
         return;
     }
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.topo->M; i += gridDim.x * blockDim.x)
-        edge_check_node(m, i, nx, ny, st, ST_CROSSINGS);
-    if (t.flag != nullptr) remesh_count_block(m, t);  // (not at set-up)
-    const int n = min(st->pad[2], c.recCap);
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const uint32_t key = c.recKey[r];
-        if (c.bnDist[key] == c.recDist[r]) atomicMin(&c.bnConn[key], c.recConn[r]);
+    n = min(n, c.recCap);
+    for (int r = tid; r < n; r += all) {
+        if (r != tid) {
+            key = c.recKey[r];
+            conn = c.recConn[r];
+            dist = c.recDist[r];
+        }
+        if (c.bnDist[key] == dist) atomicMin(&c.bnConn[key], conn);
     }
+    for (int i = tid; i < M; i += all) edge_check_node(m, i, nx, ny, st, ST_CROSSINGS);
+    if (t.flag != nullptr) remesh_count_block(m, t);  // (not at set-up)
 }
 
 // Pass 2: the winner writes its domain; the winner of a node's last present
@@ -1097,16 +1105,29 @@ __device__ __forceinline__ void record_noflux(const MembraneDev& m, CrossDev& c,
 
 __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom, int nx, int ny, Status* st) {
     pdl_wait();
-    if (st->halt) return;
-    const int n = min(st->pad[2], c.recCap);
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
-        const uint32_t key = c.recKey[r];
-        if (c.bnDist[key] != c.recDist[r] || c.bnConn[key] != c.recConn[r]) continue;
-        const uint32_t bdom = c.recDom[r];
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x, rc = min(tid, c.recCap - 1);
+    int halt = st->halt, n = st->pad[2];
+    uint32_t key = c.recKey[rc], conn = c.recConn[rc], bdom = c.recDom[rc];
+    unsigned long long dist = c.recDist[rc];
+    read_ahead(halt, n, key, conn, bdom, dist);
+    if (halt) return;
+    n = min(n, c.recCap);
+    for (int r = tid; r < n; r += all) {
+        if (r != tid) {
+            key = c.recKey[r];
+            conn = c.recConn[r];
+            bdom = c.recDom[r];
+            dist = c.recDist[r];
+        }
         const size_t node = key >> 2;
         const int s = (int)(key & 3u);
+        // the node's four slots and domain, whether or not the record wins
+        const ulonglong2 d01 = *(const ulonglong2*)(c.bnDist + node * 4), d23 = *(const ulonglong2*)(c.bnDist + node * 4 + 2);
+        const uint32_t winner = c.bnConn[key], old = dom[node];
+        const unsigned long long at[4] = {d01.x, d01.y, d23.x, d23.y};
+        if ((s == 0 ? at[0] : s == 1 ? at[1] : s == 2 ? at[2] : at[3]) != dist || winner != conn) continue;
         c.bnDom[key] = bdom;
-        if (c.nfTab != nullptr) record_noflux(m, c, (int)c.recConn[r], key, nx);
+        if (c.nfTab != nullptr) record_noflux(m, c, (int)conn, key, nx);
         if (c.bounceW != nullptr && s >= 2) {
             // DiracD2Q5's advect skips the swap with the W / S neighbour when
             // this node has a boundary node there (DiracD2Q5.cpp:166-180)
@@ -1119,10 +1140,8 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
             c.wDom[node] = bdom + 1;
             c.rowNow[(uint32_t)node / (uint32_t)nx] = 1;
         }
-        bool last = true;
-        for (int s2 = s + 1; s2 < 4; ++s2)
-            if (c.bnDist[node * 4 + s2] != kEmpty) last = false;
-        if (last && bdom != dom[node]) {
+        const bool last = (s >= 1 || at[1] == kEmpty) && (s >= 2 || at[2] == kEmpty) && (s >= 3 || at[3] == kEmpty);
+        if (last && bdom != old) {
             const int k = atomicAdd(&st->nChanged, 1);
             if (k < c.changedCap) {
                 c.changedNode[k] = (uint32_t)node;
@@ -1395,19 +1414,19 @@ __global__ void __launch_bounds__(kReinitBlock) reinit_kernel(CrossDev c, uint32
                                                               const uint32_t* ctypeTab, int nx, int ny, size_t L,
                                                               Status* st) {
     pdl_wait();
-    if (st->halt) return;
-    const int cnt = st->nChanged;
-    if (cnt == 0) return;
+    const int lane = threadIdx.x & 31, warps = kReinitBlock / 32, warp = threadIdx.x >> 5;
+    const int k0 = blockIdx.x * warps + warp;
+    int halt = st->halt, cnt = st->nChanged, typesCopied = st->cellTypesCopied;
+    uint32_t iteration = st->iteration, node0 = c.changedNode[min(k0, c.changedCap - 1)];
+    read_ahead(halt, cnt, typesCopied, iteration, node0);
+    if (halt || cnt == 0) return;
     if (cnt > kReinitMax || cnt > c.changedCap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(st, ERR_CAPACITY, cnt, ST_REINIT);
         return;
     }
     const SpeciesConst* sp = species.s;
-    const unsigned iteration = st->iteration;
-    const int typesCopied = st->cellTypesCopied;
-    const int lane = threadIdx.x & 31, warps = kReinitBlock / 32, warp = threadIdx.x >> 5;
-    for (int k = blockIdx.x * warps + warp; k < cnt; k += gridDim.x * warps) {
-        const size_t n = c.changedNode[k];
+    for (int k = k0; k < cnt; k += gridDim.x * warps) {
+        const size_t n = k == k0 ? node0 : c.changedNode[k];
         const uint32_t newDom = c.changedDom[k];
         // read with the marks, before it is known that the node may go ahead
         const ReinitLoads<Real> in = reinit_load<Real>(n, dom, g, u, nS, c, nx, ny, L);
@@ -1708,24 +1727,27 @@ __global__ void area_regulator_kernel(MembraneDev m, double* area, double* targe
     pdl_wait();
     const int cell = blockIdx.x * blockDim.x + threadIdx.x;
     if (cell >= m.nCells) return;
+    int halt = st->halt;
+    unsigned long long sum = acc != nullptr ? acc[cell] : 0ull;
+    double A = acc != nullptr ? 0.0 : area[cell], tgt = target[cell];
+    uint32_t d = m.ringDom[cell];
+    read_ahead(halt, d, A, tgt, sum);
     if (acc != nullptr) {
-        area[cell] = (double)(long long)acc[cell] * (1.0 / kAreaFix) / 2.0;
+        A = (double)(long long)sum * (1.0 / kAreaFix) / 2.0;
+        area[cell] = A;
         acc[cell] = 0ull;
     }
-    if (st->halt) return;
-    const double A = area[cell];
+    if (halt) return;
     double r;
     if (ctypeTab == nullptr) {
-        if (isnan(target[cell])) target[cell] = factor * A;
-        const double tgt = target[cell];
+        if (isnan(tgt)) target[cell] = tgt = factor * A;
         r = strength * (tgt - A) / tgt;
     } else {
-        if (isnan(target[cell])) target[cell] = factor;
-        r = strength * (target[cell] - A);
+        if (isnan(tgt)) target[cell] = tgt = factor;
+        r = strength * (tgt - A);
     }
     if (r > maxsource) r = maxsource;
     else if (r < -maxsource) r = -maxsource;
-    const uint32_t d = m.ringDom[cell];
     if (d < (uint32_t)nDomains && d != 0) {
         if (ctypeTab != nullptr && ctypeTab[d] == 1) r = maxsource;
         massTab[d] = r;
@@ -1805,7 +1827,9 @@ template void launch_growth<float>(const float*, const uint32_t*, size_t, int, i
 // the order; no ring ranking is needed.  FP64 runs keep the ring-ordered sum.
 __global__ void areas_fixed_kernel(MembraneDev m, const int* cellOfDom, int nDomains, unsigned long long* acc) {
     pdl_wait();
-    area_terms_fixed(m, blockIdx.x * blockDim.x + threadIdx.x, m.topo->C, m.ca, m.cb, m.cdom, cellOfDom, nDomains, acc);
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool in = c < m.topo->C;
+    area_term_fixed(m, in, in ? m.ca[c] : 0, in ? m.cb[c] : 0, in ? m.cdom[c] : 0u, cellOfDom, nDomains, acc);
 }
 
 void launch_areas(const MembraneDev& m, double* area, Status* st, cudaStream_t s) {

@@ -100,10 +100,10 @@ __device__ __forceinline__ bool remesh_fits(const MembraneDev& m, int K, int M, 
 // block (the same test on the same positions as the count).
 __global__ void __launch_bounds__(kRemeshBlock) remesh_apply_kernel(MembraneDev m, TopoDev t, Status* st) {
     pdl_wait();
-    if (st->halt) return;
     Topo* T = m.topo;
-    const int K = T->K;
-    if (K == 0) return;
+    int halt = st->halt, K = T->K;
+    read_ahead(halt, K);
+    if (halt || K == 0) return;
     const int C = T->C, M = T->M;
     if (!remesh_fits(m, K, M, C)) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_REMESH);
@@ -171,12 +171,19 @@ __global__ void __launch_bounds__(256) remesh_commit_kernel(MembraneDev m, TopoD
                                                             unsigned long long* areaAcc) {
     pdl_wait();
     Topo* T = m.topo;
-    const int K = T->K;
-    const int stage = st->halt ? st->haltStage : 0;
+    const int cn = blockIdx.x * blockDim.x + threadIdx.x, cc = min(cn, m.Ccap - 1);
+    int K = T->K, halt = st->halt, haltStage = st->haltStage, C0 = T->C, a0 = 0, b0 = 0;
+    uint32_t d0 = 0;
+    if (areaAcc != nullptr) {
+        a0 = m.ca[cc];
+        b0 = m.cb[cc];
+        d0 = m.cdom[cc];
+    }
+    read_ahead(K, halt, haltStage, C0, a0, b0, d0);
+    const int stage = halt ? haltStage : 0;
     if (K == 0) {
         if (areaAcc != nullptr && stage == 0)
-            area_terms_fixed(m, blockIdx.x * blockDim.x + threadIdx.x, T->C, m.ca, m.cb, m.cdom, t.cellOfDom,
-                             t.nDomains, areaAcc);
+            area_term_fixed(m, cn < C0, a0, b0, d0, t.cellOfDom, t.nDomains, areaAcc);
         return;
     }
     if ((stage != 0 && stage < ST_REMESH) || !remesh_fits(m, K, T->M, T->C)) {
@@ -210,7 +217,10 @@ __global__ void __launch_bounds__(256) remesh_commit_kernel(MembraneDev m, TopoD
         else if (X + 2.0 > nx) raise_error(st, ERR_EDGE_E, i, ST_REMESH);
         else if (Y + 2.0 > ny) raise_error(st, ERR_EDGE_N, i, ST_REMESH);
     }
-    if (areaAcc != nullptr) area_terms_fixed(m, c, C + K, t.ca2, t.cb2, t.cdom2, t.cellOfDom, t.nDomains, areaAcc);
+    if (areaAcc != nullptr) {
+        const bool in = c < C + K;
+        area_term_fixed(m, in, in ? t.ca2[c] : 0, in ? t.cb2[c] : 0, in ? t.cdom2[c] : 0u, t.cellOfDom, t.nDomains, areaAcc);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();

@@ -103,6 +103,23 @@ inline void launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t s
     launch_ex(true, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
+// Values read ahead of a test: the compiler may not move their loads below it.
+// A stage kernel's course hangs on the halt word and on counts in device memory;
+// read one after another, each costs an L2 round trip (0.6 us) before the first
+// item is touched, which is most of a kernel of a small simulation.  So a kernel
+// reads the halt word, its counts and its first items together (from addresses
+// that are valid whatever the counts are) and tests afterwards.
+__device__ __forceinline__ void read_ahead(int& v) { asm volatile("" : "+r"(v)); }
+__device__ __forceinline__ void read_ahead(uint32_t& v) { asm volatile("" : "+r"(v)); }
+__device__ __forceinline__ void read_ahead(float& v) { asm volatile("" : "+f"(v)); }
+__device__ __forceinline__ void read_ahead(double& v) { asm volatile("" : "+d"(v)); }
+__device__ __forceinline__ void read_ahead(unsigned long long& v) { asm volatile("" : "+l"(v)); }
+template <typename A, typename... More>
+__device__ __forceinline__ void read_ahead(A& a, More&... more) {
+    read_ahead(a);
+    read_ahead(more...);
+}
+
 // Direction tables: libs/LbmLib/include/Direction.hpp:34-44 and
 // libs/LbmLib/src/Direction.cpp:27-61.
 enum Dir { T = 0, E = 1, N = 2, W = 3, S = 4, NE = 5, NW = 6, SW = 7, SE = 8 };

@@ -60,19 +60,16 @@ __device__ __forceinline__ void remesh_count_block(const MembraneDev& m, const T
     }
 }
 
-// Connection c's shoelace term x_a y_b - x_b y_a (a -> b along the ring), rounded
-// to fixed point (2^-24), into its cell's sum (areas_fixed_kernel's comment,
-// k_membrane.cu).  Every lane of the warp takes part; `ca, cb, cdom` is the
-// connection list, n its length.
+// A connection's (a -> b along the ring, of domain d) shoelace term x_a y_b -
+// x_b y_a, rounded to fixed point (2^-24), into its cell's sum
+// (areas_fixed_kernel's comment, k_membrane.cu).  Every lane of the warp takes
+// part; `in`: the lane has a connection.
 constexpr double kAreaFix = 16777216.0;  // 2^24: the fixed-point scale of the shoelace terms
-__device__ __forceinline__ void area_terms_fixed(const MembraneDev& m, int c, int n, const int* ca, const int* cb,
-                                                 const uint32_t* cdom, const int* cellOfDom, int nDomains,
-                                                 unsigned long long* acc) {
+__device__ __forceinline__ void area_term_fixed(const MembraneDev& m, bool in, int a, int b, uint32_t d,
+                                                const int* cellOfDom, int nDomains, unsigned long long* acc) {
     int cell = -1;
     long long v = 0;
-    if (c < n) {
-        const int a = ca[c], b = cb[c];
-        const uint32_t d = cdom[c];
+    if (in) {
         if (d < (uint32_t)nDomains) cell = cellOfDom[d];
         v = __double2ll_rn((m.x[a] * m.y[b] - m.x[b] * m.y[a]) * kAreaFix);
     }
