@@ -143,11 +143,20 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     const uint32_t dom = a.dom[n];
     // The force field of a differentiated run is zero outside the force tiles,
     // so it and G are read and written everywhere: no load waits on another.
-    const double fx = a.force[n], fy = a.force[L + n];
+    // (With moving nodes the launch before spread it: read after the wait.)
+    double fx = 0.0, fy = 0.0;
+    if (!MOT) {
+        fx = a.force[n];
+        fy = a.force[L + n];
+    }
     double rta = 0.0;
     if (a.massTab != nullptr && dom < (uint32_t)a.nDomains) rta = a.massTab[dom];
     pdl_wait();
     pdl_launch_dependents();
+    if (MOT) {
+        fx = a.force[n];
+        fy = a.force[L + n];
+    }
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         if (a.seed) {
@@ -425,14 +434,14 @@ void launch_adjoint_step64(const AdjointArgs& a, cudaStream_t s) {
 void launch_adjoint_step64_motion(const AdjointArgs& a, cudaStream_t s) {
     const dim3 grid((unsigned)((a.nx + kAdjBlock - 1) / kAdjBlock), (unsigned)a.ny);
     switch (a.S + (a.fp32 ? 4 : 0)) {
-        case 0: adjoint_step64<0, double, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        case 1: adjoint_step64<1, double, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        case 2: adjoint_step64<2, double, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        case 3: adjoint_step64<3, double, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        case 4: adjoint_step64<0, float, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        case 5: adjoint_step64<1, float, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        case 6: adjoint_step64<2, float, true><<<grid, kAdjBlock, 0, s>>>(a); break;
-        default: adjoint_step64<3, float, true><<<grid, kAdjBlock, 0, s>>>(a); break;
+        case 0: launch_pdl(adjoint_step64<0, double, true>, grid, kAdjBlock, 0, s, a); break;
+        case 1: launch_pdl(adjoint_step64<1, double, true>, grid, kAdjBlock, 0, s, a); break;
+        case 2: launch_pdl(adjoint_step64<2, double, true>, grid, kAdjBlock, 0, s, a); break;
+        case 3: launch_pdl(adjoint_step64<3, double, true>, grid, kAdjBlock, 0, s, a); break;
+        case 4: launch_pdl(adjoint_step64<0, float, true>, grid, kAdjBlock, 0, s, a); break;
+        case 5: launch_pdl(adjoint_step64<1, float, true>, grid, kAdjBlock, 0, s, a); break;
+        case 6: launch_pdl(adjoint_step64<2, float, true>, grid, kAdjBlock, 0, s, a); break;
+        default: launch_pdl(adjoint_step64<3, float, true>, grid, kAdjBlock, 0, s, a); break;
     }
 }
 

@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256, LBIB_COLLIDE_MIN_BLOCKS) stream_collide32
     constexpr bool MASSNODE = (MODE & 2) != 0;  // per-node mass source
     constexpr bool GUO = (MODE & 4) != 0;       // Guo force model
     constexpr bool BOUNCE = (MODE & 8) != 0;    // a DiracD2Q5 species (bounce-back at boundary links)
+    constexpr bool FORCE64 = (MODE & 16) != 0;  // the force field is FP64 (moving-node differentiated runs)
     pdl_wait();
     if (a.status->halt) return;
     const int nx = a.nx, ny = a.ny;
@@ -157,8 +158,8 @@ __global__ void __launch_bounds__(256, LBIB_COLLIDE_MIN_BLOCKS) stream_collide32
     else if (a.massTab != nullptr && dom < (uint32_t)a.nDomains) rta = (float)a.massTab[dom];
     float Fx = 0.0f, Fy = 0.0f;
     if (a.tileCount[(y / kTile) * a.tilesX + (x / kTile)] > 0) {
-        Fx = a.force[n];
-        Fy = a.force[L + n];
+        Fx = FORCE64 ? (float)a.force64[n] : a.force[n];
+        Fy = FORCE64 ? (float)a.force64[L + n] : a.force[L + n];
     }
     const float drho = ((hT + hE) + (hN + hW)) + ((hS + hNE) + (hNW + hSW)) + hSE;
     const float dr = drho + rta;          // rho - 1
@@ -565,7 +566,7 @@ void launch_stream_collide32(const LatticeArgs<float>& args, cudaStream_t s) {
     const dim3 grid((unsigned)((a.nx + 255) / 256), (unsigned)a.ny);
     if (a.nfTab != nullptr) launch_noflux<float>(a, s);
     const int mode = (a.coupled ? 1 : 0) | (a.massNode != nullptr ? 2 : 0) | (a.forceModel != FM_LUO ? 4 : 0) |
-                     (a.bounceW != nullptr ? 8 : 0);
+                     (a.bounceW != nullptr ? 8 : 0) | (a.force64 != nullptr ? 16 : 0);
     // LBIB_COLLIDE_X4=1 (read when the kernel is launched or captured): four
     // nodes per thread for the plain modes on rows of a multiple of 256 nodes.
     // Off by default: slower inside the step (below).
@@ -596,6 +597,7 @@ void launch_stream_collide32(const LatticeArgs<float>& args, cudaStream_t s) {
         LBIB_SC_CASE(6, 0) LBIB_SC_CASE(6, 1) LBIB_SC_CASE(6, 2) LBIB_SC_CASE(6, 3)
         LBIB_SC_CASE(5, 2) LBIB_SC_CASE(5, 3) LBIB_SC_CASE(7, 2) LBIB_SC_CASE(7, 3)
         LBIB_SC_CASE(8, 1) LBIB_SC_CASE(8, 2) LBIB_SC_CASE(8, 3)
+        LBIB_SC_CASE(16, 0) LBIB_SC_CASE(16, 1) LBIB_SC_CASE(16, 2) LBIB_SC_CASE(16, 3)
 #undef LBIB_SC_CASE
         default: break;
     }

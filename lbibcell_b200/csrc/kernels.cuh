@@ -322,7 +322,7 @@ struct AdjointArgs {
     double* uo;            // 2*L      the post-collision velocity of step t (output)
 };
 void launch_adjoint_step64(const AdjointArgs& a, cudaStream_t s);
-// The same step in its motion form (a.gu, a.uo; G overwritten), a plain launch.
+// The same step in its motion form (a.gu, a.uo; G overwritten).
 void launch_adjoint_step64_motion(const AdjointArgs& a, cudaStream_t s);
 // Converts n doubles to floats (the force field of an FP32-shifted run).
 void launch_to_float(const double* in, float* out, size_t n, cudaStream_t s);
@@ -341,22 +341,34 @@ void launch_force_adjoint(const MembraneDev& m, const double* G, int nx, int ny,
 // stencil of each node follows from its position at the step (the 4x4
 // lattice nodes within 2 lu), its weights are calculateDiscreteDeltaDirac's.
 // out[n] += dirac(x_n - X_i) * (ax_i, ay_i) over every node's stencil (FP64
-// atomics: the spread of the node forces, or of dL/dX onto dL/du).
-void launch_motion_spread(const double* X, const double* Y, const double* ax, const double* ay, int M, int nx,
-                          int ny, size_t L, double* out, Status* st, cudaStream_t s);
+// atomics: the spread of the node forces, or of dL/dX onto dL/du); out2, when
+// given, likewise with (bx_i, by_i).
+void launch_motion_spread(const double* X, const double* Y, const double* ax, const double* ay, const double* bx,
+                          const double* by, int M, int nx, int ny, size_t L, double* out, double* out2, Status* st,
+                          cudaStream_t s);
 // X1 = X0 + the velocity interpolated from u at X0 (GeometryNode::collectVelocity
-// then move, GeometryNode.cpp:216-226, 245-254, without the perturbation).
+// then move, GeometryNode.cpp:216-226, 245-254, without the perturbation);
+// u == nullptr: X1 is known.  out != nullptr: then the spread of (fx, fy) from X1
+// into out, with `used`, the field spread from X0, cleared.
 template <typename Real>
-void launch_motion_move(const double* X0, const double* Y0, double* X1, double* Y1, int M, const Real* u, int nx,
-                        int ny, size_t L, Status* st, cudaStream_t s);
+void launch_motion_next(const double* X0, const double* Y0, double* X1, double* Y1, int M, const Real* u,
+                        const double* fx, const double* fy, double* used, double* out, int nx, int ny, size_t L,
+                        Status* st, cudaStream_t s);
 // Reverse of one step's spread, interpolation and move for node i at its
 // step-start position X: with lambda = dL/dX_after,
 //   lambda += sum_n grad_X dirac * (lambda . uo(n) + F_i . G(n)),
 //   gF_i   += sum_n dirac * G(n),
 // G = dL/d(force field) of the step, uo its post-collision velocity.
+// next: the fields of the step before, spread from its positions (lambda into
+// out, the forces into out2), with those just used cleared; out == nullptr: none.
+struct MotionNext {
+    const double* X; const double* Y;
+    double* out; double* out2;
+    double* used; double* used2;
+};
 void launch_motion_adjoint(const double* X, const double* Y, const double* fx, const double* fy, double* lx,
-                           double* ly, const double* uo, const double* G, double* gfx, double* gfy, int M, int nx,
-                           int ny, size_t L, cudaStream_t s);
+                           double* ly, const double* uo, const double* G, double* gfx, double* gfy,
+                           const MotionNext& next, int M, int nx, int ny, size_t L, Status* st, cudaStream_t s);
 
 // The state in the host's layouts (k_readout.cu): the parts of a read-out, in
 // the order they are packed (8-byte elements first).

@@ -186,16 +186,23 @@ struct DiffCtx {
     double* lam = nullptr;      // 2 * M: dL/dX after the step being reversed
     double* seedX = nullptr;    // 2 * M: dL/dX after the final step
     bool haveSeedX = false;
-    double* gu = nullptr;       // 2 * L: dL/d(post-collision velocity) of one step
+    // the fields of a step and of the next one, used in turn, in the allocation
+    // of `force` (so that one memset clears them): force, force2 (the force
+    // field), gu, gu2 (dL/d(post-collision velocity)), 2 * L each
+    double* force2 = nullptr;
+    double* gu = nullptr;
+    double* gu2 = nullptr;
     double* uo = nullptr;       // 2 * L: the post-collision velocity of one step
     double* posAt(int t) const { return pos + (size_t)t * 2 * M; }
+    double* forceOf(int t) const { return (t & 1) && motion ? force2 : force; }  // the field of step t
+    double* guOf(int t) const { return t & 1 ? gu2 : gu; }
     char* state(int i) const { return i == 0 ? x0 : ck + (size_t)(i - 1) * stateBytes; }
     ~DiffCtx() {
         auto fr = [](void* p) { if (p) cudaFree(p); };
         fr(x0); fr(u0); fr(ck); fr(seg); fr(fin); fr(P[0]); fr(P[1]); fr(G); fr(force); fr(force32); fr(fxp);
         fr(fyp); fr(gfx); fr(gfy);
         fr(srcTab); fr(seed); fr(grad); fr(racc); fr(part); fr(st); fr(massTab); fr(macc); fr(seedF); fr(seg2);
-        fr(pos); fr(lam); fr(seedX); fr(gu); fr(uo);
+        fr(pos); fr(lam); fr(seedX); fr(uo);
         for (cudaEvent_t e : {evRec[0], evRec[1], evAdj[0], evAdj[1], evFork, evJoin[0], evJoin[1]})
             if (e) cudaEventDestroy(e);
         if (recStream) cudaStreamDestroy(recStream);
@@ -2419,7 +2426,8 @@ static void diff_forward_step_t(Handle& h, DiffCtx& d, const char* in, char* out
     LatticeArgs<Real> a = lattice_args<Real>(h, it, h.cur);
     a.fin = (const Real*)in; a.fout = (Real*)out;
     a.gin = (const Real*)in + 9 * h.L; a.gout = (Real*)out + 9 * h.L;
-    a.force = sizeof(Real) == 8 ? (const Real*)d.force : (const Real*)d.force32;
+    a.force = sizeof(Real) == 8 ? (const Real*)d.forceOf(t) : (const Real*)d.force32;
+    a.force64 = d.motion ? d.forceOf(t) : nullptr;  // (rounded by the FP32-shifted kernel where it reads it)
     a.srcTab = d.srcTab;
     a.massTab = d.massUsed ? d.massTab : nullptr;
     a.tauF = d.tauF;
@@ -2430,32 +2438,39 @@ static void diff_forward_step_t(Handle& h, DiffCtx& d, const char* in, char* out
     else launch_stream_collide32(*(const LatticeArgs<float>*)&a, stream);
 }
 
-// Step t of a run with moving membrane nodes: the node forces spread from
-// the positions after step t-1, the lattice step, then (move) the positions
-// after step t.  The reverse pass replays it without the move: the positions
-// of every step are stored.
-static void diff_motion_spread(Handle& h, DiffCtx& d, int t, cudaStream_t stream) {
+// A stretch of steps of a run with moving membrane nodes begins at step t: both
+// fields cleared, the node forces spread from the positions after step t-1
+// (and, going back, dL/dX onto dL/du).
+static void diff_motion_begin(Handle& h, DiffCtx& d, int t, cudaStream_t stream, bool back = false) {
     const double* X = d.posAt(t - 1);
-    CK(cudaMemsetAsync(d.force, 0, sizeof(double) * 2 * h.L, stream));
-    launch_motion_spread(X, X + d.M, d.fxp, d.fyp, d.M, h.nx, h.ny, h.L, d.force, d.st, stream);
-    if (d.rs == 4) launch_to_float(d.force, d.force32, 2 * h.L, stream);
+    CK(cudaMemsetAsync(d.force, 0, sizeof(double) * (back ? 8 : 4) * h.L, stream));
+    if (back) {
+        launch_motion_spread(X, X + d.M, d.lam, d.lam + d.M, d.fxp, d.fyp, d.M, h.nx, h.ny, h.L, d.guOf(t),
+                             d.forceOf(t), d.st, stream);
+    } else {
+        launch_motion_spread(X, X + d.M, d.fxp, d.fyp, nullptr, nullptr, d.M, h.nx, h.ny, h.L, d.forceOf(t), nullptr,
+                             d.st, stream);
+    }
 }
 
+// Forward step t.  With moving nodes: the lattice step in the field spread from
+// the positions after step t-1, then (move) the positions after step t, and,
+// unless step t is the stretch's last, the field of step t+1.  The reverse pass
+// replays it without the move: the positions of every step are stored.
 static void diff_forward_step(Handle& h, DiffCtx& d, const char* in, char* out, int t, cudaStream_t stream,
-                              bool move = false) {
-    if (d.motion) diff_motion_spread(h, d, t, stream);
+                              bool move = false, bool last = false) {
     if (d.rs == 8) diff_forward_step_t<double>(h, d, in, out, t, stream);
     else diff_forward_step_t<float>(h, d, in, out, t, stream);
-    if (d.motion && move) {
-        const double* X0 = d.posAt(t - 1);
-        double* X1 = d.posAt(t);
-        if (d.rs == 8)
-            launch_motion_move<double>(X0, X0 + d.M, X1, X1 + d.M, d.M, (const double*)h.u, h.nx, h.ny, h.L, d.st,
-                                       stream);
-        else
-            launch_motion_move<float>(X0, X0 + d.M, X1, X1 + d.M, d.M, (const float*)h.u, h.nx, h.ny, h.L, d.st,
-                                      stream);
-    }
+    if (!d.motion || (last && !move)) return;
+    const double* X0 = d.posAt(t - 1);
+    double* X1 = d.posAt(t);
+    double* next = last ? nullptr : d.forceOf(t + 1);
+    if (d.rs == 8)
+        launch_motion_next<double>(X0, X0 + d.M, X1, X1 + d.M, d.M, move ? (const double*)h.u : nullptr, d.fxp, d.fyp,
+                                   d.forceOf(t), next, h.nx, h.ny, h.L, d.st, stream);
+    else
+        launch_motion_next<float>(X0, X0 + d.M, X1, X1 + d.M, d.M, move ? (const float*)h.u : nullptr, d.fxp, d.fyp,
+                                  d.forceOf(t), next, h.nx, h.ny, h.L, d.st, stream);
 }
 
 static void diff_check_status(Handle& h, DiffCtx& d) {
@@ -2475,6 +2490,8 @@ static void diff_forward(Handle& h, DiffCtx& d) {
         if (d.pos != nullptr) CK(cudaMemsetAsync(d.force, 0, sizeof(double) * 2 * L, h.stream));
         launch_spread<double>(mp, h.tiles, d.force, h.nx, h.ny, L, d.st, d.it0, h.stream);
         if (d.rs == 4) launch_to_float(d.force, d.force32, 2 * L, h.stream);
+    } else {
+        diff_motion_begin(h, d, 1, h.stream);
     }
     // two scratch states for the steps between checkpoints (the segment
     // buffer, free during the forward pass; with K = 2 one is enough, with
@@ -2490,13 +2507,15 @@ static void diff_forward(Handle& h, DiffCtx& d) {
         else if (t == d.T) out = d.fin;
         else if (t > lastBase) out = d.seg + (size_t)(t - lastBase - 1) * d.stateBytes;
         else out = scratch[t & 1];
-        diff_forward_step(h, d, in, out, t, h.stream, true);
+        diff_forward_step(h, d, in, out, t, h.stream, true, t == d.T);
         in = out;
     }
+    if (d.motion && d.rs == 4) launch_to_float(d.forceOf(d.T), d.force32, 2 * L, h.stream);
     d.lastSegKept = true;
     // the final state and the force field become the handle's lattice, for
     // lbib_download_lattice
-    if (d.rs == 8) CK(cudaMemcpyAsync(h.force, d.force, sizeof(double) * 2 * L, cudaMemcpyDeviceToDevice, h.stream));
+    if (d.rs == 8)
+        CK(cudaMemcpyAsync(h.force, d.forceOf(d.T), sizeof(double) * 2 * L, cudaMemcpyDeviceToDevice, h.stream));
     else CK(cudaMemcpyAsync(h.force, d.force32, sizeof(float) * 2 * L, cudaMemcpyDeviceToDevice, h.stream));
     CK(cudaMemcpyAsync(h.f[h.cur], in, 9 * L * d.rs, cudaMemcpyDeviceToDevice, h.stream));
     if (h.S)
@@ -2553,11 +2572,13 @@ static void diff_backward(Handle& h, DiffCtx& d) {
     };
     auto segLen = [&](int s) { return std::min(d.K, d.T - s * d.K); };
     auto recompute = [&](int s, cudaStream_t stream) {
+        if (d.motion && segLen(s) > 1) diff_motion_begin(h, d, s * d.K + 1, stream);
         for (int j = 1; j < segLen(s); ++j)
-            diff_forward_step(h, d, segState(s, j - 1), segState(s, j), s * d.K + j, stream);
+            diff_forward_step(h, d, segState(s, j - 1), segState(s, j), s * d.K + j, stream, false, j == segLen(s) - 1);
     };
     auto reverse = [&](int s, cudaStream_t stream) {
         const int base = s * d.K;
+        if (d.motion) diff_motion_begin(h, d, base + segLen(s), stream, true);
         for (int t = base + segLen(s); t > base; --t) {
             const char* prev = segState(s, t - 1 - base);
             a.fprev = prev;
@@ -2583,16 +2604,17 @@ static void diff_backward(Handle& h, DiffCtx& d) {
             // spread from the step-start positions, and the step's G and
             // velocity then carry dL/dX back to those positions
             const double* X = d.posAt(t - 1);
-            CK(cudaMemsetAsync(d.gu, 0, sizeof(double) * 2 * L, stream));
-            launch_motion_spread(X, X + d.M, d.lam, d.lam + d.M, d.M, h.nx, h.ny, L, d.gu, d.st, stream);
-            CK(cudaMemsetAsync(d.force, 0, sizeof(double) * 2 * L, stream));
-            launch_motion_spread(X, X + d.M, d.fxp, d.fyp, d.M, h.nx, h.ny, L, d.force, d.st, stream);
-            a.gu = d.gu;
+            a.force = d.forceOf(t);
+            a.gu = d.guOf(t);
             a.uo = d.uo;
-            a.chained = 0;
             launch_adjoint_step64_motion(a, stream);
-            launch_motion_adjoint(X, X + d.M, d.fxp, d.fyp, d.lam, d.lam + d.M, d.uo, d.G, d.gfx, d.gfy, d.M, h.nx,
-                                  h.ny, L, stream);
+            MotionNext next{};
+            if (t - 1 > base) {
+                const double* X2 = d.posAt(t - 2);
+                next = MotionNext{X2, X2 + d.M, d.guOf(t - 1), d.forceOf(t - 1), d.guOf(t), d.forceOf(t)};
+            }
+            launch_motion_adjoint(X, X + d.M, d.fxp, d.fyp, d.lam, d.lam + d.M, d.uo, d.G, d.gfx, d.gfy, next, d.M, h.nx,
+                                  h.ny, L, d.st, stream);
         }
     };
     const bool keptLast = d.lastSegKept;
@@ -2649,7 +2671,7 @@ static void diff_set_motion(Handle& h, DiffCtx& d, bool on) {
     }
     const size_t L = h.L;
     const int M = h.m.M;
-    const size_t bytes = sizeof(double) * ((size_t)(d.T + 1) * 2 * M + 4 * (size_t)M + 4 * L);
+    const size_t bytes = sizeof(double) * ((size_t)(d.T + 1) * 2 * M + 4 * (size_t)M + 8 * L);
     size_t freeB = 0, totalB = 0;
     CK(cudaMemGetInfo(&freeB, &totalB));
     if (bytes + (256u << 20) > freeB)
@@ -2659,8 +2681,15 @@ static void diff_set_motion(Handle& h, DiffCtx& d, bool on) {
     d.pos = dalloc<double>((size_t)(d.T + 1) * 2 * M + 1);
     d.lam = dalloc<double>(2 * (size_t)M + 1);
     d.seedX = dalloc<double>(2 * (size_t)M + 1);
-    d.gu = dalloc<double>(2 * L);
     d.uo = dalloc<double>(2 * L);
+    double* fields = dalloc<double>(8 * L);
+    CK(cudaMemcpyAsync(fields, d.force, sizeof(double) * 2 * L, cudaMemcpyDeviceToDevice, h.stream));
+    CK(cudaStreamSynchronize(h.stream));
+    cudaFree(d.force);
+    d.force = fields;
+    d.force2 = fields + 2 * L;
+    d.gu = fields + 4 * L;
+    d.gu2 = fields + 6 * L;
     if (M) {
         CK(cudaMemcpyAsync(d.pos, h.m.x, sizeof(double) * M, cudaMemcpyDeviceToDevice, h.stream));
         CK(cudaMemcpyAsync(d.pos + M, h.m.y, sizeof(double) * M, cudaMemcpyDeviceToDevice, h.stream));

@@ -285,6 +285,7 @@ struct LatticeArgs {
     Real* gout;           // S*5*L
     Real* u;              // 2*L
     const Real* force;    // 2*L (valid where tileCount > 0)
+    const double* force64; // FP32-shifted kernel, moving-node differentiated runs: the field in FP64 (else nullptr)
     const int* tileCount; // per 16x16 tile: membrane stencils overlapping it (TileDev::active)
     int tilesX;
     const uint32_t* dom;  // L
