@@ -26,15 +26,24 @@ namespace lbib {
 // boundary node (DiracD2Q5::advect, DiracD2Q5.cpp:166-180): the swap with the
 // W (S) neighbour is skipped when the node has a W (S) boundary node, so the
 // node's own opposite population stays.
+// Blocks of 128 nodes, and the register budget of 6 of them per SM (80; 7, 72
+// registers, with three species): 24 to 28 warps per SM cover more of the planes'
+// latency than the compiler's own 82 registers in blocks of 256, and the last
+// wave is shorter.  Per lattice step, 256 threads against this: 701x499, three
+// species 32.9 -> 30.1 us, 1500x1100 130.4 -> 121.1, 1024^2, two species 65.1 ->
+// 63.7, 512^2, one species 11.0 -> 10.2.  (8 blocks, 64 registers and 90 B of
+// spills: 1024^2, one species 53.0 -> 50.8, but 512^2 10.2 -> 11.0.)
+constexpr int kCollide64Block = 128;
+constexpr int collide64_min_blocks(int species) { return species >= 3 ? 7 : 6; }
 template <int NS, int MODE>
-__global__ void __launch_bounds__(256) stream_collide64(LatticeArgs<double> a) {
+__global__ void __launch_bounds__(kCollide64Block, collide64_min_blocks(NS)) stream_collide64(LatticeArgs<double> a) {
     constexpr bool COUPLED = (MODE & 1) != 0;   // coupled species reactions
     constexpr bool MASSNODE = (MODE & 2) != 0;  // per-node mass source
     constexpr bool GUO = (MODE & 4) != 0;       // Guo force model
     constexpr bool BOUNCE = (MODE & 8) != 0;    // a DiracD2Q5 species (bounce-back at boundary links)
     pdl_wait();
     if (a.status->halt) return;
-    // grid (nx/256, ny): one lattice node per thread
+    // grid (nx / block, ny): one lattice node per thread
     const int nx = a.nx, ny = a.ny;
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= nx) return;
@@ -324,13 +333,13 @@ template void launch_noflux<double>(const LatticeArgs<double>&, cudaStream_t);
 template void launch_noflux<float>(const LatticeArgs<float>&, cudaStream_t);
 
 void launch_stream_collide64(const LatticeArgs<double>& a, cudaStream_t s) {
-    const dim3 grid((unsigned)((a.nx + 255) / 256), (unsigned)a.ny);
+    const dim3 grid((unsigned)((a.nx + kCollide64Block - 1) / kCollide64Block), (unsigned)a.ny);
     if (a.nfTab != nullptr) launch_noflux<double>(a, s);
     const int mode = (a.coupled ? 1 : 0) | (a.massNode != nullptr ? 2 : 0) | (a.forceModel != FM_LUO ? 4 : 0) |
                      (a.bounceW != nullptr ? 8 : 0);
     switch (mode * 4 + (a.S < 3 ? a.S : 3)) {
 #define LBIB_SC_CASE(M, N) \
-    case M * 4 + N: launch_pdl(stream_collide64<N, M>, grid, 256, 0, s, a); break;
+    case M * 4 + N: launch_pdl(stream_collide64<N, M>, grid, kCollide64Block, 0, s, a); break;
         LBIB_SC_CASE(0, 0) LBIB_SC_CASE(0, 1) LBIB_SC_CASE(0, 2) LBIB_SC_CASE(0, 3)
         LBIB_SC_CASE(2, 0) LBIB_SC_CASE(2, 1) LBIB_SC_CASE(2, 2) LBIB_SC_CASE(2, 3)
         // coupled reactions need a partner species: two or three species

@@ -2786,7 +2786,7 @@ int lbib_lattice_step(lbib_handle* hh, int n, int outlet) {
     lbib::reset_status(h, h.iteration, h.cellTypesCopied);
     h.lastCollideMs = 0;
     h.lastCollideLaunches = 0;
-    h.launches = (long long)n * 2;
+    h.launches = n;
     while ((int)h.kEvents.size() < 2 * n) {
         cudaEvent_t e;
         CK(cudaEventCreate(&e));
@@ -2807,7 +2807,11 @@ int lbib_lattice_step(lbib_handle* hh, int n, int outlet) {
         }
         if (h.profiling) CK(cudaEventRecord(h.kEvents[2 * i + 1], h.stream));
         h.cur = 1 - p;
-        launch_pdl(lbib::iteration_inc_kernel, 1, 1, 0, h.stream, h.st);
+        // (read by the SIGNAL reaction alone, and set anew before the next run)
+        if (lbib::diff_needs_iteration(h)) {
+            launch_pdl(lbib::iteration_inc_kernel, 1, 1, 0, h.stream, h.st);
+            h.launches++;
+        }
         h.iteration++;
     }
     CK(cudaEventRecord(h.evB, h.stream));
