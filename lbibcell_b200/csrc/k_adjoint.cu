@@ -33,16 +33,32 @@
 // grad[1 + S + S*nDomains + domain].  A seed for the fluid (seedF, the
 // gradient of the loss with respect to the final stored distributions) joins
 // the species' seed at the final step.
+#include <type_traits>
+
 #include "kernels.cuh"
 
 namespace lbib {
 
 namespace {
 
-__device__ __constant__ int kCX[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
-__device__ __constant__ int kCY[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
+// Directions and weights as constants of the unrolled loops (T,E,N,W,S,NE,NW,SW,SE).
+__host__ __device__ constexpr int cX(int q) {
+    return q == 1 || q == 5 || q == 8 ? 1 : (q == 3 || q == 6 || q == 7 ? -1 : 0);
+}
+__host__ __device__ constexpr int cY(int q) {
+    return q == 2 || q == 5 || q == 6 ? 1 : (q == 4 || q == 7 || q == 8 ? -1 : 0);
+}
+__host__ __device__ constexpr double weight9(int q) { return q == 0 ? 4.0 / 9.0 : (q < 5 ? 1.0 / 9.0 : 1.0 / 36.0); }
 
-__device__ __forceinline__ double weight9(int q) { return q == 0 ? 4.0 / 9.0 : (q < 5 ? 1.0 / 9.0 : 1.0 / 36.0); }
+// acc + c v for a direction component c of -1, 0 or 1 (v rounded already).
+__device__ __forceinline__ double plus(int c, double v, double acc) { return c > 0 ? acc + v : (c < 0 ? acc - v : acc); }
+// c_x x + c_y y of direction q
+__device__ __forceinline__ double along(int q, double x, double y) {
+    const double X = cX(q) < 0 ? -x : x;
+    if (cY(q) == 0) return cX(q) == 0 ? 0.0 : X;
+    const double Y = cY(q) < 0 ? -y : y;
+    return cX(q) == 0 ? Y : X + Y;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -74,19 +90,24 @@ __device__ __forceinline__ void warp_keyed_add(double* grad, int key, double v) 
 
 // NS = number of species (compile-time, so that the species' inputs are
 // loaded together with the fluid state).  Grid (ceil(nx / kAdjBlock), ny).
-// The fluid's adjoint inputs are loaded after the species' reverse pass and
-// the gradient accumulators where they are updated, so that a node's values
-// are not all live at once (one species: 24 B of spills at 128 registers).
-// LBIB_ADJOINT_MIN_BLOCKS (blocks per SM the register budget is sized for)
-// trades occupancy against spills.
-#ifndef LBIB_ADJOINT_MIN_BLOCKS
-#define LBIB_ADJOINT_MIN_BLOCKS 4
-#endif
-// Threads per block (nodes of one row segment); with the blocks per SM above
-// it sets the register budget: 128 x 4 -> 128 registers.  Measured on
-// adjoint_512 (T = 2000, K = 100): 256 x 2 backward 75.6 ms, 128 x 4 73.1 ms,
-// 64 x 8 73.2 ms; 256 x 1 (no spills, 8 warps per SM) and 128 x 5 (96
-// registers, 300 B of spills) are slower.
+//
+// The directions are constants of the unrolled loops: read from constant memory,
+// each c_q v was a conversion and a multiply-add, zeros included, and a node took
+// 1,270 instructions.  Everything a node reads is under way before the first value
+// is used: the adjoint planes wait as the FP32 values they are, the accumulators
+// ride along, and the relaxation-time sums leave by reductions that nothing waits
+// for.  The step of 512^2 nodes with one species: 23 -> 14.7 us.  The arithmetic is
+// what it was, to the last bit: products that a direction's factor kept from being
+// contracted into an addition are kept apart by __dmul_rn (the adjoint planes are
+// rounded to FP32 every step, and a last bit that differs grows over the steps into
+// a difference of the size of those roundings).
+//
+// Blocks per SM the register budget is sized for: five (96 registers, 90 B of
+// spills) with up to one species, four (128) with more.  512^2 reverse pass per
+// step with its recomputation, one species: 3 blocks 25.8 us, 4 23.8, 5 23.7, 6 31.0;
+// two species: 35.0, 35.4, 38.7, 45.3; 1024^2, one species: 113.7, 102.6, 98.2, 115.2.
+constexpr int adjoint_min_blocks(int species) { return species <= 1 ? 5 : 4; }
+// Threads per block (nodes of one row segment).
 #ifndef LBIB_ADJOINT_BLOCK
 #define LBIB_ADJOINT_BLOCK 128
 #endif
@@ -98,8 +119,11 @@ constexpr int kAdjBlock = LBIB_ADJOINT_BLOCK;
 // velocity output has its own adjoint input a.gu (the nodes interpolate it),
 // the post-collision velocity is written to a.uo, and G holds this step's
 // dL/dF alone (the force field changes every step).
-template <int NS, typename Real, bool MOT = false>
-__global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_step64(AdjointArgs a) {
+// SEED: the final step, whose adjoint inputs are the caller's (FP64).
+template <int NS, typename Real, bool MOT, bool SEED>
+__global__ void __launch_bounds__(kAdjBlock, adjoint_min_blocks(NS)) adjoint_step64(AdjointArgs a) {
+    typedef typename std::conditional<SEED, double, float>::type Adj;
+    constexpr int NSA = NS > 0 ? NS : 1;
     const int nx = a.nx, ny = a.ny;
     const size_t L = a.L;
     const int xr = blockIdx.x * blockDim.x + threadIdx.x;
@@ -112,12 +136,12 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     // forward pull sources x - c_q and adjoint gather sources x + c_q (offsets
     // within a plane), formed where they are used
     auto pull = [&](int q) -> unsigned {
-        const unsigned row = kCY[q] > 0 ? rM : (kCY[q] < 0 ? rP : rC);
-        return row + (kCX[q] > 0 ? xm : (kCX[q] < 0 ? xp : x));
+        const unsigned row = cY(q) > 0 ? rM : (cY(q) < 0 ? rP : rC);
+        return row + (cX(q) > 0 ? xm : (cX(q) < 0 ? xp : x));
     };
     auto push = [&](int q) -> unsigned {
-        const unsigned row = kCY[q] > 0 ? rP : (kCY[q] < 0 ? rM : rC);
-        return row + (kCX[q] > 0 ? xp : (kCX[q] < 0 ? xm : x));
+        const unsigned row = cY(q) > 0 ? rP : (cY(q) < 0 ? rM : rC);
+        return row + (cX(q) > 0 ? xp : (cX(q) < 0 ? xm : x));
     };
 
     // ---- the inputs of the forward recomputation and of the species ------
@@ -128,17 +152,14 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     // wait): they are loaded before the wait, during the previous step's last
     // wave.  The adjoint planes and the accumulators are read after it.
     const Real* __restrict__ fprev = (const Real*)a.fprev;
-    double f[9], lf[9];
+    Real fr[9], gr[NSA][5];
 #pragma unroll
-    for (int q = 0; q < 9; ++q)
-        f[q] = sizeof(Real) == 8 ? (double)fprev[(size_t)q * L + pull(q)]
-                                 : (double)fprev[(size_t)q * L + pull(q)] + weight9(q);
-    double gA[NS > 0 ? NS : 1][5], muA[NS > 0 ? NS : 1][5];
+    for (int q = 0; q < 9; ++q) fr[q] = fprev[(size_t)q * L + pull(q)];
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
         const Real* gp = (const Real*)a.gprev + (size_t)k * 5 * L;
 #pragma unroll
-        for (int q = 0; q < 5; ++q) gA[k][q] = gp[(size_t)q * L + pull(q)];
+        for (int q = 0; q < 5; ++q) gr[k][q] = gp[(size_t)q * L + pull(q)];
     }
     const uint32_t dom = a.dom[n];
     // The force field of a differentiated run is zero outside the force tiles,
@@ -157,23 +178,35 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
         fx = a.force[n];
         fy = a.force[L + n];
     }
+    Adj lr[9], mr[NSA][5];
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-        if (a.seed) {
-            const double sd = a.seed[(size_t)k * L + n];
 #pragma unroll
-            for (int q = 0; q < 5; ++q) muA[k][q] = sd;
-        } else {
-            const float* pg = a.pg + (size_t)k * 5 * L;
-#pragma unroll
-            for (int q = 0; q < 5; ++q) muA[k][q] = (double)pg[(size_t)q * L + push(q)];
+        for (int q = 0; q < 5; ++q) {
+            if constexpr (SEED) mr[k][q] = a.seed[(size_t)k * L + n];
+            else mr[k][q] = a.pg[((size_t)k * 5 + q) * L + push(q)];
         }
     }
-    double gTauK[NS > 0 ? NS : 1];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) {
+        if constexpr (SEED) lr[q] = a.seedF ? a.seedF[(size_t)q * L + n] : 0.0;
+        else lr[q] = a.pf[(size_t)q * L + push(q)];
+    }
+    double G0 = 0.0, G1 = 0.0, racc[NSA] = {};
+    if (!MOT) {
+        G0 = a.G[n];
+        G1 = a.G[L + n];
+    }
+#pragma unroll
+    for (int k = 0; k < NS; ++k)
+        if (a.sp[k].kind == RX_LINEAR) racc[k] = a.racc[(size_t)k * L + n];
     const bool hasMass = a.macc != nullptr && a.massTab != nullptr && dom < (uint32_t)a.nDomains && isfinite(rta);
     if (!isfinite(rta)) rta = 0.0;
 
     // ---- forward recomputation of the fluid collision --------------------
+    double f[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) f[q] = sizeof(Real) == 8 ? (double)fr[q] : (double)fr[q] + weight9(q);
     const double tauI = a.tauIF;
     double rhoF = 0.0;
 #pragma unroll
@@ -182,26 +215,27 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     double jx = 0.0, jy = 0.0;
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
-        jx += kCX[q] * f[q];
-        jy += kCY[q] * f[q];
+        jx = plus(cX(q), f[q], jx);
+        jy = plus(cY(q), f[q], jy);
     }
     const double rhoI = 1.0 / rho;
-    const double ux = jx * rhoI, uy = jy * rhoI;
+    const double ux = __dmul_rn(jx, rhoI), uy = __dmul_rn(jy, rhoI);
     const double lastTerm = 1.5 * (ux * ux + uy * uy);
     // equilibrium and post-collision value of direction q
     auto feqw = [&](int q) {
-        const double cu = kCX[q] * ux + kCY[q] * uy;
+        const double cu = along(q, ux, uy);
         return weight9(q) * rho * (1.0 + 3.0 * cu + 4.5 * cu * cu - lastTerm);
     };
     auto fs = [&](int q) {
-        return f[q] - f[q] * tauI + feqw(q) * tauI + 3.0 * weight9(q) * rhoF * (kCX[q] * fx + kCY[q] * fy);
+        const double v = f[q] - f[q] * tauI + feqw(q) * tauI;
+        return q == 0 ? v : v + 3.0 * weight9(q) * rhoF * along(q, fx, fy);
     };
     double jox = 0.0, joy = 0.0;
 #pragma unroll
     for (int q = 0; q < 9; ++q) {
         const double v = fs(q);
-        jox += kCX[q] * v;
-        joy += kCY[q] * v;
+        jox = plus(cX(q), v, jox);
+        joy = plus(cY(q), v, joy);
     }
     const double uox = jox * rhoI, uoy = joy * rhoI;  // FluidSolver::velocity_ after collide
     // box outlet: node-local rescale(s) by 1/sum(f) on x = 0 and y = 0 (corner twice)
@@ -223,12 +257,17 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     // ---- species, backwards (their velocity and outlet terms feed the fluid)
     double D1 = 0.0, D2 = 0.0;      // dL/ds1, dL/ds2 from the species
     double muox = 0.0, muoy = 0.0;  // dL/d(post-collision velocity)
+    double gTauK[NSA];
 #pragma unroll
     for (int k = 0; k < NS; ++k) {
-        double* g = gA[k];
-        double* mu = muA[k];
-        const SpeciesConst sp = a.sp[k];
+        const SpeciesConst& sp = a.sp[k];
         const double tauIk = a.tauI[k];
+        double g[5], mu[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            g[q] = (double)gr[k][q];
+            mu[q] = (double)mr[k][q];
+        }
         const double C = g[0] + g[1] + g[2] + g[3] + g[4];
         const double C3 = C * (1.0 / 3.0), C6 = C * (1.0 / 6.0);
         double temp[5];
@@ -287,16 +326,13 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
             for (int q = 0; q < 5; ++q) qg[(size_t)q * L + n] = (float)((1.0 - tauIk) * mu[q] + mC);
         }
         gTauK[k] = valid ? gTau : 0.0;
-        if (valid && sp.kind == RX_LINEAR) a.racc[(size_t)k * L + n] += mR;
+        if (valid && sp.kind == RX_LINEAR) a.racc[(size_t)k * L + n] = racc[k] + mR;
     }
 
-    // ---- the fluid's adjoint inputs, loaded once the species are done (the
-    // node's values are not all held at once: no register spills) ----------
-#pragma unroll
-    for (int q = 0; q < 9; ++q)
-        lf[q] = a.seed ? (a.seedF ? a.seedF[(size_t)q * L + n] : 0.0) : (double)a.pf[(size_t)q * L + push(q)];
-
     // ---- fluid: outlet, velocity output and collide, backwards -----------
+    double lf[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) lf[q] = (double)lr[q];
     if (passes == 2) {
         double d = D2;
 #pragma unroll
@@ -321,9 +357,9 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
         }
     }
     double mrho = -(uox * muox + uoy * muoy) * rhoI;
-    const double mjox = muox * rhoI, mjoy = muoy * rhoI;
+    const double mjox = __dmul_rn(muox, rhoI), mjoy = __dmul_rn(muoy, rhoI);
 #pragma unroll
-    for (int q = 0; q < 9; ++q) lf[q] += kCX[q] * mjox + kCY[q] * mjoy;
+    for (int q = 1; q < 9; ++q) lf[q] += along(q, mjox, mjoy);
 
     double gTauF = 0.0, mrhoF = 0.0, mfx = 0.0, mfy = 0.0, mux = 0.0, muy = 0.0, mlast = 0.0;
 #pragma unroll
@@ -331,19 +367,24 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
         const double w = weight9(q);
         gTauF += lf[q] * (feqw(q) - f[q]);
         const double mfeq = lf[q] * tauI;
-        mrhoF += lf[q] * 3.0 * w * (kCX[q] * fx + kCY[q] * fy);
-        mfx += lf[q] * 3.0 * w * rhoF * kCX[q];
-        mfy += lf[q] * 3.0 * w * rhoF * kCY[q];
-        const double cu = kCX[q] * ux + kCY[q] * uy;
+        const double cu = along(q, ux, uy);
+        if (q > 0) {
+            mrhoF += lf[q] * 3.0 * w * along(q, fx, fy);
+            const double mf = __dmul_rn(lf[q] * 3.0 * w, rhoF);
+            mfx = plus(cX(q), mf, mfx);
+            mfy = plus(cY(q), mf, mfy);
+        }
         mrho += mfeq * w * (1.0 + 3.0 * cu + 4.5 * cu * cu - lastTerm);
-        const double mcu = mfeq * w * rho * (3.0 + 9.0 * cu);
-        mux += mcu * kCX[q];
-        muy += mcu * kCY[q];
+        if (q > 0) {
+            const double mcu = __dmul_rn(mfeq * w * rho, 3.0 + 9.0 * cu);
+            mux = plus(cX(q), mcu, mux);
+            muy = plus(cY(q), mcu, muy);
+        }
         mlast -= mfeq * w * rho;
     }
     mux += mlast * 3.0 * ux;
     muy += mlast * 3.0 * uy;
-    const double mjx = mux * rhoI, mjy = muy * rhoI;
+    const double mjx = __dmul_rn(mux, rhoI), mjy = __dmul_rn(muy, rhoI);
     mrho -= (ux * mux + uy * muy) * rhoI;
     mrhoF += mrho;
     // rho = sum f + rhoToAdd: dL/d rhoToAdd = dL/d rho
@@ -351,14 +392,9 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     if (valid) {
 #pragma unroll
         for (int q = 0; q < 9; ++q)
-            a.qf[(size_t)q * L + n] = (float)((1.0 - tauI) * lf[q] + mrhoF + kCX[q] * mjx + kCY[q] * mjy);
-        if (MOT) {
-            a.G[n] = mfx;
-            a.G[L + n] = mfy;
-        } else {
-            a.G[n] += mfx;
-            a.G[L + n] += mfy;
-        }
+            a.qf[(size_t)q * L + n] = (float)plus(cY(q), mjy, plus(cX(q), mjx, (1.0 - tauI) * lf[q] + mrhoF));
+        a.G[n] = G0 + mfx;
+        a.G[L + n] = G1 + mfy;
     }
     // relaxation-time gradients: block sums into this block's own slots (the
     // same slots every step), reduced over blocks once at the end of the pass
@@ -374,9 +410,10 @@ __global__ void __launch_bounds__(kAdjBlock, LBIB_ADJOINT_MIN_BLOCKS) adjoint_st
     __syncthreads();
     if (threadIdx.x <= NS) {
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w][threadIdx.x];
-        double* slot = a.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (1 + NS) + threadIdx.x;
-        *slot += t;
+#pragma unroll
+        for (int w = 0; w < kAdjBlock / 32; ++w) t += red[w][threadIdx.x];
+        // (no other block adds here: a reduction only so as not to wait for the old sum)
+        atomicAdd(a.part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (1 + NS) + threadIdx.x, t);
     }
 }
 
@@ -417,33 +454,27 @@ __global__ void set_iteration_kernel(Status* st, unsigned it) {
 
 int adjoint_blocks(int nx, int ny) { return ((nx + kAdjBlock - 1) / kAdjBlock) * ny; }
 
-void launch_adjoint_step64(const AdjointArgs& a, cudaStream_t s) {
+template <bool MOT>
+static void launch_step(const AdjointArgs& a, bool programmatic, cudaStream_t s) {
     const dim3 grid((unsigned)((a.nx + kAdjBlock - 1) / kAdjBlock), (unsigned)a.ny);
-    switch (a.S + (a.fp32 ? 4 : 0)) {
-        case 0: launch_ex(a.chained != 0, adjoint_step64<0, double>, grid, kAdjBlock, 0, s, a); break;
-        case 1: launch_ex(a.chained != 0, adjoint_step64<1, double>, grid, kAdjBlock, 0, s, a); break;
-        case 2: launch_ex(a.chained != 0, adjoint_step64<2, double>, grid, kAdjBlock, 0, s, a); break;
-        case 3: launch_ex(a.chained != 0, adjoint_step64<3, double>, grid, kAdjBlock, 0, s, a); break;
-        case 4: launch_ex(a.chained != 0, adjoint_step64<0, float>, grid, kAdjBlock, 0, s, a); break;
-        case 5: launch_ex(a.chained != 0, adjoint_step64<1, float>, grid, kAdjBlock, 0, s, a); break;
-        case 6: launch_ex(a.chained != 0, adjoint_step64<2, float>, grid, kAdjBlock, 0, s, a); break;
-        default: launch_ex(a.chained != 0, adjoint_step64<3, float>, grid, kAdjBlock, 0, s, a); break;
+    switch ((a.S < 3 ? a.S : 3) + (a.fp32 ? 4 : 0) + (a.seed != nullptr ? 8 : 0)) {
+#define LBIB_ADJ_CASE(I, N, R, SD) \
+    case I: launch_ex(programmatic, adjoint_step64<N, R, MOT, SD>, grid, kAdjBlock, 0, s, a); break;
+        LBIB_ADJ_CASE(0, 0, double, false) LBIB_ADJ_CASE(1, 1, double, false)
+        LBIB_ADJ_CASE(2, 2, double, false) LBIB_ADJ_CASE(3, 3, double, false)
+        LBIB_ADJ_CASE(4, 0, float, false) LBIB_ADJ_CASE(5, 1, float, false)
+        LBIB_ADJ_CASE(6, 2, float, false) LBIB_ADJ_CASE(7, 3, float, false)
+        LBIB_ADJ_CASE(8, 0, double, true) LBIB_ADJ_CASE(9, 1, double, true)
+        LBIB_ADJ_CASE(10, 2, double, true) LBIB_ADJ_CASE(11, 3, double, true)
+        LBIB_ADJ_CASE(12, 0, float, true) LBIB_ADJ_CASE(13, 1, float, true)
+        LBIB_ADJ_CASE(14, 2, float, true) LBIB_ADJ_CASE(15, 3, float, true)
+#undef LBIB_ADJ_CASE
     }
 }
 
-void launch_adjoint_step64_motion(const AdjointArgs& a, cudaStream_t s) {
-    const dim3 grid((unsigned)((a.nx + kAdjBlock - 1) / kAdjBlock), (unsigned)a.ny);
-    switch (a.S + (a.fp32 ? 4 : 0)) {
-        case 0: launch_pdl(adjoint_step64<0, double, true>, grid, kAdjBlock, 0, s, a); break;
-        case 1: launch_pdl(adjoint_step64<1, double, true>, grid, kAdjBlock, 0, s, a); break;
-        case 2: launch_pdl(adjoint_step64<2, double, true>, grid, kAdjBlock, 0, s, a); break;
-        case 3: launch_pdl(adjoint_step64<3, double, true>, grid, kAdjBlock, 0, s, a); break;
-        case 4: launch_pdl(adjoint_step64<0, float, true>, grid, kAdjBlock, 0, s, a); break;
-        case 5: launch_pdl(adjoint_step64<1, float, true>, grid, kAdjBlock, 0, s, a); break;
-        case 6: launch_pdl(adjoint_step64<2, float, true>, grid, kAdjBlock, 0, s, a); break;
-        default: launch_pdl(adjoint_step64<3, float, true>, grid, kAdjBlock, 0, s, a); break;
-    }
-}
+void launch_adjoint_step64(const AdjointArgs& a, cudaStream_t s) { launch_step<false>(a, a.chained != 0, s); }
+
+void launch_adjoint_step64_motion(const AdjointArgs& a, cudaStream_t s) { launch_step<true>(a, true, s); }
 
 __global__ void to_float_kernel(const double* in, float* out, size_t n) {
     pdl_wait();
