@@ -247,7 +247,7 @@ struct ReadLane {
 // kept, freed with the last handle that used them.  A call takes lanes out and
 // puts them back; calls from several threads on several handles share what
 // there is, and one that finds none makes one for itself.
-constexpr int kReadLanes = 8;
+constexpr int kReadLanes = 12;
 class LanePool {
 public:
     void join() {
@@ -420,13 +420,14 @@ struct Handle {
 
     long long hostEvents = 0;
     long long launches = 0;
-    // CUDA graphs of one step, keyed by (buffer parity, coarsening step, bio
-    // solvers' force-list operations); rebuilt when a buffer is reallocated
+    // CUDA graphs of one step or of a decade of them, keyed per step by (buffer
+    // parity, coarsening step, bio solvers' force-list operations); rebuilt
+    // when a buffer is reallocated
     struct StepGraph {
         cudaGraphExec_t exec = nullptr;
         long long launches = 0;
     };
-    std::map<int, StepGraph> graphs;
+    std::map<std::vector<int>, StepGraph> graphs;
     bool useGraphs = true;
     long long graphEpoch = 0, graphBuiltEpoch = 0;  // kernels launched by the last lbib_step / lbib_lattice_step
     long long stepsDone = 0;
@@ -929,7 +930,8 @@ static void pull_topology(Handle& h) {
 // (k_readout.cu), copies it to its pinned buffer and from there to the caller's
 // memory, with the next chunk under way meanwhile.  The copy to the caller's
 // memory (its first touch, mostly) bounds a large read-out, so several host
-// threads run a lane each, one per 2 MB up to eight; a small one is one chunk
+// threads run a lane each, one per 2 MB up to twelve (1024^2, two species: 8 lanes
+// 14.4 ms, 12 13.2, 16 12.9); a small one is one chunk
 // on the calling thread.
 constexpr size_t kReadPerLane = 2u << 20;
 
@@ -1805,9 +1807,19 @@ static bool handle_halt(Handle& h, int stage) {
     return false;
 }
 
+// Steps of one graph: a decade of steps that starts with a coarsening one.  Between
+// two graphs the GPU idles for 2 us, which a step of a small simulation (30 us)
+// notices; the decade's graph is made once a call has steps enough to use it a few
+// times (making it costs as much as ten of these gaps save).
+constexpr int kDecade = 10;
+constexpr int kDecadeFrom = 40;  // steps left in the call
+
+// The steps it, it + 1, ..., it + count - 1, the first from buffer `parity`.
 template <typename Real>
-static void launch_step_graph(Handle& h, int parity, bool coarsenStep, int bioOps) {
-    const int key = (bioOps << 2) | (coarsenStep ? 2 : 0) | parity;
+static void launch_step_graph(Handle& h, int parity, unsigned it, int count) {
+    std::vector<int> key(count);
+    for (int i = 0; i < count; ++i)
+        key[i] = (step_bio_ops(h, it + i) << 2) | ((it + i) % 10 == 0 ? 2 : 0) | ((parity + i) & 1);
     if (h.graphEpoch != h.graphBuiltEpoch) {
         for (auto& kv : h.graphs)
             if (kv.second.exec) { cudaGraphExecDestroy(kv.second.exec); kv.second.exec = nullptr; }
@@ -1817,7 +1829,10 @@ static void launch_step_graph(Handle& h, int parity, bool coarsenStep, int bioOp
     if (!g.exec) {
         cudaGraph_t graph;
         CK(cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
-        g.launches = launch_stages<Real>(h, coarsenStep, bioOps, parity, ST_FORCE, nullptr, nullptr);
+        g.launches = 0;
+        for (int i = 0; i < count; ++i)
+            g.launches += launch_stages<Real>(h, (it + i) % 10 == 0, step_bio_ops(h, it + i), (parity + i) & 1, ST_FORCE,
+                                              nullptr, nullptr);
         CK(cudaStreamEndCapture(h.stream, &graph));
         CK(cudaGraphInstantiate(&g.exec, graph, 0));
         CK(cudaGraphDestroy(graph));
@@ -1826,8 +1841,8 @@ static void launch_step_graph(Handle& h, int parity, bool coarsenStep, int bioOp
     if (check_launches()) {
         const cudaError_t e = cudaStreamSynchronize(h.stream);
         if (e != cudaSuccess)
-            std::fprintf(stderr, "lbib: step graph (parity %d, coarsen %d, bio ops %d) at iteration %u failed: %s\n",
-                         parity, coarsenStep ? 1 : 0, bioOps, h.iteration, cudaGetErrorString(e));
+            std::fprintf(stderr, "lbib: step graph (parity %d, %d steps from %u, bio ops %d) failed: %s\n", parity, count,
+                         it, step_bio_ops(h, it), cudaGetErrorString(e));
     }
     h.launches += g.launches;
 }
@@ -1860,6 +1875,7 @@ static void run_steps(Handle& h, int n) {
                          h.bio.end();
     while (n > 0) {
         int B = std::min(n, kBatch);
+        if (n > B) B -= (int)((h.iteration + B) % kDecade);  // ends with a decade
         if (hostBio) {
             // the batch ends with the next step that has host bio solvers; they follow it
             for (int b = 0; b < B; ++b)
@@ -1880,16 +1896,18 @@ static void run_steps(Handle& h, int n) {
             CK(cudaEventCreate(&e));
             h.kEvents.push_back(e);
         }
-        for (int b = 0; b < B; ++b) {
+        const bool decades = n >= kDecadeFrom;
+        for (int b = 0, count = 1; b < B; b += count) {
             const unsigned it = h.iteration + b;
-            host_step_bookkeeping(h, it);
+            count = decades && it % kDecade == 0 && b + kDecade <= B && !prof && h.useGraphs ? kDecade : 1;
+            for (int i = 0; i < count; ++i) host_step_bookkeeping(h, it + i);
             const int parity = (h.cur + b) & 1;
             if (prof || !h.useGraphs)
                 h.launches += launch_stages<Real>(h, it % 10 == 0, step_bio_ops(h, it), parity, ST_FORCE,
                                                   prof ? h.kEvents[2 * b] : nullptr,
                                                   prof ? h.kEvents[2 * b + 1] : nullptr);
             else
-                launch_step_graph<Real>(h, parity, it % 10 == 0, step_bio_ops(h, it));
+                launch_step_graph<Real>(h, parity, it, count);
         }
         CK(cudaGetLastError());
         queue_step_areas(h);
