@@ -587,7 +587,7 @@ void launch_stream_collide32(const LatticeArgs<float>& args, cudaStream_t s) {
     }
     switch (mode * 4 + (a.S < 3 ? a.S : 3)) {
 #define LBIB_SC_CASE(M, N) \
-    case M * 4 + N: launch_pdl(stream_collide32<N, M>, grid, 256, 0, s, a); break;
+    case M * 4 + N: launch_ex(!a.joined, stream_collide32<N, M>, grid, 256, 0, s, a); break;
         LBIB_SC_CASE(0, 0) LBIB_SC_CASE(0, 1) LBIB_SC_CASE(0, 2) LBIB_SC_CASE(0, 3)
         LBIB_SC_CASE(2, 0) LBIB_SC_CASE(2, 1) LBIB_SC_CASE(2, 2) LBIB_SC_CASE(2, 3)
         // coupled reactions need a partner species: two or three species

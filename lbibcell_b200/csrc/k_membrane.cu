@@ -127,14 +127,13 @@ __device__ __forceinline__ TileSlots tile_slots_take(double bx, double by, const
                                                      int ny, Status* st);
 __device__ __forceinline__ void tile_slots_put(const TileDev& t, const TileSlots& s, int i, Status* st);
 
-// `begin`: the first kernel of a step (begin_step).
 // `slots`: also enter the node in the per-tile lists of the spread (which left
 // the tile counts at zero).
 // Two records are read ahead (a membrane node has two tension records), and the
 // slot lists' atomics are under way meanwhile: 5.5 -> 4.0 us for one cell, 8.3 ->
 // 6.3 us for 150k nodes.
-__global__ void __launch_bounds__(128) force_eval_kernel(MembraneDev m, Status* st, unsigned iteration, int begin,
-                                                         TileDev t, int nx, int ny, int slots) {
+__global__ void __launch_bounds__(128) force_eval_kernel(MembraneDev m, Status* st, TileDev t, int nx,
+                                                         int ny, int slots) {
     pdl_wait();
     const int i = blockIdx.x * blockDim.x + threadIdx.x, ic = min(i, m.Mcap - 1);
     int halt = st->halt, M = m.topo->M;
@@ -142,7 +141,6 @@ __global__ void __launch_bounds__(128) force_eval_kernel(MembraneDev m, Status* 
     int r0 = m.foff[ic], r1 = m.foff[ic + 1];
     read_ahead(halt, M, x1, y1, bx, by, r0, r1);
     if (halt) return;
-    if (begin && blockIdx.x == 0 && threadIdx.x == 0) begin_step(st);
     if (i - (int)(threadIdx.x & 31) >= M) return;  // the whole warp
     bool live = i < M;
     if (!live) r0 = r1 = 0;
@@ -255,21 +253,11 @@ void launch_force_param_grad(const MembraneDev& m, const double* gfx, const doub
     force_param_grad_kernel<<<(m.Mcap + 127) / 128, 128, 0, s>>>(m, gfx, gfy, gpar);
 }
 
-template <typename Real>
-void launch_force_eval(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s, bool begin,
-                       TileDev* tiles, int nx, int ny) {
+void launch_force_eval(const MembraneDev& m, Status* st, cudaStream_t s, TileDev* tiles, int nx, int ny) {
     if (m.Mcap == 0) return;
-    TileDev t{};
-    if (tiles) {
-        t = *tiles;
-    }
-    launch_pdl(force_eval_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, st, iteration, begin ? 1 : 0, t, nx, ny,
+    launch_pdl(force_eval_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, st, tiles ? *tiles : TileDev{}, nx, ny,
                tiles ? 1 : 0);
 }
-template void launch_force_eval<double>(const MembraneDev&, Status*, unsigned, cudaStream_t, bool, TileDev*, int,
-                                        int);
-template void launch_force_eval<float>(const MembraneDev&, Status*, unsigned, cudaStream_t, bool, TileDev*, int,
-                                       int);
 
 // ---------------------------------------------------------------------------
 // Spreading
@@ -920,7 +908,7 @@ __global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, C
     pdl_wait();
     const int cn = blockIdx.x * kCrossBlock + threadIdx.x, cc = min(cn, max(m.Ccap, 1) - 1);
     const bool any = m.Ccap > 0;  // there are buffers to read from
-    int halt = st->halt, nodes = st->nPerturbNode, C = m.topo->C, a = any ? m.ca[cc] : 0, b = any ? m.cb[cc] : 0;
+    int halt = st->halt | st->err, nodes = st->nPerturbNode, C = m.topo->C, a = any ? m.ca[cc] : 0, b = any ? m.cb[cc] : 0;
     uint32_t D = any ? m.cdom[cc] : 0u;
     read_ahead(halt, nodes, C, a, b, D);
     if (halt) return;
@@ -992,7 +980,7 @@ __global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, C
             warpSum[w] = total;
             total += v;
         }
-        blockBase = total > 0 ? atomicAdd(&st->pad[2], total) : 0;
+        blockBase = total > 0 ? atomicAdd(&st->nCrossRec, total) : 0;
     }
     __syncthreads();
     if (nrec == 0) return;
@@ -1039,16 +1027,19 @@ __device__ __forceinline__ void edge_check_node(const MembraneDev& m, int i, int
 // remeshing pass will split (remesh.cuh; a kernel of its own, with the pass's
 // decision in its last block, took 6.3 us at 150k connections).  The kernel
 // first raises the halt for the connections that pass 0 listed for the host's
-// perturbation.
+// perturbation.  It is the last kernel that decides whether the domain stages run:
+// in a graph of several steps they run beside the main sequence, whose later
+// stages may halt.
 __global__ void __launch_bounds__(kRemeshBlock) cross_tie_kernel(CrossDev c, MembraneDev m, TopoDev t, int nx, int ny,
                                                                  Status* st) {
     pdl_wait();
     const int tid = blockIdx.x * kRemeshBlock + threadIdx.x, all = gridDim.x * kRemeshBlock;
     const int rc = min(tid, c.recCap - 1);
-    int halt = st->halt, conns = st->nPerturbConn, n = st->pad[2], M = m.topo->M;
+    int halt = st->halt | st->err, conns = st->nPerturbConn, n = st->nCrossRec, M = m.topo->M;
     uint32_t key = c.recKey[rc], conn = c.recConn[rc];
     unsigned long long dist = c.recDist[rc];
     read_ahead(halt, conns, n, M, key, conn, dist);
+    if (tid == 0) st->domainGo = !halt && conns == 0;
     if (halt) return;
     if (conns > 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_PERTURB_CONN);
@@ -1106,11 +1097,11 @@ __device__ __forceinline__ void record_noflux(const MembraneDev& m, CrossDev& c,
 __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom, int nx, int ny, Status* st) {
     pdl_wait();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x, rc = min(tid, c.recCap - 1);
-    int halt = st->halt, n = st->pad[2];
+    int go = st->domainGo, n = st->nCrossRec;
     uint32_t key = c.recKey[rc], conn = c.recConn[rc], bdom = c.recDom[rc];
     unsigned long long dist = c.recDist[rc];
-    read_ahead(halt, n, key, conn, bdom, dist);
-    if (halt) return;
+    read_ahead(go, n, key, conn, bdom, dist);
+    if (!go) return;
     n = min(n, c.recCap);
     for (int r = tid; r < n; r += all) {
         if (r != tid) {
@@ -1134,7 +1125,7 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
             (s == 2 ? c.bounceW : c.bounceS)[node] = 1;
             const int k = atomicAdd(c.bounceN, 1);
             if (k < c.bounceCap) c.bounceKeys[k] = key;
-            else raise_error(st, ERR_CAPACITY, (int)node, ST_CROSSINGS);
+            else raise_error_beside(st, ERR_CAPACITY, (int)node, ST_CROSSINGS);
         }
         if (s == 2) {
             c.wDom[node] = bdom + 1;
@@ -1149,7 +1140,7 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
                 c.rowNow[(uint32_t)node / (uint32_t)nx] = 1;
                 c.mark[node] = k + 1;  // the node's position in the list, for the re-initialisation
             } else {
-                raise_error(st, ERR_CAPACITY, (int)node, ST_CROSSINGS);
+                raise_error_beside(st, ERR_CAPACITY, (int)node, ST_CROSSINGS);
             }
         }
     }
@@ -1189,9 +1180,8 @@ __global__ void edge_check_kernel(MembraneDev m, int nx, int ny, Status* st, int
     edge_check_node(m, i, nx, ny, st, stage);
 }
 
-template <typename Real>
-void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, size_t L, Status* st,
-                      const TopoDev* remesh, cudaStream_t s, bool check, int* perturb, int perturbCap) {
+void launch_crossings(const MembraneDev& m, CrossDev& c, int nx, int ny, Status* st, const TopoDev* remesh,
+                       cudaStream_t s, bool check, int* perturb, int perturbCap) {
     const int blocks = (m.Ccap + kCrossBlock - 1) / kCrossBlock;
     if (m.Ccap == 0) {  // nodes without connections: the halt of the listed nodes alone
         if (check && m.Mcap > 0)
@@ -1200,7 +1190,7 @@ void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, in
     }
     if (c.nfTab != nullptr) launch_pdl(noflux_reset_kernel, 1, 1024, 0, s, c);
     if (c.bounceW != nullptr) launch_pdl(bounce_reset_kernel, 1, 1024, 0, s, c);
-    // the record count (st->pad[2]) is zero here: cleared with the status
+    // the record count (st->nCrossRec) is zero here: cleared with the status
     // word before a run and by the first kernel of each step
     launch_pdl(crossings_kernel, blocks, kCrossBlock, 0, s, m, c, nx, ny, st, check ? 1 : 0, perturb, perturbCap);
     // grid-stride over the step's records (their count is known on the device
@@ -1210,12 +1200,14 @@ void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, in
     const int recBlocks = std::min(148 * 8, (4 * m.Ccap + 255) / 256);
     launch_pdl(cross_tie_kernel, std::max(recBlocks, (m.Ccap + kRemeshBlock - 1) / kRemeshBlock), kRemeshBlock, 0, s, c, m,
                remesh ? *remesh : TopoDev{}, nx, ny, st);
-    launch_pdl(cross_win_kernel, recBlocks, 256, 0, s, c, m, dom, nx, ny, st);
 }
-template void launch_crossings<double>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
-                                       const TopoDev*, cudaStream_t, bool, int*, int);
-template void launch_crossings<float>(const MembraneDev&, CrossDev&, const uint32_t*, int, int, size_t, Status*,
-                                      const TopoDev*, cudaStream_t, bool, int*, int);
+
+void launch_cross_winners(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, Status* st,
+                          cudaStream_t s, bool programmatic) {
+    if (m.Ccap == 0) return;
+    launch_ex(programmatic, cross_win_kernel, std::min(148 * 8, (4 * m.Ccap + 255) / 256), 256, 0, s, c, m, dom, nx, ny,
+              st);
+}
 
 void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s) {
     if (m.Mcap == 0) return;
@@ -1416,12 +1408,12 @@ __global__ void __launch_bounds__(kReinitBlock) reinit_kernel(CrossDev c, uint32
     pdl_wait();
     const int lane = threadIdx.x & 31, warps = kReinitBlock / 32, warp = threadIdx.x >> 5;
     const int k0 = blockIdx.x * warps + warp;
-    int halt = st->halt, cnt = st->nChanged, typesCopied = st->cellTypesCopied;
+    int go = st->domainGo, cnt = st->nChanged, typesCopied = st->cellTypesCopied;
     uint32_t iteration = st->iteration, node0 = c.changedNode[min(k0, c.changedCap - 1)];
-    read_ahead(halt, cnt, typesCopied, iteration, node0);
-    if (halt || cnt == 0) return;
+    read_ahead(go, cnt, typesCopied, iteration, node0);
+    if (!go || cnt == 0) return;
     if (cnt > kReinitMax || cnt > c.changedCap) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(st, ERR_CAPACITY, cnt, ST_REINIT);
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_error_beside(st, ERR_CAPACITY, cnt, ST_REINIT);
         return;
     }
     const SpeciesConst* sp = species.s;
@@ -1526,25 +1518,42 @@ template void launch_reinit<float>(CrossDev&, uint32_t*, float*, const float*, i
 // access) and a block scan the kernel took 6.5 us for 1024^2 and 25 us for a
 // 2048^2 lattice with cells in its middle; this form takes 6.1 and 9.1 us.
 constexpr int kFillBlock = 128, kFillSeg = 8;
-__global__ void __launch_bounds__(kFillBlock) domain_fill_kernel(CrossDev c, uint32_t* dom, int nx, int ny,
+__device__ __forceinline__ void fill_row(const CrossDev& c, uint32_t* dom, int nx, int y, Status* st);
+
+// The last block ends the step (end_step).  `gated`: the crossings' ties ran and
+// decided whether the domain stages do (else, without connections, the halt word).
+__global__ void __launch_bounds__(kFillBlock) domain_fill_kernel(CrossDev c, uint32_t* dom, int nx, int gated,
                                                                  Status* st) {
     pdl_wait();
     const int y = blockIdx.x;
     const size_t row = (size_t)y * nx;
     // everything the block's course depends on, read at once
-    const int nrec = min(st->pad[2], c.recCap), halt = st->halt;
-    const bool marked = c.rowNow[y] | c.rowHad[y];
-    const uint32_t left = dom[row];
+    int nrec = st->nCrossRec, go = gated ? st->domainGo : !st->halt, marked = c.rowNow[y] | c.rowHad[y];
+    uint32_t left = dom[row];
+    read_ahead(nrec, go, marked, left);
+    nrec = min(nrec, c.recCap);
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nrec; k += gridDim.x * blockDim.x) {
         const uint32_t key = c.recKey[k];
         c.bnDist[key] = kEmpty;
         c.bnConn[key] = ~0u;
     }
-    if (halt || !marked) return;
-    if (left != 0) {
-        if (threadIdx.x == 0) raise_error(st, ERR_LEFT_DOMAIN, y, ST_DOMAIN);
-        return;
+    if (go && marked) {
+        if (left == 0) fill_row(c, dom, nx, y, st);
+        else if (threadIdx.x == 0) raise_error_beside(st, ERR_LEFT_DOMAIN, y, ST_DOMAIN);
     }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd((unsigned*)&c.nWait[2], 1u) == gridDim.x - 1) {
+            c.nWait[2] = 0;
+            __threadfence();
+            end_step(st, go);
+        }
+    }
+}
+
+__device__ __forceinline__ void fill_row(const CrossDev& c, uint32_t* dom, int nx, int y, Status* st) {
+    const size_t row = (size_t)y * nx;
     constexpr int warps = kFillBlock / 32;
     __shared__ uint32_t lastOf[warps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1599,9 +1608,8 @@ __global__ void __launch_bounds__(kFillBlock) domain_fill_kernel(CrossDev c, uin
     }
 }
 
-void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, size_t L, Status* st, unsigned iteration,
-                        cudaStream_t s) {
-    launch_pdl(domain_fill_kernel, ny, kFillBlock, 0, s, c, dom, nx, ny, st);
+void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, Status* st, cudaStream_t s, bool gated) {
+    launch_pdl(domain_fill_kernel, ny, kFillBlock, 0, s, c, dom, nx, gated ? 1 : 0, st);
 }
 
 
@@ -1698,7 +1706,7 @@ __global__ void __launch_bounds__(256) areas_kernel(MembraneDev m, double* area,
     const int np = e - b;
     __shared__ double terms[kAreaMax];
     if (np > kAreaMax) {
-        if (threadIdx.x == 0 && st) raise_error(st, ERR_CAPACITY, cell, ST_BIO);
+        if (threadIdx.x == 0 && st) raise_error_beside(st, ERR_CAPACITY, cell, ST_BIO);
         return;
     }
     for (int k = threadIdx.x; k < np; k += blockDim.x) {
@@ -1874,11 +1882,12 @@ void launch_area_regulator(const MembraneDev& m, double* area, double* target, d
 void launch_area_regulator_fixed(const MembraneDev& m, const int* cellOfDom, unsigned long long* acc, double* area,
                                  double* target, double* massTab, int nDomains, double factor, double strength,
                                  double maxsource, const uint32_t* ctypeTab, const Status* st, cudaStream_t s,
-                                 bool summed) {
+                                 bool summed, bool programmatic) {
     if (m.nCells == 0 || m.Ccap == 0) return;
-    if (!summed) launch_pdl(areas_fixed_kernel, (m.Ccap + 255) / 256, 256, 0, s, m, cellOfDom, nDomains, acc);
-    launch_pdl(area_regulator_kernel, (m.nCells + 127) / 128, 128, 0, s, m, area, target, massTab, nDomains, factor,
-               strength, maxsource, ctypeTab, acc, st);
+    if (!summed)
+        launch_ex(programmatic, areas_fixed_kernel, (m.Ccap + 255) / 256, 256, 0, s, m, cellOfDom, nDomains, acc);
+    launch_ex(programmatic || !summed, area_regulator_kernel, (m.nCells + 127) / 128, 128, 0, s, m, area, target, massTab,
+              nDomains, factor, strength, maxsource, ctypeTab, acc, st);
 }
 
 // ---------------------------------------------------------------------------

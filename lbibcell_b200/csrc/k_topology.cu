@@ -610,7 +610,7 @@ __device__ void ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
         while ((int)(*(volatile unsigned*)t.ringMeet - meet) < 0) {
             __nanosleep(64);
             if (++tries > 4000000u) {
-                raise_error(st, ERR_STATE, (int)blockIdx.x, ST_BIO);
+                raise_error_beside(st, ERR_STATE, (int)blockIdx.x, ST_BIO);
                 break;
             }
         }
@@ -626,7 +626,8 @@ __device__ void ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
 // change cost 75 us at 390 cells of 380 nodes (the seven launches 25 us), now
 // 26 us.  Values that other blocks wrote in this launch are read past the L1
 // cache.
-__global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, int nCells, Status* st) {
+// beside: launched beside the main sequence (raise_error_beside).
+__global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, int nCells, Status* st, int beside) {
     if (!m.topo->changed) return;
     const int M = m.topo->M, C = m.topo->C;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
@@ -685,7 +686,10 @@ __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, in
     for (int cell = blockIdx.x; cell < nCells; cell += gridDim.x) {
         const int b = __ldcg(&t.cellStart[cell]), len = __ldcg(&t.cellCount[cell]);
         if (len > kRingMax) {
-            if (threadIdx.x == 0) raise_error(st, ERR_CAPACITY, cell, ST_BIO);
+            if (threadIdx.x == 0) {
+                if (beside) raise_error_beside(st, ERR_CAPACITY, cell, ST_BIO);
+                else raise_error(st, ERR_CAPACITY, cell, ST_BIO);
+            }
             continue;
         }
         __syncthreads();
@@ -722,6 +726,7 @@ __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, in
             const int i = __ldcg(&t.members[b + p]);
             const int d = sDist[p];
             if (d >= 0 && d < len) m.ringNode[b + (len - 1 - d)] = i;
+            else if (beside) raise_error_beside(st, ERR_STATE, i, ST_BIO);
             else raise_error(st, ERR_STATE, i, ST_BIO);
         }
         if (threadIdx.x == 0) m.ringStart[cell] = b;
@@ -772,7 +777,7 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
     conn_perturb_gather_kernel<<<(n + 127) / 128, 128, 0, s>>>(m, t, n, out);
 }
 
-int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
+int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside) {
     const int nCells = t.nCellsCap;
     if (m.Mcap == 0 || nCells == 0) return 0;
     // two blocks per SM at most: never more than are resident together
@@ -786,7 +791,7 @@ int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, rings_kernel, m, t, nCells, st);
+    cudaLaunchKernelEx(&cfg, rings_kernel, m, t, nCells, st, beside ? 1 : 0);
     return 1;
 }
 

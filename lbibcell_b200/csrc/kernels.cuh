@@ -93,7 +93,8 @@ struct CrossDev {
     int* mark;                   // L, position + 1 of a node in this step's changed list (0: none)
     int* reinitDone;             // changedCap: 1 = re-initialised by the wide pass, 2 + w = waiting at waitList[w]
     int* waitList;               // changedCap: list positions of the nodes that wait for another
-    int* nWait;                  // [0] entries of waitList, [1] blocks of the re-initialisation that are through
+    int* nWait;                  // [0] entries of waitList, [1], [2] blocks of the re-initialisation and of the fill
+                                 // that are through
     uint32_t* changedNode;       // capacity: nodes whose domain changes
     uint32_t* changedDom;
     int changedCap;
@@ -178,30 +179,31 @@ void launch_init32(float* f, float* g, float* u, int nS, size_t L, double tauF, 
                    const double* vel, const SpeciesConst* sp, const double* init, cudaStream_t s);
 
 // Membrane pipeline.  `Real` is the lattice precision (velocity / force planes).
-template <typename Real>
 // `tiles`: also fill the spread's per-tile slot lists (then call launch_spread
 // with slotsFilled).
-void launch_force_eval(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s, bool begin = false,
-                       TileDev* tiles = nullptr, int nx = 0, int ny = 0);
+void launch_force_eval(const MembraneDev& m, Status* st, cudaStream_t s, TileDev* tiles = nullptr, int nx = 0,
+                       int ny = 0);
 template <typename Real>
 void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny, size_t L, Status* st,
                    unsigned iteration, cudaStream_t s, bool slotsFilled = false);
 template <typename Real>
 void launch_interp_move(const MembraneDev& m, const Real* u, int nx, int ny, size_t L, CrossDev& c, Status* st,
                         unsigned iteration, cudaStream_t s);
-// The crossings, and (remesh != nullptr) the count of the step's remeshing pass.
-// `check`: first raise the halts of the move's listed nodes and of connections
-// that need the host's perturbation (listed in perturb[0..perturbCap)).
-template <typename Real>
-void launch_crossings(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, size_t L, Status* st,
-                      const TopoDev* remesh, cudaStream_t s, bool check = false, int* perturb = nullptr,
-                      int perturbCap = 0);
+// The crossings and their ties, and (remesh != nullptr) the count of the step's
+// remeshing pass.  `check`: first raise the halts of the move's listed nodes and of
+// connections that need the host's perturbation (listed in perturb[0..perturbCap)).
+void launch_crossings(const MembraneDev& m, CrossDev& c, int nx, int ny, Status* st, const TopoDev* remesh,
+                      cudaStream_t s, bool check = false, int* perturb = nullptr, int perturbCap = 0);
+// The domain stages: the crossings' winners (programmatic: the launch before it on
+// the stream is the ties' own), the re-initialisation, and the fill, which ends
+// the step (gated: the ties decide whether it runs).
+void launch_cross_winners(const MembraneDev& m, CrossDev& c, const uint32_t* dom, int nx, int ny, Status* st,
+                          cudaStream_t s, bool programmatic);
 template <typename Real>
 void launch_reinit(CrossDev& c, uint32_t* dom, Real* g, const Real* u, int nS, const SpeciesConst* sp,
                    const double* srcTab, int nDomains, const uint32_t* ctypeTab, int cellTypesCopied, int nx,
                    int ny, size_t L, Status* st, unsigned iteration, cudaStream_t s);
-void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, size_t L, Status* st, unsigned iteration,
-                        cudaStream_t s);
+void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, Status* st, cudaStream_t s, bool gated);
 void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s);
 void launch_remesh_check(Status* st, unsigned iteration, cudaStream_t s);
 void launch_coarsen_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s);
@@ -244,11 +246,12 @@ void launch_areas_fixed(const MembraneDev& m, const int* cellOfDom, int nDomains
                         double* area, cudaStream_t s);
 // FP32-shifted runs: areas from the connections in fixed point (no ring order
 // needed), then the regulator.  acc (nCells) must start at zero; it is left zero.
-// summed: the remeshing commit formed the sums already.
+// summed: the remeshing commit formed the sums already.  programmatic: the launch
+// before it on the stream is all it waits for.
 void launch_area_regulator_fixed(const MembraneDev& m, const int* cellOfDom, unsigned long long* acc, double* area,
                                  double* target, double* massTab, int nDomains, double factor, double strength,
                                  double maxsource, const uint32_t* ctypeTab, const Status* st, cudaStream_t s,
-                                 bool summed = false);
+                                 bool summed = false, bool programmatic = true);
 // massNode[n] = massTab[dom[n]] (0 outside cells).
 void launch_mass_expand(const uint32_t* dom, size_t L, const double* massTab, int nDomains, double* massNode,
                         const Status* st, cudaStream_t s);
@@ -283,7 +286,8 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
 int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly = false,
                   unsigned long long* areaAcc = nullptr);
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
-int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
+// beside: beside the main sequence (raise_error_beside).
+int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside = false);
 size_t topo_scan_bytes(int n);
 
 // Adjoint of one FP64 lattice step of a differentiated run (k_adjoint.cu).

@@ -145,7 +145,10 @@ struct Status {
     int nFailedReinit; // reinit without any neighbour (division by zero)
     unsigned iteration;   // Parameters' current iteration of the step being run
     int cellTypesCopied;  // copyCellTypeToPhysicalNodes has run (after the first step)
-    int pad[4];           // [0] steps of a run completed before its current one, [2] crossing records of the step, [3] first step of a run
+    int stepsDone;     // steps whose domain stage is through (end_step)
+    int errStage;      // stage of an error raised beside the main sequence (raise_error_beside)
+    int nCrossRec;     // crossing records of the step
+    int domainGo;      // this step's domain stages (winners, re-initialisation, fill) run
 };
 
 // Stage numbers (halt points), in the reference's order of
@@ -189,28 +192,26 @@ __device__ __forceinline__ void raise_error(Status* st, int code, int index, int
     atomicCAS(&st->haltStage, 0, stage);
 }
 
-// The start of a step, run by thread 0 of the step's first kernel when no halt
-// is pending: the step before it in the same run is then complete, so it is
-// counted (Parameters++, SimulationRunner.cpp:98) before this step's kernels
-// read the iteration; then the step's counters are cleared.  pad[3], set with
-// the status word, marks the first step of a run, which has no predecessor
-// there.  (The host counts the run's last step itself: it completed unless a
-// halt is pending.)
-__device__ __forceinline__ void begin_step(Status* st) {
-    if (st->pad[3]) {
-        st->pad[3] = 0;
-    } else {
-        st->pad[0] += 1;
+// An error of a stage that runs beside the main sequence (the domain stages, the
+// cell areas): the main sequence must not see a halt that its own kernels did not
+// wait for.  The next step's crossings stop on the error word.
+__device__ __forceinline__ void raise_error_beside(Status* st, int code, int index, int stage) {
+    if (atomicCAS(&st->err, 0, code) == 0) st->errIndex = index;
+    atomicCAS(&st->errStage, 0, stage);
+}
+
+// The end of a step's domain stages, run by one thread once all their blocks are
+// through: the step counts as done (Parameters++, SimulationRunner.cpp:98; the host
+// takes it back when a later stage of the step halts), copyCellTypeToPhysicalNodes
+// has run, and the counters are clear for the next crossings.
+__device__ __forceinline__ void end_step(Status* st, bool ran) {
+    if (ran && st->err == 0) {
+        st->stepsDone += 1;
         st->iteration += 1;
         st->cellTypesCopied = 1;
     }
-    st->pad[2] = 0;
-    st->nPerturbNode = 0;
-    st->nPerturbConn = 0;
+    st->nCrossRec = 0;
     st->nChanged = 0;
-    st->nRecords = 0;
-    st->remesh = 0;
-    st->coarsen = 0;
 }
 
 __device__ __forceinline__ void raise_halt(Status* st, int stage) {
@@ -300,6 +301,7 @@ struct LatticeArgs {
     SpeciesConst sp[kMaxSpecies];
     int coupled;               // some species has a coupled_kind reaction
     const Status* status;
+    int joined;                // the launch follows a join of two streams (no programmatic launch)
     int outlet;                // MassSolverBoxOutlet registered: rescale x=0 / y=0 nodes
     // no-flux boundary nodes of the previous step's crossings (nullptr: none)
     const uint8_t* nfSpec;     // 4*L: descriptor index + 1 per (node, slot E,N,W,S), 0 none
