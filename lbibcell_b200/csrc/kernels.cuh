@@ -135,10 +135,11 @@ struct TileDev {
 constexpr int kTileSlots = 1024;
 
 // Scratch of the device-side topology edits and the ring ranking.
+constexpr int kMeetBlocks = 296;  // blocks of a launch that meets at ring_barrier: two per SM
 struct TopoDev {
     int* flag;          // Ccap + 1
     int* rank;          // Ccap + 1
-    int* nflag;         // Mcap + 1
+    int* blockSum;      // 3 * kMeetBlocks
     int* nrank;         // Mcap + 1
     int* ca2; int* cb2; uint32_t* cdom2; int* cdesc2;    // Ccap
     double* dalt;       // 10 * Mcap node doubles
@@ -157,8 +158,7 @@ struct TopoDev {
     int* succ; int* dist;                                 // Mcap
     int* rngList;       // Mcap: new nodes of a remesh pass that need the host's random perturbation
     int* startNode;     // nCells
-    unsigned* ringMeet; // rings_kernel: [0] arrivals at its barriers, ever; [1] those of the launches that are through
-    void* scanTmp; size_t scanTmpBytes;
+    unsigned* ringMeet; // ring_barrier: [0] arrivals, ever; [1] those of the launches that are through
     int nDomains;
 };
 
@@ -285,10 +285,10 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
 // ST_REMESH_RNG).  areaAcc: also add the shoelace terms of the final list.
 int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly = false,
                   unsigned long long* areaAcc = nullptr);
+// ForceSolver::deleteAllForces (on a halted step too), then coarsenBoundary.
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
 // beside: beside the main sequence (raise_error_beside).
 int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside = false);
-size_t topo_scan_bytes(int n);
 
 // Adjoint of one FP64 lattice step of a differentiated run (k_adjoint.cu).
 struct AdjointArgs {

@@ -472,11 +472,11 @@ Handle::~Handle() {
     fr(cross.nfSpec); fr(cross.nfU); fr(cross.nfN); fr(nfTabDev);
     fr(cross.bounceW); fr(cross.bounceS); fr(cross.bounceKeys); fr(cross.bounceN);
     fr(m.cdesc);  // m.topo lives in the status allocation
-    fr(td.flag); fr(td.rank); fr(td.nflag); fr(td.nrank); fr(td.ca2); fr(td.cb2); fr(td.cdom2); fr(td.cdesc2);
+    fr(td.flag); fr(td.rank); fr(td.blockSum); fr(td.nrank); fr(td.ca2); fr(td.cb2); fr(td.cdom2); fr(td.cdesc2);
     fr(td.dalt); fr(td.id2); fr(td.prev2); fr(td.next2); fr(td.inConn); fr(td.outConn); fr(td.removed);
     fr(td.connAlive); fr(td.ncA); fr(td.ncB); fr(td.ncDom); fr(td.ncDesc); fr(td.ncAlive); fr(td.cellOfDom);
     fr(td.firstConn); fr(td.cellCount); fr(td.cellStart); fr(td.cellFill); fr(td.members); fr(td.succ); fr(td.rngList);
-    fr(td.dist); fr(td.startNode); fr(td.scanTmp); fr(td.ringMeet);
+    fr(td.dist); fr(td.startNode); fr(td.ringMeet);
     fr(st);
     if (stHost) cudaFreeHost(stHost);  // topoHost lives in the same block
     if (evA) cudaEventDestroy(evA);
@@ -1155,11 +1155,11 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
         fr(h.m.x); fr(h.m.y); fr(h.m.ox); fr(h.m.oy); fr(h.m.vx); fr(h.m.vy); fr(h.m.fx); fr(h.m.fy); fr(h.m.bx); fr(h.m.by);
         fr(h.m.id); fr(h.m.prev); fr(h.m.next); fr(h.outPos); fr(h.inPos); fr(h.cross.perturbList);
         fr(h.m.foff); fr(h.m.ringNode);
-        fr(h.td.nflag); fr(h.td.nrank); fr(h.td.dalt); fr(h.td.id2); fr(h.td.prev2); fr(h.td.next2);
+        fr(h.td.blockSum); fr(h.td.nrank); fr(h.td.dalt); fr(h.td.id2); fr(h.td.prev2); fr(h.td.next2);
         fr(h.td.inConn); fr(h.td.outConn); fr(h.td.removed); fr(h.td.ncA); fr(h.td.ncB); fr(h.td.ncDom);
         fr(h.td.ncDesc); fr(h.td.ncAlive); fr(h.td.members); fr(h.td.succ); fr(h.td.dist); fr(h.td.rngList);
         const int n = h.Mcap;
-        h.td.nflag = dalloc<int>(n + 1); h.td.nrank = dalloc<int>(n + 1);
+        h.td.blockSum = dalloc<int>(3 * kMeetBlocks); h.td.nrank = dalloc<int>(n + 1);
         h.td.dalt = dalloc<double>(10 * (size_t)n);
         h.td.id2 = dalloc<uint32_t>(n); h.td.prev2 = dalloc<int>(n); h.td.next2 = dalloc<int>(n);
         h.td.inConn = dalloc<int>(n); h.td.outConn = dalloc<int>(n);
@@ -1237,13 +1237,6 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
         h.td.cellFill = dalloc<int>(h.cellCap); h.td.startNode = dalloc<int>(h.cellCap);
     }
     ensure_force_scratch(h);
-    // scan scratch for the largest scan (nodes, connections or cells)
-    const size_t need = topo_scan_bytes(std::max(std::max(h.Mcap, h.Ccap), h.cellCap) + 1);
-    if (need > h.td.scanTmpBytes) {
-        if (h.td.scanTmp) cudaFree(h.td.scanTmp);
-        CK(cudaMalloc(&h.td.scanTmp, need));
-        h.td.scanTmpBytes = need;
-    }
     h.m.Mcap = h.Mcap;
     h.m.Ccap = h.Ccap;
 }
@@ -1403,8 +1396,8 @@ __global__ void iteration_inc_kernel(Status* st) {
 // cell areas and the area regulator depend on nothing that the rest of the step and
 // the next step's force and spread change, and the other way round: they run on
 // `side`, beside them, and join before the next step's lattice kernel.  Long calls,
-// one after the other against so: 200^2 FP32 29.5 -> 25.4 us a step, FP64 37 -> 30.7,
-// 337x521 56 -> 48, 1024^2 FP32 125 -> 113, FP64 200 -> 176.  In graphs of one step
+// one after the other against so: 200^2 FP32 29.5 -> 25.0 us a step, FP64 37 -> 31.4,
+// 337x521 56 -> 49, 1024^2 FP32 125 -> 111, FP64 200 -> 177.  In graphs of one step
 // only the remeshing runs beside them: 1024^2 136 -> 130 us, 200^2 34.4 -> 31.5.
 struct StepFork {
     cudaStream_t side;
@@ -1494,8 +1487,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
                             summed ? h.areaAcc : nullptr);
     if (fromStage <= ST_COARSEN && coarsenStep) {
         // SimulationRunner.cpp:84-87: ForceSolver::deleteAllForces, then coarsenBoundary
-        launch_clear_forces(h.m, s);
-        nl += 1 + launch_coarsen(h.m, h.td, h.st, s);
+        nl += launch_coarsen(h.m, h.td, h.st, s);
     }
     // ST_OUTLET: MassSolverBoxOutlet runs inside the stream-collide kernel
     if (fromStage <= ST_BIO) {

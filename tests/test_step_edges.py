@@ -19,6 +19,8 @@ SIZES = {
     "row of 257": (257, 33, [(100.3, 16.6, 9.0, 128), (230.1, 16.3, 9.5, 129)], 3, 22),
     "dense tile list": (48, 50, [(24.2, 25.3, 5.0, 300)], 1, 12),
     "dense, coarsened": (64, 64, [(32.2, 31.3, 9.0, 700)], 2, 22),
+    "256 nodes, coarsened": (48, 48, [(24.2, 24.3, 4.0, 256)], 1, 12),
+    "one of two coarsened, 513 nodes": (72, 48, [(20.2, 24.3, 4.0, 453), (50.1, 23.2, 9.6, 60)], 1, 22),
     "column of 600": (40, 600, [(20.2, 40.0 + 130.0 * k, 9.0 + k, 110 + 19 * k) for k in range(5)], 1, 22),
 }
 
