@@ -362,10 +362,10 @@ __device__ __forceinline__ int pack_stencil(const Stencil& s, int tileX0, int ti
 // The tile's list as the spread takes it: its length, noted for the readers of
 // the force field, and the counter left at zero for the next step's lists (a
 // memset node between two kernels of the step cost 3.5 us).
-// -1 on a halted step.  `first`: entry threadIdx.x of the list, if it has one.
-__device__ __forceinline__ int take_tile_count(const TileDev& t, int tile, const Status* st, int& first) {
+// -1 on a halted step.  `first`: the list's entry of that place, if it has one.
+__device__ __forceinline__ int take_tile_count(const TileDev& t, int tile, const Status* st, int place, int& first) {
     int halt = st->halt, count = t.count[tile];
-    first = t.slots[(size_t)tile * kTileSlots + threadIdx.x];
+    first = t.slots[(size_t)tile * kTileSlots + place];
     read_ahead(halt, count, first);
     if (halt) return -1;
     __syncthreads();
@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) spread_kernel(MembraneDev m, TileDev t, R
     pdl_wait();
     const int tile = blockIdx.x;
     int first;
-    const int cnt = take_tile_count(t, tile, st, first);
+    const int cnt = take_tile_count(t, tile, st, threadIdx.x, first);
     if (cnt <= 0) return;
     if (cnt > kSpreadMax) {
         if (threadIdx.x == 0) raise_error(st, ERR_CAPACITY, tile, ST_SPREAD);
@@ -520,6 +520,12 @@ __global__ void __launch_bounds__(256) spread_kernel(MembraneDev m, TileDev t, R
 // the ordered gather and rounded once; the integer sums are exact, so the
 // field does not depend on the order of the list (it is deterministic) and no
 // sort is needed.  The rounding is far below FP32 resolution.
+// Bound by instruction issue where tiles hold many nodes, by the chain of reads
+// where there is one cell.  Two lanes form a node's factors, one per axis, the
+// force is staged with the products' power of two (an exact scaling), and the
+// usual 4 x 4 stencil has its own loop: 150k nodes on 1024^2 21.6 -> 19.0 us, one
+// cell on 200^2 4.5 -> 3.9 us against a lane per node and one loop.  Blocks of 64
+// to 192 threads, or a warp's entries spread along the list: no gain.
 constexpr double kForceFix = 17592186044416.0;  // 2^44
 constexpr int kScatterChunk = 256;
 __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDev t, float* force, int nx, int ny,
@@ -527,15 +533,16 @@ __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDe
     pdl_wait();
     const int tile = blockIdx.x;
     int first;
-    const int cnt = min(take_tile_count(t, tile, st, first), kTileSlots);
+    const int cnt = min(take_tile_count(t, tile, st, threadIdx.x >> 1, first), kTileSlots);
     if (cnt <= 0) return;
     // each 64-bit fixed-point sum is kept as a signed high part (bits 22..63)
     // and an unsigned low part (bits 0..21), each summed with 32-bit integer
     // atomics: the low parts of up to 1024 contributions cannot overflow
     __shared__ int accHi[2][kTile * kTile];
     __shared__ unsigned accLo[2][kTile * kTile];
-    __shared__ double fa[kScatterChunk][5], fb[kScatterChunk][5], sF[2][kScatterChunk];
-    __shared__ int org[kScatterChunk];
+    // per axis and node: the Dirac factors, the force (scaled), the stencil's origin + 4 and its width << 8
+    __shared__ double fab[2][kScatterChunk][5], sF[2][kScatterChunk];
+    __shared__ int org[2][kScatterChunk];
     for (int j = threadIdx.x; j < kTile * kTile; j += blockDim.x) {
         accHi[0][j] = accHi[1][j] = 0;
         accLo[0][j] = accLo[1][j] = 0u;
@@ -548,55 +555,51 @@ __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDe
     for (int c0 = 0; c0 < cnt; c0 += kScatterChunk) {
         const int nc = min(kScatterChunk, cnt - c0);
         __syncthreads();
-        for (int e = threadIdx.x; e < nc; e += blockDim.x) {
-            const int i = c0 == 0 ? first : list[c0 + e];  // (a chunk is a block's threads)
-            const double X = m.x[i], Y = m.y[i];
-            Stencil sc;
-            stencil_range(m.bx[i], m.by[i], nx, ny, sc);
-            org[e] = pack_stencil(sc, tileX0, tileY0);
+        for (int j = threadIdx.x; j < 2 * nc; j += blockDim.x) {
+            const int e = j >> 1, axis = j & 1;
+            const int i = c0 == 0 && j == threadIdx.x ? first : list[c0 + e];
+            const double X = axis ? m.y[i] : m.x[i], B = axis ? m.by[i] : m.bx[i];
+            const double F = axis ? m.fy[i] : m.fx[i];
+            const int lo = (int)ceil(B - 2.0), hi = (int)floor(B + 2.0);  // (stencil_range)
+            org[axis][e] = (lo - (axis ? tileY0 : tileX0) + 4) | ((hi - lo) << 8);
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                fa[e][q] = 1.0 + fast_cos(halfPi * ((double)(sc.x0 + q) - X));
-                fb[e][q] = 1.0 + fast_cos(halfPi * ((double)(sc.y0 + q) - Y));
-            }
-            sF[0][e] = m.fx[i];
-            sF[1][e] = m.fy[i];
+            for (int q = 0; q < 5; ++q) fab[axis][e][q] = 1.0 + fast_cos(halfPi * ((double)(lo + q) - X));
+            sF[axis][e] = F * (kForceFix / 16.0);
         }
         __syncthreads();
         // one item per (node, slot row r): slots k = 4 r .. 4 r + 3 of the
         // node's 16 (in a 4 x 4 stencil, column dx = r, rows dy = 0..3)
         for (int j = threadIdx.x; j < 4 * nc; j += blockDim.x) {
             const int e = j >> 2, r = j & 3;
-            const int c = org[e];
-            const int ox = (c & 0xff) - 4, oy = ((c >> 8) & 0xff) - 4, hx = (c >> 16) & 0xf, hy = (c >> 20) & 0xf;
-            const bool plain = hx == 3 && hy == 3;
-            if (plain && (unsigned)(ox + r) >= (unsigned)kTile) continue;  // the column lies outside the tile
-            const Stencil sc{ox + tileX0, ox + tileX0 + hx, oy + tileY0, oy + tileY0 + hy};
+            const int cx = org[0][e], cy = org[1][e];
+            const int ox = (cx & 0xff) - 4, oy = (cy & 0xff) - 4, hx = cx >> 8, hy = cy >> 8;
             const double Fx = sF[0][e], Fy = sF[1][e];
-#pragma unroll
-            for (int t4 = 0; t4 < 4; ++t4) {
-                int dx, dy;  // node of slot k relative to the stencil origin
-                if (plain) {
-                    dx = r;
-                    dy = t4;
-                } else {
-                    // wider stencil: the node bound to slot k (last writer of the slot)
-                    int xk, yk;
-                    stencil_slot(sc, 4 * r + t4, xk, yk);
-                    if (xk < 0) continue;
-                    dx = xk - sc.x0;
-                    dy = yk - sc.y0;
-                }
-                const int lx = ox + dx, ly = oy + dy;
-                if ((unsigned)lx >= (unsigned)kTile || (unsigned)ly >= (unsigned)kTile) continue;
-                const double dl = (fa[e][dx] * fb[e][dy]) / 16.0;
-                const long long vx = __double2ll_rn(Fx * dl * kForceFix);
-                const long long vy = __double2ll_rn(Fy * dl * kForceFix);
-                const int node = ly * kTile + lx;
+            auto add = [&](int node, double w) {  // w: 16 x the Dirac weight
+                const long long vx = __double2ll_rn(Fx * w);
+                const long long vy = __double2ll_rn(Fy * w);
                 atomicAdd(&accHi[0][node], (int)(vx >> 22));
                 atomicAdd(&accLo[0][node], (unsigned)(vx & 0x3fffff));
                 atomicAdd(&accHi[1][node], (int)(vy >> 22));
                 atomicAdd(&accLo[1][node], (unsigned)(vy & 0x3fffff));
+            };
+            if (hx == 3 && hy == 3) {
+                if ((unsigned)(ox + r) >= (unsigned)kTile) continue;  // the column lies outside the tile
+                const double a = fab[0][e][r];
+                const int node = oy * kTile + ox + r;
+#pragma unroll
+                for (int t4 = 0; t4 < 4; ++t4)
+                    if ((unsigned)(oy + t4) < (unsigned)kTile) add(node + t4 * kTile, a * fab[1][e][t4]);
+            } else {
+                // wider stencil: the node bound to slot k (last writer of the slot)
+                const Stencil sc{ox + tileX0, ox + tileX0 + hx, oy + tileY0, oy + tileY0 + hy};
+                for (int t4 = 0; t4 < 4; ++t4) {
+                    int xk, yk;
+                    stencil_slot(sc, 4 * r + t4, xk, yk);
+                    if (xk < 0) continue;
+                    const int lx = xk - tileX0, ly = yk - tileY0;
+                    if ((unsigned)lx >= (unsigned)kTile || (unsigned)ly >= (unsigned)kTile) continue;
+                    add(ly * kTile + lx, fab[0][e][xk - sc.x0] * fab[1][e][yk - sc.y0]);
+                }
             }
         }
     }
