@@ -401,8 +401,8 @@ struct Handle {
     bool statusContinues = false;
     int lastPad0 = 0;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;  // captured into the step graphs (StepFork), made with the first
-    cudaEvent_t evForked = nullptr, evCommitted = nullptr, evJoined = nullptr;
+    cudaStream_t side = nullptr, sums = nullptr;  // captured into the step graphs (StepFork), made with the first
+    cudaEvent_t evForked = nullptr, evCommitted = nullptr, evJoined = nullptr, evSummed = nullptr;
 
     std::mt19937 genNode{1};
     std::mt19937 genConn{1};
@@ -490,9 +490,10 @@ Handle::~Handle() {
     fr(fs.inCnt); fr(fs.inOff); fr(fs.inList); fr(fs.inFill);
     if (readReady) cudaEventDestroy(readReady);
     if (inLanePool) lane_pool(device).leave();
-    for (cudaEvent_t e : {evForked, evCommitted, evJoined})
+    for (cudaEvent_t e : {evForked, evCommitted, evJoined, evSummed})
         if (e) cudaEventDestroy(e);
     if (side) cudaStreamDestroy(side);
+    if (sums) cudaStreamDestroy(sums);
     if (stream) cudaStreamDestroy(stream);
 }
 
@@ -1392,16 +1393,19 @@ __global__ void iteration_inc_kernel(Status* st) {
     pdl_wait(); st->iteration += 1; }
 
 // A step within a graph.  Its domain stages (the crossings' winners, the
-// re-initialisation, the domain fill: short latency-bound kernels on few blocks), the
-// cell areas and the area regulator depend on nothing that the rest of the step and
-// the next step's force and spread change, and the other way round: they run on
-// `side`, beside them, and join before the next step's lattice kernel.  Long calls,
-// one after the other against so: 200^2 FP32 29.5 -> 25.0 us a step, FP64 37 -> 31.4,
-// 337x521 56 -> 49, 1024^2 FP32 125 -> 111, FP64 200 -> 177.  In graphs of one step
-// only the remeshing runs beside them: 1024^2 136 -> 130 us, 200^2 34.4 -> 31.5.
+// re-initialisation, the domain fill: short latency-bound kernels on few blocks)
+// depend on nothing that the rest of the step and the next step's force and spread
+// change, and the other way round: they run on `side`, beside them, and join before
+// the next step's lattice kernel.  So do, on `sums`, the ring order, the cell areas
+// and the area regulator, which need the committed positions alone.  Long calls, in
+// one stream, with `side`, with both: 200^2 FP32 29.5, 25.0, 24.5 us a step, FP64 37,
+// 31.4, 28.4; 337x521 56, 49, 48; 1024^2 FP32 125, 111, 109, FP64 200, 177, 172.
+// (`sums` at 200^2 FP32: 0.9 us slower on one device of four, 0.4 to 2 faster on the
+// others, so it has no lower bound.)  In graphs of one step only the remeshing runs
+// beside them: 1024^2 136 -> 130 us, 200^2 34.4 -> 31.5.
 struct StepFork {
-    cudaStream_t side;
-    cudaEvent_t forked, committed, joined;
+    cudaStream_t side, sums;
+    cudaEvent_t forked, committed, joined, summed;
     bool first, last;  // of the graph
 };
 
@@ -1455,7 +1459,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
         launch_interp_move<Real>(h.m, (const Real*)h.u, h.nx, h.ny, h.L, h.cross, h.st, it, s);
         nl += hasM;
     }
-    cudaStream_t d = s;  // the domain stages' stream
+    cudaStream_t d = s, a = s;  // the streams of the domain stages and of the cell areas
     if (fromStage <= ST_CROSSINGS) {
         // ST_PERTURB_CONN: the test runs with the crossings
         launch_crossings(h.m, h.cross, h.nx, h.ny, h.st, &h.td, s, fromStage <= ST_PERTURB_CONN, h.td.rngList, h.Mcap);
@@ -1491,26 +1495,27 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
     }
     // ST_OUTLET: MassSolverBoxOutlet runs inside the stream-collide kernel
     if (fromStage <= ST_BIO) {
-        if (fork != nullptr && d != s) {  // the final positions and connections, for the areas
+        if (fork != nullptr && (area || sizeof(Real) == 8)) {  // the final positions and connections, for the areas
+            a = fork->sums;
             CK(cudaEventRecord(fork->committed, s));
-            CK(cudaStreamWaitEvent(d, fork->committed, 0));
+            CK(cudaStreamWaitEvent(a, fork->committed, 0));
         }
         // FP64 runs sum the areas in ring order (the reference's order), so the
         // rings are re-ranked after any topology change; FP32-shifted runs sum
         // in exact fixed point and need no ring order here
-        if (sizeof(Real) == 8) nl += launch_rings(h.m, h.td, h.st, d, d != s);
+        if (sizeof(Real) == 8) nl += launch_rings(h.m, h.td, h.st, a, a != s);
         for (size_t q = 0; q < h.bio.size(); ++q) {
             const int b = h.bio[q], op = (bioOps >> (2 * q)) & 3;
             if (b == 2) {
                 const uint32_t* ct = h.areaTutorial ? h.ctypeTab : nullptr;
                 if (sizeof(Real) == 8) {
                     launch_area_regulator(h.m, h.area, h.target, h.massTab, h.nDomains, h.areaFactor,
-                                          h.areaStrength, h.areaMax, ct, h.st, d);
+                                          h.areaStrength, h.areaMax, ct, h.st, a);
                     nl += h.m.nCells > 0 ? 2 : 0;
                 } else {
                     launch_area_regulator_fixed(h.m, h.td.cellOfDom, h.areaAcc, h.area, h.target, h.massTab,
-                                                h.nDomains, h.areaFactor, h.areaStrength, h.areaMax, ct, h.st, d, summed,
-                                                d == s);
+                                                h.nDomains, h.areaFactor, h.areaStrength, h.areaMax, ct, h.st, a, summed,
+                                                a == s);
                     nl += h.m.nCells > 0 ? (summed ? 1 : 2) : 0;
                 }
                 if (h.massNode != nullptr) {
@@ -1534,6 +1539,10 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
         if (!fork->last) nl += launch_front<Real>(h, ST_FORCE);  // the next step's
         CK(cudaEventRecord(fork->joined, d));
         CK(cudaStreamWaitEvent(s, fork->joined, 0));
+        if (a != s) {
+            CK(cudaEventRecord(fork->summed, a));
+            CK(cudaStreamWaitEvent(s, fork->summed, 0));
+        }
     }
     return nl;
 }
@@ -1863,13 +1872,13 @@ static void launch_step_graph(Handle& h, int parity, unsigned it, int count) {
         // across the two streams: those runs keep to one
         const bool forked = h.m.Ccap > 0 && h.cross.nfTab == nullptr && h.massNode == nullptr;
         if (forked && !h.side) {
-            CK(cudaStreamCreateWithFlags(&h.side, cudaStreamNonBlocking));
-            for (cudaEvent_t* e : {&h.evForked, &h.evCommitted, &h.evJoined})
+            for (cudaStream_t* q : {&h.side, &h.sums}) CK(cudaStreamCreateWithFlags(q, cudaStreamNonBlocking));
+            for (cudaEvent_t* e : {&h.evForked, &h.evCommitted, &h.evJoined, &h.evSummed})
                 CK(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
         }
         CK(cudaStreamBeginCapture(h.stream, cudaStreamCaptureModeThreadLocal));
         for (int i = 0; i < count; ++i) {
-            StepFork fork{h.side, h.evForked, h.evCommitted, h.evJoined, i == 0, i == count - 1};
+            StepFork fork{h.side, h.sums, h.evForked, h.evCommitted, h.evJoined, h.evSummed, i == 0, i == count - 1};
             g.launches += launch_stages<Real>(h, (it + i) % 10 == 0, step_bio_ops(h, it + i), (parity + i) & 1, ST_FORCE,
                                               nullptr, nullptr, forked ? &fork : nullptr);
         }

@@ -203,11 +203,16 @@ __device__ __forceinline__ void raise_error_beside(Status* st, int code, int ind
 // The end of a step's domain stages, run by one thread once all their blocks are
 // through: the step counts as done (Parameters++, SimulationRunner.cpp:98; the host
 // takes it back when a later stage of the step halts), copyCellTypeToPhysicalNodes
-// has run, and the counters are clear for the next crossings.
+// has run, and the counters are clear for the next crossings.  An error of the step's
+// later stages, which may be running beside, doesn't change the count.
 __device__ __forceinline__ void end_step(Status* st, bool ran) {
-    if (ran && st->err == 0) {
-        st->stepsDone += 1;
-        st->iteration += 1;
+    int err = st->err, errStage = st->errStage, haltStage = st->haltStage, done = st->stepsDone;
+    int iteration = (int)st->iteration;
+    read_ahead(err, errStage, haltStage, done, iteration);
+    const int stage = errStage ? errStage : haltStage;
+    if (ran && (err == 0 || stage == 0 || stage >= ST_REMESH)) {
+        st->stepsDone = done + 1;
+        st->iteration = (unsigned)iteration + 1u;
         st->cellTypesCopied = 1;
     }
     st->nCrossRec = 0;
