@@ -52,11 +52,16 @@ __device__ __forceinline__ int gen_count(const ForceScratch& fs, int gen, int i)
     return (fs.closest[i] >= 0 ? 1 : 0) + fs.inCnt[i];
 }
 
+// The scan that follows runs on a halted step as well: there the counts are those
+// of the list as it stands, so that the scan leaves its offsets as they are.
 __global__ void force_count_kernel(MembraneDev m, ForceScratch fs, int delType, int gen, Status* st) {
     pdl_wait();
-    if (st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > m.Mcap) return;
+    if (st->halt) {
+        fs.cnt[i] = i < m.Mcap ? m.foff[i + 1] - m.foff[i] : 0;
+        return;
+    }
     const int M = m.topo->M;
     if (i >= M) {
         fs.cnt[i] = 0;

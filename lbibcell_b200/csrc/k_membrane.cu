@@ -1648,30 +1648,35 @@ void launch_coarsen_check(const MembraneDev& m, Status* st, unsigned iteration, 
     launch_pdl(coarsen_check_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, st);
 }
 
-__global__ void clear_forces_kernel(MembraneDev m) {
+// st: a step's stage, which a halted step skips (else nullptr).
+__global__ void clear_forces_kernel(MembraneDev m, const Status* st) {
     pdl_wait();
+    if (st != nullptr && st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= m.topo->M) m.foff[i] = 0;
 }
 
-void launch_clear_forces(MembraneDev& m, cudaStream_t s) {
-    launch_pdl(clear_forces_kernel, (m.Mcap + 1 + 255) / 256, 256, 0, s, m);
+void launch_clear_forces(MembraneDev& m, cudaStream_t s, const Status* st) {
+    launch_pdl(clear_forces_kernel, (m.Mcap + 1 + 255) / 256, 256, 0, s, m, st);
 }
 
 // Tension renewal when the force list holds only tension pairs: node i gets
 // one type-6 record toward each ring neighbour, ordered by the position of the
 // contributing connection in the connection vector
 // (tutorial_01_BioSolverMembraneTension.cpp:52-73 adds them in that order).
-__global__ void tension_pos_kernel(MembraneDev m, int* outPos, int* inPos) {
+__global__ void tension_pos_kernel(MembraneDev m, int* outPos, int* inPos, const Status* st) {
     pdl_wait();
+    if (st->halt) return;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.topo->C) return;
     outPos[m.ca[c]] = c;
     inPos[m.cb[c]] = c;
 }
 
-__global__ void tension_fill_kernel(MembraneDev m, const int* outPos, const int* inPos, double force) {
+__global__ void tension_fill_kernel(MembraneDev m, const int* outPos, const int* inPos, double force,
+                                    const Status* st) {
     pdl_wait();
+    if (st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i > m.topo->M) return;
     m.foff[i] = 2 * i;
@@ -1688,10 +1693,10 @@ __global__ void tension_fill_kernel(MembraneDev m, const int* outPos, const int*
     }
 }
 
-void launch_tension_renewal(MembraneDev& m, int* outPos, int* inPos, double force, cudaStream_t s) {
+void launch_tension_renewal(MembraneDev& m, int* outPos, int* inPos, double force, const Status* st, cudaStream_t s) {
     if (m.Mcap == 0) return;
-    launch_pdl(tension_pos_kernel, (m.Ccap + 127) / 128, 128, 0, s, m, outPos, inPos);
-    launch_pdl(tension_fill_kernel, (m.Mcap + 1 + 127) / 128, 128, 0, s, m, outPos, inPos, force);
+    launch_pdl(tension_pos_kernel, (m.Ccap + 127) / 128, 128, 0, s, m, outPos, inPos, st);
+    launch_pdl(tension_fill_kernel, (m.Mcap + 1 + 127) / 128, 128, 0, s, m, outPos, inPos, force, st);
 }
 
 // ---------------------------------------------------------------------------

@@ -247,14 +247,15 @@ int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaSt
 // ---------------------------------------------------------------------------
 // Coarsen
 
-// Clears the force list (on a halted step too); node -> its incoming / outgoing
-// connection; candidates.
+// Clears the force list; node -> its incoming / outgoing connection; candidates.
+// (A halted step leaves the list alone: the steps between the one that halted and
+// this one, queued behind it, have yet to use it.)
 __global__ void coarsen_begin_kernel(MembraneDev m, TopoDev t, Status* st) {
     pdl_wait();
+    if (st->halt) return;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int M = m.topo->M;
     if (i <= M) m.foff[i] = 0;
-    if (st->halt) return;
     if (i < m.topo->C) {
         t.outConn[m.ca[i]] = i;
         t.inConn[m.cb[i]] = i;
@@ -843,7 +844,7 @@ __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, 
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {
     const int nCells = t.nCellsCap;
     if (m.Mcap == 0 || nCells == 0) {
-        launch_clear_forces(m, s);
+        launch_clear_forces(m, s, st);
         return 1;
     }
     const int blocks = (std::max(m.Mcap, m.Ccap) + 1 + 255) / 256;

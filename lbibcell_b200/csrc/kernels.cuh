@@ -207,7 +207,7 @@ void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, Status* st, 
 void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s);
 void launch_remesh_check(Status* st, unsigned iteration, cudaStream_t s);
 void launch_coarsen_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s);
-void launch_clear_forces(MembraneDev& m, cudaStream_t s);
+void launch_clear_forces(MembraneDev& m, cudaStream_t s, const Status* st = nullptr);
 // ForceSolver::deleteForceType(6) + the membrane-tension records, on a list that
 // holds other forces too (launches returned).
 int launch_tension_edit(MembraneDev& m, ForceScratch& fs, double force, Status* st, cudaStream_t s);
@@ -229,7 +229,7 @@ void launch_range_query(MembraneDev& m, ForceScratch& fs, int nx, int ny, const 
                         const long long* avoid, int nq, double radius, int mode, unsigned* ids, int cap, int* count,
                         long long* closest, cudaStream_t s);
 size_t junction_sort_bytes(int n, int bits);
-void launch_tension_renewal(MembraneDev& m, int* outPos, int* inPos, double force, cudaStream_t s);
+void launch_tension_renewal(MembraneDev& m, int* outPos, int* inPos, double force, const Status* st, cudaStream_t s);
 // ctypeTab != nullptr selects tutorial_01_BioSolverAreaRegulator's rule (fixed
 // target, cell type 1 at maxsource); nullptr the LbibAreaRegulator rule.
 void launch_area_regulator(const MembraneDev& m, double* area, double* target, double* massTab, int nDomains,
@@ -285,7 +285,7 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
 // ST_REMESH_RNG).  areaAcc: also add the shoelace terms of the final list.
 int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaStream_t s, bool commitOnly = false,
                   unsigned long long* areaAcc = nullptr);
-// ForceSolver::deleteAllForces (on a halted step too), then coarsenBoundary.
+// ForceSolver::deleteAllForces, then coarsenBoundary.
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
 // beside: beside the main sequence (raise_error_beside).
 int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside = false);

@@ -1526,7 +1526,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
                 launch_growth<Real>(gcur, h.dom, h.L, h.growthR, h.growthL, h.massNode, h.st, s);
                 nl += 1;
             } else if (b == 1 && op == BIO_TENSION_FILL) {
-                launch_tension_renewal(h.m, h.outPos, h.inPos, h.tensionForce, s);
+                launch_tension_renewal(h.m, h.outPos, h.inPos, h.tensionForce, h.st, s);
                 nl += hasM ? 2 : 0;
             } else if (b == 1 && op == BIO_TENSION_EDIT) {
                 nl += launch_tension_edit(h.m, h.fs, h.tensionForce, h.st, s);
