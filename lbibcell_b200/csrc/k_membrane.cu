@@ -1150,9 +1150,11 @@ __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom,
 }
 
 // Clears the previous step's no-flux boundary nodes (after the stream-collide
-// that used them, before this step's crossings set the new ones).
-__global__ void noflux_reset_kernel(CrossDev c) {
+// that used them, before this step's crossings set the new ones).  A halted
+// step, which ran no stream-collide, leaves them to the step that will.
+__global__ void noflux_reset_kernel(CrossDev c, const Status* st) {
     pdl_wait();
+    if (st->halt) return;
     const int n = min(*c.nfN, c.nfCap);
     for (int k = threadIdx.x; k < n; k += blockDim.x) c.nfSpec[c.nfKeys[k]] = 0;
     __syncthreads();
@@ -1160,9 +1162,11 @@ __global__ void noflux_reset_kernel(CrossDev c) {
 }
 
 // Clears the previous step's W / S boundary-node marks (after the
-// stream-collide that used them, before this step's crossings set new ones).
-__global__ void bounce_reset_kernel(CrossDev c) {
+// stream-collide that used them, before this step's crossings set new ones);
+// not on a halted step (noflux_reset_kernel).
+__global__ void bounce_reset_kernel(CrossDev c, const Status* st) {
     pdl_wait();
+    if (st->halt) return;
     const int n = min(*c.bounceN, c.bounceCap);
     for (int k = threadIdx.x; k < n; k += blockDim.x) {
         const uint32_t key = c.bounceKeys[k];
@@ -1191,8 +1195,8 @@ void launch_crossings(const MembraneDev& m, CrossDev& c, int nx, int ny, Status*
             launch_pdl(crossings_kernel, 1, kCrossBlock, 0, s, m, c, nx, ny, st, 1, perturb, perturbCap);
         return;
     }
-    if (c.nfTab != nullptr) launch_pdl(noflux_reset_kernel, 1, 1024, 0, s, c);
-    if (c.bounceW != nullptr) launch_pdl(bounce_reset_kernel, 1, 1024, 0, s, c);
+    if (c.nfTab != nullptr) launch_pdl(noflux_reset_kernel, 1, 1024, 0, s, c, st);
+    if (c.bounceW != nullptr) launch_pdl(bounce_reset_kernel, 1, 1024, 0, s, c, st);
     // the record count (st->nCrossRec) is zero here: cleared with the status
     // word before a run and by the first kernel of each step
     launch_pdl(crossings_kernel, blocks, kCrossBlock, 0, s, m, c, nx, ny, st, check ? 1 : 0, perturb, perturbCap);
