@@ -523,8 +523,12 @@ __device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
 // 26 us.  Values that other blocks wrote in this launch are read past the L1
 // cache.
 // beside: launched beside the main sequence (raise_error_beside).
+// A remeshing pass that is applied but not committed (it waits for the host; the
+// step is halted) has linked nodes into the rings that the counts and the
+// connections do not hold yet: the ranking waits for the commit.  No kernel that
+// may run beside this one changes K.
 __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, int nCells, Status* st, int beside) {
-    if (!m.topo->changed) return;
+    if (!m.topo->changed || m.topo->K != 0) return;
     const int M = m.topo->M, C = m.topo->C;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
     unsigned meet = *(volatile unsigned*)&t.ringMeet[1];  // arrivals of the launches before this one

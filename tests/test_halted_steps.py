@@ -150,3 +150,43 @@ def test_moved_node_event_in_a_graph_of_ten_steps(lbib, oracle_mod, tmp_path, ma
         st = o.state()
         _equal({k: a[k] for k in ("f", "g", "vel", "force", "dom", "ctype", "ids", "node", "conn")},
                {k: getattr(st, k) for k in ("f", "g", "vel", "force", "dom", "ctype", "ids", "node", "conn")})
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_new_node_event_at_a_coarsening_step(lbib, oracle_mod, tmp_path, precision):
+    """A growing cell is remeshed in iterations 7 to 13.  The geometry is
+    shifted until a node made at iteration 10, a coarsening step, lies on a
+    lattice line: the step halts with the pass applied and not committed, and
+    with a ring order that the passes before have outdated."""
+    rng = np.random.default_rng(10)
+    shift = 0.0
+    for attempt in range(12 if precision == lbib.FP64 else 80):
+        cfg = configs.toy(n=64, r=12.0, nodes=155, iterations=200, report_step=50, species=1)
+        cfg.cells = [(1, configs.circle(32.2 + shift, 31.7, 12.0, 155, phase=0.3))]
+        cfg.tension, cfg.area = (0.1, 10), (3.0, 0.2, 0.05)
+        paths = cfg.write(str(tmp_path / str(attempt)))
+        sim = lbib.Simulation(paths, precision)
+        at = _single_steps(sim, 10)
+        before = sim.membrane()[0]
+        at += _single_steps(sim, 1)
+        if at == [10]:
+            break
+        ids, node = sim.membrane()
+        assert len(before) > 155 and len(ids) > len(before)
+        x = node[np.isin(ids, np.setdiff1d(ids, before)), 0]
+        off = x - np.round(x)
+        shift -= off[np.argmin(np.abs(off))] + (0.0 if precision == lbib.FP64 else rng.uniform(-1e-8, 1e-8))
+        sim.close()
+    assert at == [10], f"no event at iteration 10: {at}"
+    assert _single_steps(sim, 44 - 11) == []
+    whole = lbib.Simulation(paths, precision)
+    whole.step(44)
+    assert whole.sizes()["host_events"] == 1
+    a = _state(whole)
+    _equal(a, _state(sim))
+    if precision == lbib.FP64:
+        o = oracle_mod.Oracle(paths)
+        o.step(44)
+        st = o.state()
+        _equal({k: a[k] for k in ("f", "g", "vel", "force", "dom", "ctype", "ids", "node", "conn")},
+               {k: getattr(st, k) for k in ("f", "g", "vel", "force", "dom", "ctype", "ids", "node", "conn")})
