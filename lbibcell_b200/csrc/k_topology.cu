@@ -493,8 +493,15 @@ constexpr int kRingPerThread = 16;  // 256 threads x 16 = 4096 nodes per ring
 constexpr int kRingMax = 256 * kRingPerThread;
 
 // All blocks of the launch meet (a cooperative launch: they are resident).
-// The wait is bounded; a block that gives up raises the error, and false is returned.
-__device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
+// The wait is bounded; a block that gives up raises the error, and false is
+// returned: the block then leaves, since what the others were to write may be
+// missing.  The arrivals no longer tell where a launch stands after that, so
+// later launches that would meet do nothing (ringMeet[2]).
+// stage: that of the main sequence, which the error halts; 0: beside it.
+#ifndef LBIB_MEET_TRIES
+#define LBIB_MEET_TRIES 4000000u
+#endif
+__device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st, int stage) {
     __syncthreads();
     int late = 0;
     if (threadIdx.x == 0) {
@@ -504,8 +511,10 @@ __device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
         unsigned tries = 0;
         while ((int)(*(volatile unsigned*)t.ringMeet - meet) < 0) {
             __nanosleep(64);
-            if (++tries > 4000000u) {
-                raise_error_beside(st, ERR_STATE, (int)blockIdx.x, ST_BIO);
+            if (++tries > LBIB_MEET_TRIES) {
+                t.ringMeet[2] = 1u;
+                if (stage != 0) raise_error(st, ERR_STATE, (int)blockIdx.x, stage);
+                else raise_error_beside(st, ERR_STATE, (int)blockIdx.x, ST_BIO);
                 late = 1;
                 break;
             }
@@ -528,7 +537,8 @@ __device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st) {
 // connections do not hold yet: the ranking waits for the commit.  No kernel that
 // may run beside this one changes K.
 __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, int nCells, Status* st, int beside) {
-    if (!m.topo->changed || m.topo->K != 0) return;
+    if (!m.topo->changed || m.topo->K != 0 || t.ringMeet[2] != 0u) return;
+    const int stage = beside ? 0 : ST_BIO;
     const int M = m.topo->M, C = m.topo->C;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
     unsigned meet = *(volatile unsigned*)&t.ringMeet[1];  // arrivals of the launches before this one
@@ -544,7 +554,7 @@ __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, in
             agg_min(&t.firstConn[m.cdom[c]], (int)m.cdom[c], c);
         }
     }
-    ring_barrier(t, meet, st);
+    if (!ring_barrier(t, meet, st, stage)) return;
     for (int i0 = blockIdx.x * blockDim.x; i0 < M; i0 += all) {
         const int i = i0 + threadIdx.x;
         if (i < M) {
@@ -552,7 +562,7 @@ __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, in
             agg_add(&t.cellCount[cell], cell);
         }
     }
-    ring_barrier(t, meet, st);
+    if (!ring_barrier(t, meet, st, stage)) return;
     if (blockIdx.x == 0) {  // the cells' places: an exclusive prefix of their counts
         typedef cub::BlockScan<int, 256> Scan;
         __shared__ typename Scan::TempStorage tmp;
@@ -566,7 +576,7 @@ __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, in
             ex += __ldcg(&t.cellCount[c]);
         }
     }
-    ring_barrier(t, meet, st);
+    if (!ring_barrier(t, meet, st, stage)) return;
     for (int i0 = blockIdx.x * blockDim.x; i0 < M; i0 += all) {
         const int i = i0 + threadIdx.x;
         if (i < M) {
@@ -580,7 +590,7 @@ __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, in
             t.dist[i] = k;  // the node's place among its cell's members
         }
     }
-    ring_barrier(t, meet, st);
+    if (!ring_barrier(t, meet, st, stage)) return;
     // each ring's ranks by pointer jumping, one block per cell
     __shared__ int sNext[kRingMax], sDist[kRingMax];  // by place: the next node's place (-1: none), the links to the end
     for (int cell = blockIdx.x; cell < nCells; cell += gridDim.x) {
@@ -739,7 +749,7 @@ __device__ __forceinline__ void block_places(const bool (&flag)[3], int (&place)
 // 49.2 -> 46.8, 1024^2 FP64 178 -> 172 (FP32 111 -> 110).
 __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, TopoDev t, int, Status* st, int) {
     Topo* T = m.topo;
-    if (st->halt) return;
+    if (st->halt || t.ringMeet[2] != 0u) return;
     if (T->removed == 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) T->nCand = 0;
         return;
@@ -759,7 +769,7 @@ __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, 
         cnt[2] += __syncthreads_count(i < M && t.ncAlive[i]);
     }
     if (threadIdx.x < 3) t.blockSum[threadIdx.x * nb + blockIdx.x] = cnt[threadIdx.x];
-    if (!ring_barrier(t, meet, st)) return;
+    if (!ring_barrier(t, meet, st, ST_COARSEN)) return;
     for (int k = 0; k < 3; ++k) {
         int lo = 0, sum = 0;
         for (int b = threadIdx.x; b < nb; b += 256) {
@@ -797,7 +807,7 @@ __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, 
 #pragma unroll
         for (int k = 0; k < 3; ++k) at[k] += sum[k];
     }
-    if (!ring_barrier(t, meet, st)) return;
+    if (!ring_barrier(t, meet, st, ST_COARSEN)) return;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, stride = nb * blockDim.x;
     for (int i0 = beg; i0 < end; i0 += 256) {
         const int i = i0 + threadIdx.x;
@@ -826,7 +836,7 @@ __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, 
         m.id[i] = __ldcg(&t.id2[i]);
         if (i == Mn - 1) T->maxId = __ldcg(&t.id2[i]);
     }
-    if (!ring_barrier(t, meet, st)) return;
+    if (!ring_barrier(t, meet, st, ST_COARSEN)) return;
     for (int i = tid; i < Mn; i += stride) {
         m.prev[i] = __ldcg(&t.prev2[i]);
         m.next[i] = __ldcg(&t.next2[i]);

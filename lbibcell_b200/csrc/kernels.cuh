@@ -158,7 +158,7 @@ struct TopoDev {
     int* succ; int* dist;                                 // Mcap
     int* rngList;       // Mcap: new nodes of a remesh pass that need the host's random perturbation
     int* startNode;     // nCells
-    unsigned* ringMeet; // ring_barrier: [0] arrivals, ever; [1] those of the launches that are through
+    unsigned* ringMeet; // ring_barrier: [0] arrivals, ever; [1] those of the launches that are through; [2] a wait ran out
     int nDomains;
 };
 

@@ -2162,8 +2162,8 @@ static void create(Handle& h, const std::string& params, const std::string& geom
     CK(cudaMemsetAsync(h.tiles.count, 0, sizeof(int) * h.tiles.nTiles, h.stream));
     CK(cudaMemsetAsync(h.tiles.active, 0, sizeof(int) * h.tiles.nTiles, h.stream));
 
-    h.td.ringMeet = dalloc<unsigned>(2);
-    CK(cudaMemsetAsync(h.td.ringMeet, 0, 2 * sizeof(unsigned), h.stream));
+    h.td.ringMeet = dalloc<unsigned>(3);
+    CK(cudaMemsetAsync(h.td.ringMeet, 0, 3 * sizeof(unsigned), h.stream));
 
     // crossing planes
     h.cross.bnDist = dalloc<unsigned long long>(4 * h.L);
