@@ -688,11 +688,12 @@ void launch_conn_perturb_gather(const MembraneDev& m, const TopoDev& t, int n, C
 }
 
 // Blocks that meet at ring_barrier: two per SM at most, never more than are
-// resident together.
+// resident together (meet_blocks).  A launch that the device refuses leaves its
+// error for the caller's cudaGetLastError.
 static void launch_meeting(void (*kernel)(MembraneDev, TopoDev, int, Status*, int), int blocks, const MembraneDev& m,
                            const TopoDev& t, int arg, Status* st, int arg2, cudaStream_t s) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)std::min(kMeetBlocks, blocks));
+    cfg.gridDim = dim3((unsigned)std::min(t.meetBlocks, blocks));
     cfg.blockDim = dim3(256);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -853,6 +854,16 @@ __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, 
         T->removed = 0;
         T->nCand = 0;
     }
+}
+
+cudaError_t meet_blocks(int* blocks) {
+    int device = 0, sms = 0, rings = 0, compact = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&rings, rings_kernel, 256, 0);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&compact, coarsen_compact_kernel, 256, 0);
+    *blocks = std::max(1, sms * std::min(2, std::min(rings, compact)));
+    return e;
 }
 
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s) {

@@ -135,11 +135,11 @@ struct TileDev {
 constexpr int kTileSlots = 1024;
 
 // Scratch of the device-side topology edits and the ring ranking.
-constexpr int kMeetBlocks = 296;  // blocks of a launch that meets at ring_barrier: two per SM
 struct TopoDev {
     int* flag;          // Ccap + 1
     int* rank;          // Ccap + 1
-    int* blockSum;      // 3 * kMeetBlocks
+    int meetBlocks;     // most blocks of a launch that meets at ring_barrier (meet_blocks)
+    int* blockSum;      // 3 * meetBlocks
     int* nrank;         // Mcap + 1
     int* ca2; int* cb2; uint32_t* cdom2; int* cdesc2;    // Ccap
     double* dalt;       // 10 * Mcap node doubles
@@ -289,6 +289,9 @@ int launch_remesh(MembraneDev& m, TopoDev& t, int nx, int ny, Status* st, cudaSt
 int launch_coarsen(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s);
 // beside: beside the main sequence (raise_error_beside).
 int launch_rings(MembraneDev& m, TopoDev& t, Status* st, cudaStream_t s, bool beside = false);
+// The blocks of a launch whose blocks wait for one another (launch_rings, the
+// compaction) that the current device holds at once, at most two per SM.
+cudaError_t meet_blocks(int* blocks);
 
 // Adjoint of one FP64 lattice step of a differentiated run (k_adjoint.cu).
 struct AdjointArgs {

@@ -1160,7 +1160,7 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
         fr(h.td.inConn); fr(h.td.outConn); fr(h.td.removed); fr(h.td.ncA); fr(h.td.ncB); fr(h.td.ncDom);
         fr(h.td.ncDesc); fr(h.td.ncAlive); fr(h.td.members); fr(h.td.succ); fr(h.td.dist); fr(h.td.rngList);
         const int n = h.Mcap;
-        h.td.blockSum = dalloc<int>(3 * kMeetBlocks); h.td.nrank = dalloc<int>(n + 1);
+        h.td.blockSum = dalloc<int>(3 * h.td.meetBlocks); h.td.nrank = dalloc<int>(n + 1);
         h.td.dalt = dalloc<double>(10 * (size_t)n);
         h.td.id2 = dalloc<uint32_t>(n); h.td.prev2 = dalloc<int>(n); h.td.next2 = dalloc<int>(n);
         h.td.inConn = dalloc<int>(n); h.td.outConn = dalloc<int>(n);
@@ -1883,6 +1883,7 @@ static void launch_step_graph(Handle& h, int parity, unsigned it, int count) {
                                               nullptr, nullptr, forked ? &fork : nullptr);
         }
         CK(cudaStreamEndCapture(h.stream, &graph));
+        CK(cudaGetLastError());  // a launch that was refused is not in the graph
         CK(cudaGraphInstantiate(&g.exec, graph, 0));
         CK(cudaGraphDestroy(graph));
     }
@@ -2162,6 +2163,7 @@ static void create(Handle& h, const std::string& params, const std::string& geom
     CK(cudaMemsetAsync(h.tiles.count, 0, sizeof(int) * h.tiles.nTiles, h.stream));
     CK(cudaMemsetAsync(h.tiles.active, 0, sizeof(int) * h.tiles.nTiles, h.stream));
 
+    CK(meet_blocks(&h.td.meetBlocks));
     h.td.ringMeet = dalloc<unsigned>(3);
     CK(cudaMemsetAsync(h.td.ringMeet, 0, 3 * sizeof(unsigned), h.stream));
 

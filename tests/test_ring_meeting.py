@@ -1,7 +1,8 @@
 """The meetings of the cooperative launches (ring order, compaction): a wait
 that runs out ends the launch with an error, on the main sequence also with the
 halt, before anything that the other blocks would have written is used; the
-launches after it do nothing.  The kernels are compiled here with a short limit
+launches after it do nothing.  Their grids are no larger than the device holds at
+once, and a launch that it refuses is reported.  The kernels are compiled here with a short limit
 and launched as one block that is told to wait for arrivals that never come."""
 import ctypes
 import os
@@ -71,6 +72,28 @@ extern "C" int meet(int compaction, int beside, unsigned missing, int* out) {
     cudaFree(a);
     return 0;
 }
+
+// The error of a ring launch over a membrane of 2^24 nodes, unchanged since its
+// last ranking (every block returns at once), on a grid of at most `blocks`
+// (0: meet_blocks).  *most: meet_blocks.
+extern "C" int grid(int blocks, int* most) {
+    if (meet_blocks(most) != cudaSuccess) return -1;
+    int* a;
+    if (cudaMalloc(&a, 4096) != cudaSuccess) return -1;
+    cudaMemset(a, 0, 4096);
+    MembraneDev m{};
+    m.topo = (Topo*)a;
+    m.Mcap = m.Ccap = 1 << 24;
+    TopoDev t{};
+    t.nCellsCap = 1;
+    t.meetBlocks = blocks ? blocks : *most;
+    t.ringMeet = (unsigned*)(a + 512);
+    launch_rings(m, t, (Status*)(a + 256), 0);
+    const int e = (int)cudaGetLastError();
+    if (cudaDeviceSynchronize() != cudaSuccess) return -1;
+    cudaFree(a);
+    return e;
+}
 """
 ERR_STATE, ST_COARSEN, ST_BIO = 91, 11, 13
 
@@ -88,8 +111,10 @@ def meet(tmp_path_factory):
     subprocess.run([build.NVCC] + build.ARCH + build.COMMON + [
         "--fmad=false", "-DLBIB_MEET_TRIES=20000u", "-I" + build.CSRC, "-shared", "-cudart", "static", source, "-o",
         library], check=True)
-    function = ctypes.CDLL(library).meet
+    L = ctypes.CDLL(library)
+    function = L.meet
     function.argtypes = [ctypes.c_int, ctypes.c_int, ctypes.c_uint, ctypes.c_void_p]
+    L.grid.argtypes = [ctypes.c_int, ctypes.c_void_p]
 
     def call(compaction, beside, missing):
         out = (ctypes.c_int * 10)()
@@ -97,6 +122,11 @@ def meet(tmp_path_factory):
         keys = ("err", "errStage", "halt", "haltStage", "changed", "removed", "ran_out", "ringStart", "err2",
                 "changed2")
         return dict(zip(keys, out))
+
+    def grid(blocks):
+        most = ctypes.c_int()
+        return L.grid(blocks, ctypes.byref(most)), most.value
+    call.grid = grid
     return call
 
 
@@ -122,3 +152,13 @@ def test_a_wait_that_runs_out(meet, compaction, beside):
     assert got["ran_out"] == 1
     # the next launch leaves at once, without another error
     assert (got["err2"], got["changed2"]) == (0, 1)
+
+
+def test_grid_fits_the_device(meet):
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    e, most = meet.grid(0)
+    assert e == 0 and sms <= most <= 2 * sms and most % sms == 0
+    e, _ = meet.grid(most * 64)
+    assert e == 720  # cudaErrorCooperativeLaunchTooLarge
+    assert meet.grid(0)[0] == 0
