@@ -367,8 +367,7 @@ __device__ __forceinline__ int take_tile_count(const TileDev& t, int tile, const
     int halt = st->halt, count = t.count[tile];
     first = t.slots[(size_t)tile * kTileSlots + place];
     read_ahead(halt, count, first);
-    if (halt) return -1;
-    __syncthreads();
+    if (__syncthreads_or(halt)) return -1;  // (the block as one: the spread raises errors itself)
     if (threadIdx.x == 0) {
         t.active[tile] = count;
         if (count != 0) t.count[tile] = 0;
@@ -914,16 +913,16 @@ __global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, C
     int halt = st->halt | st->err, nodes = st->nPerturbNode, C = m.topo->C, a = any ? m.ca[cc] : 0, b = any ? m.cb[cc] : 0;
     uint32_t D = any ? m.cdom[cc] : 0u;
     read_ahead(halt, nodes, C, a, b, D);
-    if (halt) return;
-    if (check && nodes > 0) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
-        return;
-    }
+    // Other blocks may raise an error meanwhile, between the reads of two warps
+    // of this block: a warp that sees it has no records, and takes part in the
+    // block's count of them all the same.
+    const bool wait = check && nodes > 0;
+    if (wait && !halt && blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
     int nrec = 0;
     bool simple = false;
     CrossRec r[4];
     bool have[4] = {false, false, false, false};
-    if (cn < C) {
+    if (cn < C && !halt && !wait) {
         const double x1 = m.x[a], y1 = m.y[a], x2 = m.x[b], y2 = m.y[b];
         if (check && (fabs(x1 - x2) < kEPSILON || fabs(y1 - y2) < kEPSILON)) {
             const int k = atomicAdd(&st->nPerturbConn, 1);

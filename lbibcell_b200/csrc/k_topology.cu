@@ -285,7 +285,8 @@ constexpr size_t kCoarsenSmem = (size_t)kCoarsenMax * (2 * sizeof(double) + size
 // removing node h - Ccap.
 __global__ void __launch_bounds__(256) coarsen_cell_kernel(MembraneDev m, TopoDev t, Status* st) {
     pdl_wait();
-    if (st->halt || m.topo->nCand == 0) return;
+    // (the block as one: a ring that is too long raises an error here)
+    if (__syncthreads_or(st->halt) || m.topo->nCand == 0) return;
     const int cell = blockIdx.x;
     const int b = m.ringStart[cell], len = m.ringStart[cell + 1] - b;
     if (len > kCoarsenMax) {
@@ -537,7 +538,8 @@ __device__ bool ring_barrier(const TopoDev& t, unsigned& meet, Status* st, int s
 // connections do not hold yet: the ranking waits for the commit.  No kernel that
 // may run beside this one changes K.
 __global__ void __launch_bounds__(256) rings_kernel(MembraneDev m, TopoDev t, int nCells, Status* st, int beside) {
-    if (!m.topo->changed || m.topo->K != 0 || t.ringMeet[2] != 0u) return;
+    if (!m.topo->changed || m.topo->K != 0) return;
+    if (__syncthreads_or((int)t.ringMeet[2])) return;
     const int stage = beside ? 0 : ST_BIO;
     const int M = m.topo->M, C = m.topo->C;
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x;
@@ -750,7 +752,8 @@ __device__ __forceinline__ void block_places(const bool (&flag)[3], int (&place)
 // 49.2 -> 46.8, 1024^2 FP64 178 -> 172 (FP32 111 -> 110).
 __global__ void __launch_bounds__(256, 2) coarsen_compact_kernel(MembraneDev m, TopoDev t, int, Status* st, int) {
     Topo* T = m.topo;
-    if (st->halt || t.ringMeet[2] != 0u) return;
+    // (the block as one: a meeting that fails raises an error here)
+    if (__syncthreads_or(st->halt | (int)t.ringMeet[2])) return;
     if (T->removed == 0) {
         if (blockIdx.x == 0 && threadIdx.x == 0) T->nCand = 0;
         return;
