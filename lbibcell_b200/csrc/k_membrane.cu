@@ -672,8 +672,13 @@ __global__ void __launch_bounds__(kInterpBlock) interp_move_kernel(MembraneDev m
     double2* p = prod[threadIdx.x >> 5];
     const int i = blockIdx.x * kInterpNodes + (int)(threadIdx.x >> 2), ic = min(i, m.Mcap - 1);
     int halt = st->halt, M = m.topo->M;
+    unsigned long long beside = st->beside;
     double X = m.x[ic], Y = m.y[ic], bind = (col < 2 ? m.bx : m.by)[ic];
-    read_ahead(halt, M, X, Y, bind);
+    read_ahead(halt, beside, M, X, Y, bind);
+    if (beside != 0) {  // the streams have joined: an error beside the step before stops the main sequence here
+        if (blockIdx.x == 0 && threadIdx.x == 0) raise_halt(st, ST_INTERP_MOVE);
+        return;
+    }
     if (halt || i - e >= M) return;  // the whole warp
     const bool live = i < M;
     if (!live) X = Y = bind = 32.0;
@@ -910,7 +915,7 @@ __global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, C
     pdl_wait();
     const int cn = blockIdx.x * kCrossBlock + threadIdx.x, cc = min(cn, max(m.Ccap, 1) - 1);
     const bool any = m.Ccap > 0;  // there are buffers to read from
-    int halt = st->halt | st->err, nodes = st->nPerturbNode, C = m.topo->C, a = any ? m.ca[cc] : 0, b = any ? m.cb[cc] : 0;
+    int halt = st->halt, nodes = st->nPerturbNode, C = m.topo->C, a = any ? m.ca[cc] : 0, b = any ? m.cb[cc] : 0;
     uint32_t D = any ? m.cdom[cc] : 0u;
     read_ahead(halt, nodes, C, a, b, D);
     // Other blocks may raise an error meanwhile, between the reads of two warps
@@ -1010,17 +1015,19 @@ __global__ void __launch_bounds__(kCrossBlock) crossings_kernel(MembraneDev m, C
 // (GeometryHandler.cpp:608-644): a node that left its previous unit cell
 // (GeometryNode::isUpdateNeeded, GeometryNode.cpp:256-261, Rectangle.cpp
 // pointWithinBounds) is bound again from its current position, after the
-// edge test; the others keep their binding.
-__device__ __forceinline__ void edge_check_node(const MembraneDev& m, int i, int nx, int ny, Status* st, int stage) {
+// edge test; the others keep their binding.  True if the test raised an error.
+__device__ __forceinline__ bool edge_check_node(const MembraneDev& m, int i, int nx, int ny, Status* st, int stage) {
     const double X = m.x[i], Y = m.y[i], ox = m.ox[i], oy = m.oy[i];
     const bool within = (X >= floor(ox)) && (X < ceil(ox)) && (Y <= ceil(oy)) && (Y > floor(oy));
-    if (within) return;
+    if (within) return false;
     m.bx[i] = X;
     m.by[i] = Y;
     if (X - 2.0 < 0) raise_error(st, ERR_EDGE_W, i, stage);
     else if (Y - 2.0 < 0) raise_error(st, ERR_EDGE_S, i, stage);
     else if (X + 2.0 > nx) raise_error(st, ERR_EDGE_E, i, stage);
     else if (Y + 2.0 > ny) raise_error(st, ERR_EDGE_N, i, stage);
+    else return false;
+    return true;
 }
 
 // Pass 1: among records at the closest distance, the earliest connection.
@@ -1037,7 +1044,7 @@ __global__ void __launch_bounds__(kRemeshBlock) cross_tie_kernel(CrossDev c, Mem
     pdl_wait();
     const int tid = blockIdx.x * kRemeshBlock + threadIdx.x, all = gridDim.x * kRemeshBlock;
     const int rc = min(tid, c.recCap - 1);
-    int halt = st->halt | st->err, conns = st->nPerturbConn, n = st->nCrossRec, M = m.topo->M;
+    int halt = st->halt, conns = st->nPerturbConn, n = st->nCrossRec, M = m.topo->M;
     uint32_t key = c.recKey[rc], conn = c.recConn[rc];
     unsigned long long dist = c.recDist[rc];
     read_ahead(halt, conns, n, M, key, conn, dist);
@@ -1056,7 +1063,8 @@ __global__ void __launch_bounds__(kRemeshBlock) cross_tie_kernel(CrossDev c, Mem
         }
         if (c.bnDist[key] == dist) atomicMin(&c.bnConn[key], conn);
     }
-    for (int i = tid; i < M; i += all) edge_check_node(m, i, nx, ny, st, ST_CROSSINGS);
+    for (int i = tid; i < M; i += all)
+        if (edge_check_node(m, i, nx, ny, st, ST_CROSSINGS)) st->domainStop = 1;
     if (t.flag != nullptr) remesh_count_block(m, t);  // (not at set-up)
 }
 
@@ -1099,11 +1107,11 @@ __device__ __forceinline__ void record_noflux(const MembraneDev& m, CrossDev& c,
 __global__ void cross_win_kernel(CrossDev c, MembraneDev m, const uint32_t* dom, int nx, int ny, Status* st) {
     pdl_wait();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, all = gridDim.x * blockDim.x, rc = min(tid, c.recCap - 1);
-    int go = st->domainGo, n = st->nCrossRec;
+    int go = st->domainGo, stop = st->domainStop, n = st->nCrossRec;
     uint32_t key = c.recKey[rc], conn = c.recConn[rc], bdom = c.recDom[rc];
     unsigned long long dist = c.recDist[rc];
-    read_ahead(go, n, key, conn, bdom, dist);
-    if (!go) return;
+    read_ahead(go, stop, n, key, conn, bdom, dist);
+    if (!go || stop) return;
     n = min(n, c.recCap);
     for (int r = tid; r < n; r += all) {
         if (r != tid) {
@@ -1414,10 +1422,10 @@ __global__ void __launch_bounds__(kReinitBlock) reinit_kernel(CrossDev c, uint32
     pdl_wait();
     const int lane = threadIdx.x & 31, warps = kReinitBlock / 32, warp = threadIdx.x >> 5;
     const int k0 = blockIdx.x * warps + warp;
-    int go = st->domainGo, cnt = st->nChanged, typesCopied = st->cellTypesCopied;
+    int go = st->domainGo, stop = st->domainStop, cnt = st->nChanged, typesCopied = st->cellTypesCopied;
     uint32_t iteration = st->iteration, node0 = c.changedNode[min(k0, c.changedCap - 1)];
-    read_ahead(go, cnt, typesCopied, iteration, node0);
-    if (!go || cnt == 0) return;
+    read_ahead(go, stop, cnt, typesCopied, iteration, node0);
+    if (!go || stop || cnt == 0) return;
     if (cnt > kReinitMax || cnt > c.changedCap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error_beside(st, ERR_CAPACITY, cnt, ST_REINIT);
         return;
@@ -1534,10 +1542,12 @@ __global__ void __launch_bounds__(kFillBlock) domain_fill_kernel(CrossDev c, uin
     const int y = blockIdx.x;
     const size_t row = (size_t)y * nx;
     // everything the block's course depends on, read at once
-    int nrec = st->nCrossRec, go = gated ? st->domainGo : !st->halt, marked = c.rowNow[y] | c.rowHad[y];
+    int nrec = st->nCrossRec, go = gated ? st->domainGo : !st->halt, stop = st->domainStop;
+    int marked = c.rowNow[y] | c.rowHad[y];
     uint32_t left = dom[row];
-    read_ahead(nrec, go, marked, left);
+    read_ahead(nrec, go, stop, marked, left);
     nrec = min(nrec, c.recCap);
+    go = go && !stop;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nrec; k += gridDim.x * blockDim.x) {
         const uint32_t key = c.recKey[k];
         c.bnDist[key] = kEmpty;
@@ -1710,14 +1720,19 @@ void launch_tension_renewal(MembraneDev& m, int* outPos, int* inPos, double forc
 // sum is part of the result).
 constexpr int kAreaMax = 4096;
 
-__global__ void __launch_bounds__(256) areas_kernel(MembraneDev m, double* area, Status* st) {
+// beside: launched beside the main sequence (raise_error_beside), whose step counts
+// if it got to its domain stages.
+__global__ void __launch_bounds__(256) areas_kernel(MembraneDev m, double* area, Status* st, int beside) {
     pdl_wait();
     const int cell = blockIdx.x;
     const int b = m.ringStart[cell], e = m.ringStart[cell + 1];
     const int np = e - b;
     __shared__ double terms[kAreaMax];
     if (np > kAreaMax) {
-        if (threadIdx.x == 0 && st) raise_error_beside(st, ERR_CAPACITY, cell, ST_BIO);
+        if (threadIdx.x == 0 && st) {
+            if (!beside) raise_error(st, ERR_CAPACITY, cell, ST_BIO);
+            else if (st->domainGo && !st->domainStop) raise_error_beside(st, ERR_CAPACITY, cell, ST_BIO);
+        }
         return;
     }
     for (int k = threadIdx.x; k < np; k += blockDim.x) {
@@ -1853,7 +1868,7 @@ __global__ void areas_fixed_kernel(MembraneDev m, const int* cellOfDom, int nDom
 
 void launch_areas(const MembraneDev& m, double* area, Status* st, cudaStream_t s) {
     if (m.nCells == 0) return;
-    launch_pdl(areas_kernel, m.nCells, 256, 0, s, m, area, st);
+    launch_pdl(areas_kernel, m.nCells, 256, 0, s, m, area, st, 0);
 }
 
 // The fixed-point sums as areas (the conversion of area_regulator_kernel),
@@ -1883,11 +1898,11 @@ cudaError_t static_area_scratch(double** ptr) {
 
 void launch_area_regulator(const MembraneDev& m, double* area, double* target, double* massTab, int nDomains,
                            double factor, double strength, double maxsource, const uint32_t* ctypeTab,
-                           const Status* st, cudaStream_t s) {
+                           Status* st, cudaStream_t s, bool beside) {
     if (m.nCells == 0) return;
-    launch_pdl(areas_kernel, m.nCells, 256, 0, s, m, area, (Status*)st);
+    launch_pdl(areas_kernel, m.nCells, 256, 0, s, m, area, st, beside ? 1 : 0);
     launch_pdl(area_regulator_kernel, (m.nCells + 127) / 128, 128, 0, s, m, area, target, massTab, nDomains, factor,
-               strength, maxsource, ctypeTab, (unsigned long long*)nullptr, st);
+               strength, maxsource, ctypeTab, (unsigned long long*)nullptr, (const Status*)st);
 }
 
 void launch_area_regulator_fixed(const MembraneDev& m, const int* cellOfDom, unsigned long long* acc, double* area,

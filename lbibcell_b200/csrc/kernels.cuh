@@ -234,7 +234,7 @@ void launch_tension_renewal(MembraneDev& m, int* outPos, int* inPos, double forc
 // target, cell type 1 at maxsource); nullptr the LbibAreaRegulator rule.
 void launch_area_regulator(const MembraneDev& m, double* area, double* target, double* massTab, int nDomains,
                            double factor, double strength, double maxsource, const uint32_t* ctypeTab,
-                           const Status* st, cudaStream_t s);
+                           Status* st, cudaStream_t s, bool beside = false);
 // st != nullptr: a ring longer than the kernel's limit raises ERR_CAPACITY there.
 void launch_areas(const MembraneDev& m, double* area, Status* st, cudaStream_t s);
 // dL/d of each force record's 4 parameters from the node-force gradient (gfx, gfy).

@@ -1510,7 +1510,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
                 const uint32_t* ct = h.areaTutorial ? h.ctypeTab : nullptr;
                 if (sizeof(Real) == 8) {
                     launch_area_regulator(h.m, h.area, h.target, h.massTab, h.nDomains, h.areaFactor,
-                                          h.areaStrength, h.areaMax, ct, h.st, a);
+                                          h.areaStrength, h.areaMax, ct, h.st, a, a != s);
                     nl += h.m.nCells > 0 ? 2 : 0;
                 } else {
                     launch_area_regulator_fixed(h.m, h.td.cellOfDom, h.areaAcc, h.area, h.target, h.massTab,
@@ -1558,6 +1558,22 @@ static int resume_stage(int stage) {
     }
 }
 
+// The error of a status word as read: the main sequence's own (err, its stage that
+// of the halt) or one raised beside it, whichever the step's order has first.  An
+// error beside belongs to the step before the one in whose move it stopped the main
+// sequence, which by then had run that step's later stages and the next one's forces
+// and spread.  (A step whose own earlier stages fail runs nothing beside them that
+// raises.)
+static void status_error(Status& st) {
+    st.errStage = st.err ? st.haltStage : 0;
+    if (st.beside == 0) return;
+    const int stage = beside_stage(st.beside);
+    if (st.err && stage >= ST_REMESH && st.haltStage >= ST_REMESH) return;
+    st.err = 255 - (int)((st.beside >> 32) & 0xff);
+    st.errIndex = (int)~(unsigned)st.beside;
+    st.errStage = stage;
+}
+
 // Reads the status word and, in the same synchronisation, the device counts:
 // their `changed` flag says whether the ring order of the cell areas is stale
 // (remeshing or coarsening on the device set it; a ring rebuild clears it).
@@ -1566,6 +1582,7 @@ static void read_status(Handle& h) {
     h.statusWithAreas = false;
     CK(cudaMemcpyAsync(h.stHost, h.st, kAreaOffset + areas, cudaMemcpyDeviceToHost, h.stream));
     CK(cudaStreamSynchronize(h.stream));
+    status_error(*h.stHost);
     if (h.m.topo) h.ringsCurrent = h.topoHost->changed == 0;
 }
 
@@ -1966,7 +1983,7 @@ static void run_steps(Handle& h, int n) {
         const Status st = *h.stHost;
         // a step counts as done at the end of its domain stages; one that halted
         // later is not
-        const int stage0 = st.halt ? st.haltStage : (st.err ? st.errStage : 0);
+        const int stage0 = st.err ? st.errStage : (st.halt ? st.haltStage : 0);
         const int done = st.stepsDone - (pad0 < 0 ? 0 : pad0) - (stage0 >= ST_REMESH ? 1 : 0);
         if (!st.halt && !st.err) {
             h.statusContinues = true;

@@ -146,9 +146,11 @@ struct Status {
     unsigned iteration;   // Parameters' current iteration of the step being run
     int cellTypesCopied;  // copyCellTypeToPhysicalNodes has run (after the first step)
     int stepsDone;     // steps whose domain stage is through (end_step)
-    int errStage;      // stage of an error raised beside the main sequence (raise_error_beside)
+    int errStage;      // the error's stage (host: status_error)
     int nCrossRec;     // crossing records of the step
-    int domainGo;      // this step's domain stages (winners, re-initialisation, fill) run
+    int domainGo;      // this step's domain stages (winners, re-initialisation, fill) run, unless
+    int domainStop;    // a moved node was too near the edge
+    unsigned long long beside;  // error raised beside the main sequence (raise_error_beside; 0: none)
 };
 
 // Stage numbers (halt points), in the reference's order of
@@ -194,23 +196,28 @@ __device__ __forceinline__ void raise_error(Status* st, int code, int index, int
 
 // An error of a stage that runs beside the main sequence (the domain stages, the
 // cell areas): the main sequence must not see a halt that its own kernels did not
-// wait for.  The next step's crossings stop on the error word.
+// wait for.  The next step's move, which comes after the streams have joined, stops
+// on it.  Of several errors the one of the earliest stage stays, of one stage that
+// of the smallest code and index (the word's largest value): the word does not
+// depend on the streams' timing.
 __device__ __forceinline__ void raise_error_beside(Status* st, int code, int index, int stage) {
-    if (atomicCAS(&st->err, 0, code) == 0) st->errIndex = index;
-    atomicCAS(&st->errStage, 0, stage);
+    atomicMax(&st->beside, ((unsigned long long)(255 - stage) << 40) | ((unsigned long long)(255 - code) << 32) |
+                               (unsigned)~index);
 }
+__host__ __device__ __forceinline__ int beside_stage(unsigned long long word) { return 255 - (int)(word >> 40); }
 
 // The end of a step's domain stages, run by one thread once all their blocks are
 // through: the step counts as done (Parameters++, SimulationRunner.cpp:98; the host
 // takes it back when a later stage of the step halts), copyCellTypeToPhysicalNodes
-// has run, and the counters are clear for the next crossings.  An error of the step's
-// later stages, which may be running beside, doesn't change the count.
+// has run, and the counters are clear for the next crossings.  Only an error of the
+// domain stages themselves keeps a step that ran them from counting: those of the
+// step's later stages and of the next step's forces and spread, which may be
+// running beside, do not.
 __device__ __forceinline__ void end_step(Status* st, bool ran) {
-    int err = st->err, errStage = st->errStage, haltStage = st->haltStage, done = st->stepsDone;
-    int iteration = (int)st->iteration;
-    read_ahead(err, errStage, haltStage, done, iteration);
-    const int stage = errStage ? errStage : haltStage;
-    if (ran && (err == 0 || stage == 0 || stage >= ST_REMESH)) {
+    unsigned long long beside = st->beside;
+    int done = st->stepsDone, iteration = (int)st->iteration;
+    read_ahead(beside, done, iteration);
+    if (ran && (beside == 0 || beside_stage(beside) >= ST_REMESH)) {
         st->stepsDone = done + 1;
         st->iteration = (unsigned)iteration + 1u;
         st->cellTypesCopied = 1;

@@ -21,9 +21,11 @@ void launch_clear_forces(MembraneDev&, cudaStream_t, const Status*) {}
 using namespace lbib;
 
 // One launch of one block over a membrane without nodes; `missing`: arrivals
-// that it waits for in vain.  out: err, errStage, halt, haltStage, changed,
-// removed, a wait ran out, ringStart[0]; then err and `changed` after a second
-// launch whose status word is clear.
+// that it waits for in vain.  out: the error and, if it was raised beside the main
+// sequence, its stage, halt, haltStage, changed, removed, a wait ran out,
+// ringStart[0]; then the error and `changed` after a second launch whose status
+// word is clear.
+static int error_of(const Status& s) { return s.beside ? 255 - (int)((s.beside >> 32) & 255) : s.err; }
 extern "C" int meet(int compaction, int beside, unsigned missing, int* out) {
     const int n = 64;
     int* a;
@@ -62,12 +64,12 @@ extern "C" int meet(int compaction, int beside, unsigned missing, int* out) {
         if (launch == 1) break;
         cudaMemcpy(meetings, t.ringMeet, sizeof meetings, cudaMemcpyDeviceToHost);
         cudaMemcpy(&five, m.ringStart, sizeof five, cudaMemcpyDeviceToHost);
-        const int got[8] = {s.err, s.errStage, s.halt, s.haltStage, tp.changed, tp.removed, (int)meetings[2], five};
+        const int got[8] = {error_of(s), s.beside ? beside_stage(s.beside) : 0, s.halt, s.haltStage, tp.changed, tp.removed, (int)meetings[2], five};
         std::memcpy(out, got, sizeof got);
         std::memset(&s, 0, sizeof s);
         cudaMemcpy(st, &s, sizeof s, cudaMemcpyHostToDevice);
     }
-    out[8] = s.err;
+    out[8] = error_of(s);
     out[9] = tp.changed;
     cudaFree(a);
     return 0;
