@@ -574,14 +574,14 @@ void launch_stream_collide32(const LatticeArgs<float>& args, cudaStream_t s) {
     if ((mode == 0 || mode == 2) && a.nx % 256 == 0 && x4 && x4[0] == '1') {
         const dim3 grid4((unsigned)(a.nx / 256), (unsigned)a.ny);
         switch (mode * 4 + (a.S < 3 ? a.S : 3)) {
-            case 0: launch_pdl(stream_collide32x4<0, 0>, grid4, 64, 0, s, a); break;
-            case 1: launch_pdl(stream_collide32x4<1, 0>, grid4, 64, 0, s, a); break;
-            case 2: launch_pdl(stream_collide32x4<2, 0>, grid4, 64, 0, s, a); break;
-            case 3: launch_pdl(stream_collide32x4<3, 0>, grid4, 64, 0, s, a); break;
-            case 8: launch_pdl(stream_collide32x4<0, 2>, grid4, 64, 0, s, a); break;
-            case 9: launch_pdl(stream_collide32x4<1, 2>, grid4, 64, 0, s, a); break;
-            case 10: launch_pdl(stream_collide32x4<2, 2>, grid4, 64, 0, s, a); break;
-            default: launch_pdl(stream_collide32x4<3, 2>, grid4, 64, 0, s, a); break;
+            case 0: launch_ex(!a.joined, stream_collide32x4<0, 0>, grid4, 64, 0, s, a); break;
+            case 1: launch_ex(!a.joined, stream_collide32x4<1, 0>, grid4, 64, 0, s, a); break;
+            case 2: launch_ex(!a.joined, stream_collide32x4<2, 0>, grid4, 64, 0, s, a); break;
+            case 3: launch_ex(!a.joined, stream_collide32x4<3, 0>, grid4, 64, 0, s, a); break;
+            case 8: launch_ex(!a.joined, stream_collide32x4<0, 2>, grid4, 64, 0, s, a); break;
+            case 9: launch_ex(!a.joined, stream_collide32x4<1, 2>, grid4, 64, 0, s, a); break;
+            case 10: launch_ex(!a.joined, stream_collide32x4<2, 2>, grid4, 64, 0, s, a); break;
+            default: launch_ex(!a.joined, stream_collide32x4<3, 2>, grid4, 64, 0, s, a); break;
         }
         return;
     }
