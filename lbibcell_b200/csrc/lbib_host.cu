@@ -138,6 +138,7 @@ struct DiffCtx {
     int rs = 8;               // bytes of a stored value: 8 (FP64) or 4 (FP32-shifted)
     char* x0 = nullptr;       // state at step 0
     char* u0 = nullptr;       // velocity and force planes at step 0 (restored by lbib_diff_end), 4*L values
+    int* active0 = nullptr;   // the tiles whose force those planes hold (TileDev::active, restored with them)
     char* ck = nullptr;       // states at steps K, 2K, ... (nSeg - 1 of them)
     char* seg = nullptr;      // states base+1 .. base+K-1 of the segment being reversed
     // A second segment buffer for FP32 states, when the device has room for
@@ -199,7 +200,7 @@ struct DiffCtx {
     char* state(int i) const { return i == 0 ? x0 : ck + (size_t)(i - 1) * stateBytes; }
     ~DiffCtx() {
         auto fr = [](void* p) { if (p) cudaFree(p); };
-        fr(x0); fr(u0); fr(ck); fr(seg); fr(fin); fr(P[0]); fr(P[1]); fr(G); fr(force); fr(force32); fr(fxp);
+        fr(x0); fr(u0); fr(active0); fr(ck); fr(seg); fr(fin); fr(P[0]); fr(P[1]); fr(G); fr(force); fr(force32); fr(fxp);
         fr(fyp); fr(gfx); fr(gfy);
         fr(srcTab); fr(seed); fr(grad); fr(racc); fr(part); fr(st); fr(massTab); fr(macc); fr(seedF); fr(seg2);
         fr(pos); fr(lam); fr(seedX); fr(uo);
@@ -2433,6 +2434,7 @@ static void diff_begin(Handle& h, int T, int K) {
     d->T = T; d->K = K; d->nSeg = nSeg; d->stateBytes = stateBytes; d->rs = rs;
     d->x0 = dalloc<char>(stateBytes);
     d->u0 = dalloc<char>(4 * L * rs);
+    d->active0 = dalloc<int>(h.tiles.nTiles);
     d->ck = dalloc<char>((size_t)(nSeg - 1) * stateBytes);
     d->seg = dalloc<char>((size_t)(K - 1) * stateBytes);
     d->fin = dalloc<char>(stateBytes);
@@ -2484,6 +2486,7 @@ static void diff_begin(Handle& h, int T, int K) {
     if (S) CK(cudaMemcpyAsync(d->x0 + 9 * L * rs, h.g[h.cur], 5 * S * L * rs, cudaMemcpyDeviceToDevice, h.stream));
     CK(cudaMemcpyAsync(d->u0, h.u, 2 * L * rs, cudaMemcpyDeviceToDevice, h.stream));
     CK(cudaMemcpyAsync(d->u0 + 2 * L * rs, h.force, 2 * L * rs, cudaMemcpyDeviceToDevice, h.stream));
+    CK(cudaMemcpyAsync(d->active0, h.tiles.active, sizeof(int) * h.tiles.nTiles, cudaMemcpyDeviceToDevice, h.stream));
     if (S) CK(cudaMemcpyAsync(d->srcTab, h.srcTab, sizeof(double) * S * h.nDomains, cudaMemcpyDeviceToDevice, h.stream));
     if (h.m.M) {
         CK(cudaMemcpyAsync(d->fxp, h.m.fx, sizeof(double) * h.m.M, cudaMemcpyDeviceToDevice, h.stream));
@@ -3510,6 +3513,7 @@ int lbib_diff_end(lbib_handle* hh) {
             CK(cudaMemcpyAsync(h.g[h.cur], d.x0 + 9 * L * rs, 5 * h.S * L * rs, cudaMemcpyDeviceToDevice, h.stream));
         CK(cudaMemcpyAsync(h.u, d.u0, 2 * L * rs, cudaMemcpyDeviceToDevice, h.stream));
         CK(cudaMemcpyAsync(h.force, d.u0 + 2 * L * rs, 2 * L * rs, cudaMemcpyDeviceToDevice, h.stream));
+        CK(cudaMemcpyAsync(h.tiles.active, d.active0, sizeof(int) * h.tiles.nTiles, cudaMemcpyDeviceToDevice, h.stream));
         CK(cudaStreamSynchronize(h.stream));
         delete h.diff;
         h.diff = nullptr;
