@@ -2580,6 +2580,10 @@ static void diff_forward(Handle& h, DiffCtx& d) {
         launch_spread<double>(mp, h.tiles, d.force, h.nx, h.ny, L, d.st, d.it0, h.stream);
         if (d.rs == 4) launch_to_float(d.force, d.force32, 2 * L, h.stream);
     } else {
+        // the nodes may go anywhere: the forward's lattice kernels read the whole
+        // field (zero where no stencil is), as the reverse step does, and so does
+        // a read-out of it afterwards
+        CK(cudaMemsetAsync(h.tiles.active, 1, sizeof(int) * h.tiles.nTiles, h.stream));
         diff_motion_begin(h, d, 1, h.stream);
     }
     // two scratch states for the steps between checkpoints (the segment
