@@ -7,9 +7,11 @@
  * these calls.  All calls return 0 or an LBIB_ERR_* code and never throw or
  * abort across the ABI; lbib_last_error() gives the message and the index of
  * the node or connection involved.  The caller owns every host buffer; the
- * handle owns every device buffer.  A handle uses one CUDA stream and is not
- * thread-safe; the calls that copy large states to the host use further
- * streams and threads of their own, which end with the call.
+ * handle owns every device buffer.  A handle is not thread-safe.  Its work is
+ * ordered on one CUDA stream of its own; within a step graph, and within the
+ * reverse pass of a differentiated run, parts run on further streams of the
+ * handle that join that one, and the calls that copy large states to the host
+ * use streams and threads whose work ends with the call.
  *
  * The comment of each call names the reference interface it replaces (paths
  * relative to the LBIBCell project root).

@@ -519,8 +519,10 @@ __global__ void __launch_bounds__(256) spread_kernel(MembraneDev m, TileDev t, R
 // the ordered gather and rounded once; the integer sums are exact, so the
 // field does not depend on the order of the list (it is deterministic) and no
 // sort is needed.  The rounding is far below FP32 resolution.
-// Bound by instruction issue where tiles hold many nodes, by the chain of reads
-// where there is one cell.  Two lanes form a node's factors, one per axis, the
+// Where tiles hold many nodes, the barriers between the staging of a chunk's
+// factors and its scatter are the first stall and the scheduler issues in 44 % of
+// the cycles (tiles are filled unevenly); where there is one cell, the chain of
+// reads bounds it.  Two lanes form a node's factors, one per axis, the
 // force is staged with the products' power of two (an exact scaling), and the
 // usual 4 x 4 stencil has its own loop: 150k nodes on 1024^2 21.6 -> 19.0 us, one
 // cell on 200^2 4.5 -> 3.9 us against a lane per node and one loop.  Blocks of 64
@@ -615,7 +617,7 @@ __global__ void __launch_bounds__(256) spread_fixed_kernel(MembraneDev m, TileDe
 
 template <typename Real>
 void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny, size_t L, Status* st,
-                   unsigned iteration, cudaStream_t s, bool slotsFilled) {
+                   cudaStream_t s, bool slotsFilled) {
     if (m.Mcap == 0) {
         cudaMemsetAsync(t.active, 0, sizeof(int) * t.nTiles, s);
         return;
@@ -628,9 +630,9 @@ void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny
     else
         launch_pdl(spread_kernel<Real>, t.nTiles, 256, 0, s, m, t, force, nx, ny, L, st);
 }
-template void launch_spread<double>(const MembraneDev&, TileDev&, double*, int, int, size_t, Status*, unsigned,
+template void launch_spread<double>(const MembraneDev&, TileDev&, double*, int, int, size_t, Status*,
                                     cudaStream_t, bool);
-template void launch_spread<float>(const MembraneDev&, TileDev&, float*, int, int, size_t, Status*, unsigned,
+template void launch_spread<float>(const MembraneDev&, TileDev&, float*, int, int, size_t, Status*,
                                    cudaStream_t, bool);
 
 // ---------------------------------------------------------------------------
@@ -664,8 +666,7 @@ __device__ __forceinline__ int interp_place(int slot, int e) { return slot * 8 +
 
 template <typename Real>
 __global__ void __launch_bounds__(kInterpBlock) interp_move_kernel(MembraneDev m, const Real* u, int nx, int ny,
-                                                                   size_t L, CrossDev c, Status* st,
-                                                                   unsigned iteration) {
+                                                                   size_t L, CrossDev c, Status* st) {
     pdl_wait();
     __shared__ double2 prod[kInterpBlock / 32][16 * 8];
     const int lane = threadIdx.x & 31, col = lane & 3, e = lane >> 2;
@@ -761,15 +762,15 @@ __global__ void __launch_bounds__(kInterpBlock) interp_move_kernel(MembraneDev m
 
 template <typename Real>
 void launch_interp_move(const MembraneDev& m, const Real* u, int nx, int ny, size_t L, CrossDev& c, Status* st,
-                        unsigned iteration, cudaStream_t s) {
+                        cudaStream_t s) {
     if (m.Mcap == 0) return;
     launch_pdl(interp_move_kernel<Real>, (m.Mcap + kInterpNodes - 1) / kInterpNodes, kInterpBlock, 0, s, m, u, nx, ny, L,
-               c, st, iteration);
+               c, st);
 }
 template void launch_interp_move<double>(const MembraneDev&, const double*, int, int, size_t, CrossDev&, Status*,
-                                         unsigned, cudaStream_t);
+                                         cudaStream_t);
 template void launch_interp_move<float>(const MembraneDev&, const float*, int, int, size_t, CrossDev&, Status*,
-                                        unsigned, cudaStream_t);
+                                        cudaStream_t);
 
 // Adjoint of the spread for a differentiated run with frozen positions.  The
 // spread adds dirac(x - X_i) * F_i to every lattice node x of node i's stencil
@@ -853,8 +854,7 @@ __device__ __forceinline__ bool make_record(int nx, int ny, int px, int py, int 
 // Calls fn(k, record) for the candidate records of connection cn in a fixed
 // order (k = 0, 1, ...); returns the number of records, or -1 after raising
 // the error of a connection that cannot be processed.  The kernel enumerates
-// three times (count, emit, list first writers) so that no per-thread record
-// array is needed.
+// twice (count, emit) so that no per-thread record array is needed.
 template <class Fn>
 __device__ __forceinline__ int for_each_record(const MembraneDev& m, int cn, int nx, int ny, Status* st, bool report,
                                                Fn fn) {
@@ -1205,7 +1205,7 @@ void launch_crossings(const MembraneDev& m, CrossDev& c, int nx, int ny, Status*
     if (c.nfTab != nullptr) launch_pdl(noflux_reset_kernel, 1, 1024, 0, s, c, st);
     if (c.bounceW != nullptr) launch_pdl(bounce_reset_kernel, 1, 1024, 0, s, c, st);
     // the record count (st->nCrossRec) is zero here: cleared with the status
-    // word before a run and by the first kernel of each step
+    // word before a run and at the end of each step's domain fill (end_step)
     launch_pdl(crossings_kernel, blocks, kCrossBlock, 0, s, m, c, nx, ny, st, check ? 1 : 0, perturb, perturbCap);
     // grid-stride over the step's records (their count is known on the device
     // only): up to 8 blocks per SM, so that each thread's chain of dependent
@@ -1223,7 +1223,7 @@ void launch_cross_winners(const MembraneDev& m, CrossDev& c, const uint32_t* dom
               st);
 }
 
-void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s) {
+void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, cudaStream_t s) {
     if (m.Mcap == 0) return;
     launch_pdl(edge_check_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, nx, ny, st, ST_REMESH);
 }
@@ -1502,19 +1502,17 @@ __global__ void __launch_bounds__(kReinitBlock) reinit_kernel(CrossDev c, uint32
 
 template <typename Real>
 void launch_reinit(CrossDev& c, uint32_t* dom, Real* g, const Real* u, int nS, const SpeciesConst* sp,
-                   const double* srcTab, int nDomains, const uint32_t* ctypeTab, int cellTypesCopied, int nx, int ny,
-                   size_t L, Status* st, unsigned iteration, cudaStream_t s) {
+                   const double* srcTab, int nDomains, const uint32_t* ctypeTab, int nx, int ny, size_t L, Status* st,
+                   cudaStream_t s) {
     if (c.changedCap <= 0) return;
     const SpeciesSet species{{sp[0], sp[1], sp[2]}};
     launch_pdl(reinit_kernel<Real>, 148, kReinitBlock, 0, s, c, dom, g, u, nS, species, srcTab, nDomains, ctypeTab, nx,
                ny, L, st);
 }
 template void launch_reinit<double>(CrossDev&, uint32_t*, double*, const double*, int, const SpeciesConst*,
-                                    const double*, int, const uint32_t*, int, int, int, size_t, Status*, unsigned,
-                                    cudaStream_t);
+                                    const double*, int, const uint32_t*, int, int, size_t, Status*, cudaStream_t);
 template void launch_reinit<float>(CrossDev&, uint32_t*, float*, const float*, int, const SpeciesConst*,
-                                   const double*, int, const uint32_t*, int, int, int, size_t, Status*, unsigned,
-                                   cudaStream_t);
+                                   const double*, int, const uint32_t*, int, int, size_t, Status*, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // Domain fill: one block per row; the row's domain id at x >= 1 is the domain
@@ -1630,36 +1628,7 @@ void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, Status* st, 
 
 
 // ---------------------------------------------------------------------------
-// Topology checks
-
-__global__ void remesh_check_kernel(Status* st) {
-    pdl_wait();
-    if (st->halt) return;
-    if (st->remesh) raise_halt(st, ST_REMESH);
-}
-
-void launch_remesh_check(Status* st, unsigned iteration, cudaStream_t s) { launch_pdl(remesh_check_kernel, 1, 1, 0, s, st); }
-
-// GeometryHandler::coarsenBoundary's test (GeometryHandler.cpp:444-449): the
-// span from the previous node to the next node is below MAXLENGTH.
-__global__ void coarsen_check_kernel(MembraneDev m, Status* st) {
-    pdl_wait();
-    if (st->halt) return;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.topo->M) return;
-    const int p = m.prev[i], q = m.next[i];
-    const double dx = m.x[q] - m.x[p], dy = m.y[q] - m.y[p];
-    const double length = sqrt(dx * dx + dy * dy);
-    if (length < kMAXLENGTH) {
-        st->coarsen = 1;
-        raise_halt(st, ST_COARSEN);
-    }
-}
-
-void launch_coarsen_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s) {
-    if (m.Mcap == 0) return;
-    launch_pdl(coarsen_check_kernel, (m.Mcap + 127) / 128, 128, 0, s, m, st);
-}
+// Force list
 
 // st: a step's stage, which a halted step skips (else nullptr).
 __global__ void clear_forces_kernel(MembraneDev m, const Status* st) {

@@ -1,17 +1,17 @@
 // k_topology.cu — membrane topology edits on the device.
 //
 //   remesh    GeometryHandler::remeshBoundary (GeometryHandler.cpp:385-431) as
-//             count + scatter (block counts and their prefix in one kernel):
+//             count (with the crossings' ties, remesh.cuh), apply and commit:
 //             every connection longer than MAXLENGTH gets a new node at its
 //             midpoint; the new node ids continue from the largest id in
 //             connection order (Geometry::addGeometryNode,
 //             Geometry.cpp:382-400); the split connection leaves the vector and
 //             its two halves are appended (Geometry::eraseConnection /
-//             addConnection, Geometry.cpp:433-452).  Up to two passes run on
-//             the device (SimulationRunner.cpp:190-199 repeats until nothing is
-//             split); a third pass that would still split, a new node that
-//             needs the random perturbation, or a full buffer hands the step to
-//             the host.
+//             addConnection, Geometry.cpp:433-452).  One pass runs on the
+//             device (SimulationRunner.cpp:190-199 repeats until nothing is
+//             split); a second that would still split, or a full buffer, hands
+//             the step to the host; a new node that needs the random
+//             perturbation waits for it before the commit.
 //   coarsen   GeometryHandler::coarsenBoundary (GeometryHandler.cpp:433-461):
 //             nodes are visited in id order and removed when their neighbours
 //             are closer than MAXLENGTH; a removal erases the node's two
@@ -83,7 +83,7 @@ __device__ __forceinline__ void agg_min(int* addr, int key, int v) {
 
 // The pass was counted with the crossings' ties (remesh_count_block): K
 // connections to split.  It runs unless it would overflow a buffer (the host
-// runs it then; so it does a third pass, remesh_commit_kernel).  New nodes that
+// runs it then; so it does a second pass, remesh_commit_kernel).  New nodes that
 // need the random perturbation are made on the device all the same and listed
 // for the host, which perturbs them before the pass is committed.
 __device__ __forceinline__ bool remesh_fits(const MembraneDev& m, int K, int M, int C) {

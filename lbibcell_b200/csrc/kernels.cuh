@@ -157,7 +157,6 @@ struct TopoDev {
     int* members;       // Mcap
     int* succ; int* dist;                                 // Mcap
     int* rngList;       // Mcap: new nodes of a remesh pass that need the host's random perturbation
-    int* startNode;     // nCells
     unsigned* ringMeet; // ring_barrier: [0] arrivals, ever; [1] those of the launches that are through; [2] a wait ran out
     int nDomains;
 };
@@ -185,10 +184,10 @@ void launch_force_eval(const MembraneDev& m, Status* st, cudaStream_t s, TileDev
                        int ny = 0);
 template <typename Real>
 void launch_spread(const MembraneDev& m, TileDev& t, Real* force, int nx, int ny, size_t L, Status* st,
-                   unsigned iteration, cudaStream_t s, bool slotsFilled = false);
+                   cudaStream_t s, bool slotsFilled = false);
 template <typename Real>
 void launch_interp_move(const MembraneDev& m, const Real* u, int nx, int ny, size_t L, CrossDev& c, Status* st,
-                        unsigned iteration, cudaStream_t s);
+                        cudaStream_t s);
 // The crossings and their ties, and (remesh != nullptr) the count of the step's
 // remeshing pass.  `check`: first raise the halts of the move's listed nodes and of
 // connections that need the host's perturbation (listed in perturb[0..perturbCap)).
@@ -201,12 +200,10 @@ void launch_cross_winners(const MembraneDev& m, CrossDev& c, const uint32_t* dom
                           cudaStream_t s, bool programmatic);
 template <typename Real>
 void launch_reinit(CrossDev& c, uint32_t* dom, Real* g, const Real* u, int nS, const SpeciesConst* sp,
-                   const double* srcTab, int nDomains, const uint32_t* ctypeTab, int cellTypesCopied, int nx,
-                   int ny, size_t L, Status* st, unsigned iteration, cudaStream_t s);
+                   const double* srcTab, int nDomains, const uint32_t* ctypeTab, int nx, int ny, size_t L, Status* st,
+                   cudaStream_t s);
 void launch_domain_fill(CrossDev& c, uint32_t* dom, int nx, int ny, Status* st, cudaStream_t s, bool gated);
-void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, unsigned iteration, cudaStream_t s);
-void launch_remesh_check(Status* st, unsigned iteration, cudaStream_t s);
-void launch_coarsen_check(const MembraneDev& m, Status* st, unsigned iteration, cudaStream_t s);
+void launch_edge_check(const MembraneDev& m, int nx, int ny, Status* st, cudaStream_t s);
 void launch_clear_forces(MembraneDev& m, cudaStream_t s, const Status* st = nullptr);
 // ForceSolver::deleteForceType(6) + the membrane-tension records, on a list that
 // holds other forces too (launches returned).

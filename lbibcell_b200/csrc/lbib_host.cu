@@ -398,9 +398,9 @@ struct Handle {
     bool workAfterEvB = false;  // GPU work was issued after the step loop's last timing event
     // the device status word carries on from the last batch of steps (no
     // halt, nothing wrote it since): the next batch needs no reset; the steps
-    // done until then were lastPad0
+    // done until then were lastStepsDone
     bool statusContinues = false;
-    int lastPad0 = 0;
+    int lastStepsDone = 0;
     cudaStream_t stream = nullptr;
     cudaStream_t side = nullptr, sums = nullptr;  // captured into the step graphs (StepFork), made with the first
     cudaEvent_t evForked = nullptr, evCommitted = nullptr, evJoined = nullptr, evSummed = nullptr;
@@ -477,7 +477,7 @@ Handle::~Handle() {
     fr(td.dalt); fr(td.id2); fr(td.prev2); fr(td.next2); fr(td.inConn); fr(td.outConn); fr(td.removed);
     fr(td.connAlive); fr(td.ncA); fr(td.ncB); fr(td.ncDom); fr(td.ncDesc); fr(td.ncAlive); fr(td.cellOfDom);
     fr(td.firstConn); fr(td.cellCount); fr(td.cellStart); fr(td.cellFill); fr(td.members); fr(td.succ); fr(td.rngList);
-    fr(td.dist); fr(td.startNode); fr(td.ringMeet);
+    fr(td.dist); fr(td.ringMeet);
     fr(st);
     if (stHost) cudaFreeHost(stHost);  // topoHost lives in the same block
     if (evA) cudaEventDestroy(evA);
@@ -1229,14 +1229,14 @@ static void ensure_capacity(Handle& h, int M, int C, int F, int cells) {
     if (grow(cells, h.cellCap)) {
         auto fr = [](void* p) { if (p) cudaFree(p); };
         fr(h.m.ringStart); fr(h.m.ringDom); fr(h.target); fr(h.areaAcc);
-        fr(h.td.cellCount); fr(h.td.cellStart); fr(h.td.cellFill); fr(h.td.startNode);
+        fr(h.td.cellCount); fr(h.td.cellStart); fr(h.td.cellFill);
         h.m.ringStart = dalloc<int>(h.cellCap + 1); h.m.ringDom = dalloc<uint32_t>(h.cellCap);
         resize_status_block(h);
         h.target = dalloc<double>(h.cellCap);
         h.areaAcc = dalloc<unsigned long long>(h.cellCap);
         CK(cudaMemset(h.areaAcc, 0, sizeof(unsigned long long) * h.cellCap));
         h.td.cellCount = dalloc<int>(h.cellCap + 1); h.td.cellStart = dalloc<int>(h.cellCap + 1);
-        h.td.cellFill = dalloc<int>(h.cellCap); h.td.startNode = dalloc<int>(h.cellCap);
+        h.td.cellFill = dalloc<int>(h.cellCap);
     }
     ensure_force_scratch(h);
     h.m.Mcap = h.Mcap;
@@ -1349,7 +1349,7 @@ static bool remesh(Handle& h, HostMembrane& hm) {
 // Stage launcher
 
 template <typename Real>
-static LatticeArgs<Real> lattice_args(Handle& h, unsigned iteration, int parity) {
+static LatticeArgs<Real> lattice_args(Handle& h, int parity) {
     LatticeArgs<Real> a{};
     a.nx = h.nx; a.ny = h.ny; a.L = h.L; a.S = h.S;
     a.fin = (const Real*)h.f[parity];
@@ -1423,7 +1423,7 @@ static long long launch_front(Handle& h, int fromStage) {
     }
     if (fromStage <= ST_SPREAD) {
         const bool filled = hasM && fromStage <= ST_FORCE;
-        launch_spread<Real>(h.m, h.tiles, (Real*)h.force, h.nx, h.ny, h.L, h.st, 0, s, filled);
+        launch_spread<Real>(h.m, h.tiles, (Real*)h.force, h.nx, h.ny, h.L, h.st, s, filled);
         nl += hasM ? (filled ? 1 : 2) : 0;
     }
     return nl;
@@ -1439,17 +1439,16 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
     cudaStream_t s = h.stream;
     Real* gcur = (Real*)h.g[1 - parity];
     const bool hasM = h.m.Mcap > 0;
-    const unsigned it = 0;  // kernels read the iteration from the status word
     long long nl = 0;
     if (fork == nullptr || fork->first) nl += launch_front<Real>(h, fromStage);
     if (fromStage <= ST_COLLIDE) {
         if (evCollideA) cudaEventRecord(evCollideA, s);
         if (sizeof(Real) == 8) {
-            LatticeArgs<double> a = lattice_args<double>(h, it, parity);
+            LatticeArgs<double> a = lattice_args<double>(h, parity);
             a.joined = fork != nullptr && !fork->first;
             launch_stream_collide64(a, s);
         } else {
-            LatticeArgs<float> a = lattice_args<float>(h, it, parity);
+            LatticeArgs<float> a = lattice_args<float>(h, parity);
             a.joined = fork != nullptr && !fork->first;
             launch_stream_collide32(a, s);
         }
@@ -1457,7 +1456,7 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
         nl += 1 + (h.cross.nfTab != nullptr ? 2 : 0);
     }
     if (fromStage <= ST_INTERP_MOVE) {
-        launch_interp_move<Real>(h.m, (const Real*)h.u, h.nx, h.ny, h.L, h.cross, h.st, it, s);
+        launch_interp_move<Real>(h.m, (const Real*)h.u, h.nx, h.ny, h.L, h.cross, h.st, s);
         nl += hasM;
     }
     cudaStream_t d = s, a = s;  // the streams of the domain stages and of the cell areas
@@ -1475,8 +1474,8 @@ static long long launch_stages(Handle& h, bool coarsenStep, int bioOps, int pari
     if (fromStage <= ST_REINIT) {
         SpeciesConst spc[kMaxSpecies] = {};
         for (int k = 0; k < h.S; ++k) spc[k] = h.sp[k].c;
-        launch_reinit<Real>(h.cross, h.dom, gcur, (const Real*)h.u, h.S, spc, h.srcTab, h.nDomains, h.ctypeTab, 0,
-                            h.nx, h.ny, h.L, h.st, it, d);
+        launch_reinit<Real>(h.cross, h.dom, gcur, (const Real*)h.u, h.S, spc, h.srcTab, h.nDomains, h.ctypeTab,
+                            h.nx, h.ny, h.L, h.st, d);
         nl += 1;
     }
     if (fromStage <= ST_DOMAIN) {
@@ -1854,7 +1853,7 @@ static bool handle_halt(Handle& h, int stage) {
         }
         // new nodes are bound to the lattice now (GeometryHandler.cpp:427-428)
         reset_status(h, h.iteration, true);
-        launch_edge_check(h.m, h.nx, h.ny, h.st, 0, h.stream);
+        launch_edge_check(h.m, h.nx, h.ny, h.st, h.stream);
         read_status(h);
         if (h.stHost->err) fail(h.stHost->err, "geometry point moved too close to the boundary", h.stHost->errIndex);
     } else {
@@ -1953,9 +1952,9 @@ static void run_steps(Handle& h, int n) {
         }
         // a status word that carries on from the last batch needs no reset
         // (one host-to-device copy less per call); its count of steps done starts
-        // at lastPad0
-        int pad0 = -1;
-        if (h.statusContinues) pad0 = h.lastPad0;
+        // at lastStepsDone
+        int doneBefore = 0;
+        if (h.statusContinues) doneBefore = h.lastStepsDone;
         else reset_status(h, h.iteration, h.cellTypesCopied);
         const bool prof = h.profiling;
         while ((int)h.kEvents.size() < 2 * B) {
@@ -1985,10 +1984,10 @@ static void run_steps(Handle& h, int n) {
         // a step counts as done at the end of its domain stages; one that halted
         // later is not
         const int stage0 = st.err ? st.errStage : (st.halt ? st.haltStage : 0);
-        const int done = st.stepsDone - (pad0 < 0 ? 0 : pad0) - (stage0 >= ST_REMESH ? 1 : 0);
+        const int done = st.stepsDone - doneBefore - (stage0 >= ST_REMESH ? 1 : 0);
         if (!st.halt && !st.err) {
             h.statusContinues = true;
-            h.lastPad0 = st.stepsDone;
+            h.lastStepsDone = st.stepsDone;
         }
         if (prof) {
             for (int b = 0; b < std::min(done, B); ++b) {
@@ -2393,7 +2392,7 @@ static void cure_lattice(Handle& h, HostMembrane& hm) {
     CK(cudaMemcpyAsync(h.m.y, hm.y.data(), sizeof(double) * hm.y.size(), cudaMemcpyHostToDevice, h.stream));
     std::memset(h.stHost, 0, sizeof(Status));
     write_status(h);
-    launch_edge_check(h.m, h.nx, h.ny, h.st, 0, h.stream);
+    launch_edge_check(h.m, h.nx, h.ny, h.st, h.stream);
     launch_crossings(h.m, h.cross, h.nx, h.ny, h.st, nullptr, h.stream);
     launch_cross_winners(h.m, h.cross, h.dom, h.nx, h.ny, h.st, h.stream, true);
     launch_domain_fill(h.cross, h.dom, h.nx, h.ny, h.st, h.stream, h.m.Ccap > 0);
@@ -2510,9 +2509,8 @@ static bool diff_needs_iteration(const Handle& h) {
 // `out`, in the handle's lattice precision.
 template <typename Real>
 static void diff_forward_step_t(Handle& h, DiffCtx& d, const char* in, char* out, int t, cudaStream_t stream) {
-    const unsigned it = d.it0 + (unsigned)(t - 1);
-    if (diff_needs_iteration(h)) launch_set_iteration(d.st, it, stream);
-    LatticeArgs<Real> a = lattice_args<Real>(h, it, h.cur);
+    if (diff_needs_iteration(h)) launch_set_iteration(d.st, d.it0 + (unsigned)(t - 1), stream);
+    LatticeArgs<Real> a = lattice_args<Real>(h, h.cur);
     a.fin = (const Real*)in; a.fout = (Real*)out;
     a.gin = (const Real*)in + 9 * h.L; a.gout = (Real*)out + 9 * h.L;
     a.force = sizeof(Real) == 8 ? (const Real*)d.forceOf(t) : (const Real*)d.force32;
@@ -2577,7 +2575,7 @@ static void diff_forward(Handle& h, DiffCtx& d) {
     if (!d.motion) {
         // after a moving-node pass the field holds values outside the force tiles
         if (d.pos != nullptr) CK(cudaMemsetAsync(d.force, 0, sizeof(double) * 2 * L, h.stream));
-        launch_spread<double>(mp, h.tiles, d.force, h.nx, h.ny, L, d.st, d.it0, h.stream);
+        launch_spread<double>(mp, h.tiles, d.force, h.nx, h.ny, L, d.st, h.stream);
         if (d.rs == 4) launch_to_float(d.force, d.force32, 2 * L, h.stream);
     } else {
         // the nodes may go anywhere: the forward's lattice kernels read the whole
@@ -2648,7 +2646,8 @@ static void diff_backward(Handle& h, DiffCtx& d) {
     // Segment s (steps base+1 .. base+len) is reversed from the states
     // base .. base+len-1: the checkpoint, then its recomputed states in a
     // segment buffer (d.seg always, or alternately d.seg and d.seg2).
-    // (a run with moving nodes refills the one force field every step: serial)
+    // (a run with moving nodes spreads its fields anew every step, for the
+    // recomputation as for the reverse: serial)
     const bool two = d.seg2 != nullptr && !d.motion;
     if (d.motion) {
         if (d.haveSeedX)
@@ -2890,11 +2889,11 @@ int lbib_lattice_step(lbib_handle* hh, int n, int outlet) {
         const int p = h.cur;
         if (h.profiling) CK(cudaEventRecord(h.kEvents[2 * i], h.stream));
         if (h.precision == LBIB_FP64) {
-            auto a = lbib::lattice_args<double>(h, h.iteration, p);
+            auto a = lbib::lattice_args<double>(h, p);
             a.outlet = outlet ? 1 : 0;
             lbib::launch_stream_collide64(a, h.stream);
         } else {
-            auto a = lbib::lattice_args<float>(h, h.iteration, p);
+            auto a = lbib::lattice_args<float>(h, p);
             a.outlet = outlet ? 1 : 0;
             lbib::launch_stream_collide32(a, h.stream);
         }
@@ -4227,7 +4226,7 @@ int lbib_upload_membrane(lbib_handle* hh, const unsigned* ids, const double* xy,
     // new nodes are bound to the lattice at once: the edge test of
     // connectGeometryNodesToPhysicalNodes (GeometryHandler.cpp:618-636)
     lbib::reset_status(h, h.iteration, h.cellTypesCopied);
-    lbib::launch_edge_check(h.m, h.nx, h.ny, h.st, 0, h.stream);
+    lbib::launch_edge_check(h.m, h.nx, h.ny, h.st, h.stream);
     lbib::read_status(h);
     if (h.stHost->err) lbib::fail(h.stHost->err, "geometry point moved too close to the boundary", h.stHost->errIndex);
     h.graphEpoch++;

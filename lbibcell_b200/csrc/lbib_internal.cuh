@@ -138,9 +138,6 @@ struct Status {
     int nPerturbNode;  // membrane nodes whose position needs the host RNG
     int nPerturbConn;  // connections that need Connection::perturbConnection
     int nChanged;      // lattice nodes whose domain id changed (reinit list)
-    int nRecords;      // crossing records this step
-    int remesh;        // a connection is longer than MAXLENGTH
-    int coarsen;       // a node is a coarsening candidate
     int nDiagReinit;   // reinit from diagonal neighbours
     int nFailedReinit; // reinit without any neighbour (division by zero)
     unsigned iteration;   // Parameters' current iteration of the step being run
