@@ -389,8 +389,9 @@ __device__ __forceinline__ int take_tile_count(const TileDev& t, int tile, const
 // node testing every entry, the spread took 96 us for 150k nodes on 1024^2 and
 // 21 us for one cell.  Adding each entry's 16 products to shared memory, a
 // lane each, took 48 and 17 us (a chain of shared-memory round trips); this
-// form takes 40 (instruction issue) and 6.5 us.  Four rows per warp of a
-// 128-thread block: 40 and 8.2 us.
+// form takes 40 (issue in 55 % of the cycles; the barriers of unevenly filled tiles
+// stall it first) and 6.5 us.  Four rows per warp of a 128-thread block: 40 and
+// 8.2 us.
 constexpr int kSpreadMax = 768;    // entries of a tile
 constexpr int kSpreadChunk = 128;  // entries whose factors are held at once
 template <typename Real>
